@@ -38,7 +38,7 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode_fn() {
 }
 
 int auto_chunk(const dg_ctx *c) {
-    return c->chunk > 0 ? c->chunk : choose_chunk(c->nx, c->ny, c->nz, c->kind);
+    return c->chunk > 0 ? c->chunk : c->chunk_auto;
 }
 
 int encode_map(dg_ctx *c, int i) {
@@ -266,6 +266,7 @@ int32_t dg_create(const dg_sim_info *info, dg_ctx **out) {
     c->ny = info->ny + 4;
     c->nz = info->nz + 4;
     c->pitch = (c->nz + 31) / 32 * 32;
+    c->chunk_auto = choose_chunk(c->nx, c->ny, c->nz, c->kind);
     // Test hook: a context created while DG_DEBUG_WAIT_BUDGET is set gives
     // its step kernels' waits for staged planes that many SM clocks (0 or
     // less: every such wait gives up at once, without waiting) instead of

@@ -24,6 +24,7 @@ struct dg_ctx {
     CUtensorMap tmap[2];
     cudaStream_t stream;
     int chunk;                 // 0 = automatic
+    int chunk_auto;            // choose_chunk of this grid
     bool exact;                // reference-rounding policy
     int kind;                  // KernelKind of the step kernel
     long long wait_budget;     // 0: default; from DG_DEBUG_WAIT_BUDGET (tests of the timeout path)

@@ -172,13 +172,42 @@ inline int step_grid_blocks(int nx, int ny, int nz, int kind, int chunk) {
     const int tiles_y = (ny - 4 + ty - 1) / ty;
     return tiles_z * tiles_y * chunks;
 }
+// Blocks' finishing time on the SMs, in planes, of a sweep launch over
+// `tiles` tiles and nxi planes in `chunk`-plane blocks, one block per SM, the
+// shorter last chunk's blocks dispatched last: every SM takes full chunks in
+// turn, then the remainders go to whichever SMs are free first.  A block
+// costs its planes plus kBlockPlanes: the two planes it computes beyond its
+// chunk and about two planes' time of launch, first copies and reduction
+// (measured on the FP32 kernel: 8 us + 4.1 us per plane marched).
+constexpr int kBlockPlanes = 4;
+inline long long sweep_makespan(long long tiles, int nxi, int chunk) {
+    const long long full = tiles * (nxi / chunk), rest = nxi % chunk ? tiles : 0;
+    const long long cf = chunk + kBlockPlanes, cr = nxi % chunk + kBlockPlanes;
+    // SMs that got one full block more than the others
+    long long n_late = full % kSms, t_late = (full / kSms + (n_late ? 1 : 0)) * cf;
+    long long n_free = kSms - n_late, t_free = full / kSms * cf, left = rest, end = n_late ? t_late : t_free;
+    while (left > 0) {
+        long long &t = (n_late == 0 || t_free <= t_late) ? t_free : t_late;
+        left -= &t == &t_free ? n_free : n_late;
+        t += cr;
+        if (t > end) end = t;
+    }
+    return end;
+}
+
 // Default x-planes per block.  Reference-rounding kernels: enough blocks for
 // ~14 waves of resident CTAs (2 per SM), at least 20 planes per block (each
 // block re-stages 4 planes at its ends); measured flat within 1 % from 43
 // to 74 planes on 512^3.  Sweep kernels (one block per SM): with interior
-// tiles, the frame launch's chunk (the interior launch marches whole
-// columns); without, the split of x into chunks that minimises waves x
-// (planes per block + 3 re-staged), with at least 24 planes per block.
+// tiles that fill the SMs, the frame launch's chunk (the interior launch
+// marches whole columns); with fewer interior tiles, the split of x that
+// minimises waves x (planes + 3 re-staged), at least 24 planes per block
+// unless that leaves SMs idle (40x300x130: 181 -> 102 us); with none, the split that ends first (sweep_makespan), down
+// to single planes: a small grid is latency-bound, a block's time being its
+// planes one after another, so short chunks on all SMs win although each
+// block recomputes two planes (FP32, periodic, us per step, at least 24
+// planes per block -> this rule: 48^3 116 -> 25, 64^3 146 -> 29, 128^3
+// 124 -> 93, 300x40x70 116 -> 75).
 inline int choose_chunk(int nx, int ny, int nz, int kind) {
     const int ty = step_tile_rows(kind), tzc = step_tile_cols(kind);
     // sweep steps whose interior tiles fill the SMs (interior_chunk): the
@@ -189,16 +218,30 @@ inline int choose_chunk(int nx, int ny, int nz, int kind) {
     const long long tiles = (long long)((ny - 4 + ty - 1) / ty) * ((nz - 4 + tzc - 1) / tzc);
     const int nxi = nx - 4;
     if (is_sweep(kind)) {
-        const int maxc = nxi / 24 > 0 ? nxi / 24 : 1;
-        long long best = -1;
-        int bestc = 1;
-        for (int c = 1; c <= maxc && c <= 64; ++c) {
-            const long long per = (nxi + c - 1) / c;
-            const long long waves = (tiles * c + kSms - 1) / kSms;
-            const long long cost = waves * (per + 3);
-            if (best < 0 || cost < best) { best = cost; bestc = c; }
+        if (InteriorTiles(ny, nz, ty, tzc).interior() > 0) {
+            const int maxc = nxi / 24 > 0 ? nxi / 24 : 1;
+            long long best = -1;
+            int bestc = 1;
+            for (int c = 1; c <= nxi && c <= 64; ++c) {
+                if (c > maxc && tiles * c > 4 * kSms) break;
+                const long long per = (nxi + c - 1) / c;
+                const long long waves = (tiles * c + kSms - 1) / kSms;
+                const long long cost = waves * (per + 3);
+                if (best < 0 || cost < best) { best = cost; bestc = c; }
+            }
+            return (nxi + bestc - 1) / bestc;
         }
-        return (nxi + bestc - 1) / bestc;
+        int bestp = nxi;
+        long long best = sweep_makespan(tiles, nxi, nxi);
+        for (int p = nxi - 1; p >= 1; --p) {
+            // short chunks only where they fill idle SMs: a large grid's count
+            // of blocks (and of partials) stays that of 24 planes or more
+            const long long c = (nxi + p - 1) / p;
+            if ((p < 24 || c > 64) && tiles * c > 4 * kSms) continue;
+            const long long t = sweep_makespan(tiles, nxi, p);
+            if (t < best) { best = t; bestp = p; }
+        }
+        return bestp;
     }
     const long long target = 2LL * kSms * 14;
     long long chunks = (target + tiles - 1) / tiles;
