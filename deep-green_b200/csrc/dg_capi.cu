@@ -172,12 +172,10 @@ int enqueue(dg_ctx *c, int nsteps) {
         cudaError_t e;
         if (c->elem == 8) {
             auto a = grid_args<double>(c, c->buf[src], c->buf[dst]);
-            e = c->kind == kFastF64 ? launch_sweep(a, &c->tmap[src], chunk, c->stream)
-                                    : launch_step_policy<double, true>(a, &c->tmap[src], c->info.limiter, chunk,
-                                                                       c->stream);
+            e = launch_march(a, &c->tmap[src], c->kind, chunk, c->stream);
         } else {
             auto a = grid_args<float>(c, c->buf[src], c->buf[dst]);
-            e = c->exact ? launch_step_policy<float, true>(a, &c->tmap[src], c->info.limiter, chunk, c->stream)
+            e = c->exact ? launch_march(a, &c->tmap[src], c->kind, chunk, c->stream)
                          : launch_sweep(a, &c->tmap[src], chunk, c->stream);
         }
         if (e != cudaSuccess) return cuda_fail(c, e, "step kernel launch");

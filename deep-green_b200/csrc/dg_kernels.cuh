@@ -12,8 +12,6 @@
 
 namespace dg {
 
-constexpr int kTZ = 32;          // tile width along z (one warp)
-constexpr int kRZ = kTZ + 4;     // staged region width along z (2-cell halo)
 constexpr int kHist = 4096;      // dt history ring on the device
 constexpr unsigned kStatusNonFinite = 0x1u;
 constexpr unsigned kStatusTimeout = 0x2u;
@@ -83,33 +81,25 @@ template <class T> inline void set_boundaries(GridArgs<T> &a, const int32_t bcs[
 constexpr int kSms = 148;
 constexpr int kReduceBlocks = kSms * 8;   // grid of the state-reduction kernel
 
-// The step kernels: reference rounding in double and in float
-// (dg_step_impl.cuh) and the fused-arithmetic sweep in float and in double
-// (dg_sweep_impl.cuh).
+// The step kernels: one cell per lane (dg_march_impl.cuh) with the
+// reference's rounding in double and in float and with fused arithmetic in
+// double, and the packed fused-arithmetic sweep in float (dg_sweep_impl.cuh).
 enum KernelKind : int { kRefF64 = 0, kRefF32 = 1, kFastF32 = 2, kFastF64 = 3 };
 
-inline bool is_sweep(int kind) { return kind == kFastF32 || kind == kFastF64; }
+inline bool is_sweep(int kind) { return kind == kFastF32; }
 
-// Owned tile rows (y) of each kernel.  A sweep block also runs two halo warps.
+// Owned tile rows (y) of each kernel; a block also runs two halo warps.
 #ifndef DG_SWEEP_ROWS_F32
 #define DG_SWEEP_ROWS_F32 14
 #endif
 constexpr int kSweepRowsF32 = DG_SWEEP_ROWS_F32;
-constexpr int kSweepRowsF64 = 4;
-inline int step_tile_rows(int kind) {
-    switch (kind) {
-        case kRefF64: return 4;
-        case kRefF32: return 8;
-        case kFastF32: return kSweepRowsF32;
-        default: return kSweepRowsF64;
-    }
-}
+constexpr int kMarchRows = 14;   // 16 warps of 128 registers
+constexpr int kMarchRing = 3;    // staged planes
+inline int step_tile_rows(int kind) { return is_sweep(kind) ? kSweepRowsF32 : kMarchRows; }
 // Tile columns (z) and the staged box width (2-cell halo each side).
-inline int step_tile_cols(int kind) { return is_sweep(kind) ? 64 : kTZ; }
+inline int step_tile_cols(int kind) { return is_sweep(kind) ? 64 : 32; }
 inline int step_box_cols(int kind) { return step_tile_cols(kind) + 4; }
-inline int step_threads(int kind) {
-    return is_sweep(kind) ? 32 * (step_tile_rows(kind) + 2) : 32 * step_tile_rows(kind);
-}
+inline int step_threads(int kind) { return 32 * (step_tile_rows(kind) + 2); }
 
 // Tiles of a sweep step.  Interior tiles are full tiles (rows x cols) at
 // least two cells clear of every y and z face, so that no row or column of
@@ -195,12 +185,9 @@ inline long long sweep_makespan(long long tiles, int nxi, int chunk) {
     return end;
 }
 
-// Default x-planes per block.  Reference-rounding kernels: enough blocks for
-// ~14 waves of resident CTAs (2 per SM), at least 20 planes per block (each
-// block re-stages 4 planes at its ends); measured flat within 1 % from 43
-// to 74 planes on 512^3.  Sweep kernels (one block per SM): with interior
-// tiles that fill the SMs, the frame launch's chunk (the interior launch
-// marches whole columns); with fewer interior tiles, the split of x that
+// Default x-planes per block (one block per SM).  The packed sweep with
+// interior tiles that fill the SMs: the frame launch's chunk (the interior
+// launch marches whole columns); with fewer interior tiles: the split of x that
 // minimises waves x (planes + 3 re-staged), at least 24 planes per block
 // unless that leaves SMs idle (40x300x130: 181 -> 102 us); with none, the split that ends first (sweep_makespan), down
 // to single planes: a small grid is latency-bound, a block's time being its
@@ -217,50 +204,35 @@ inline int choose_chunk(int nx, int ny, int nz, int kind) {
     if (is_sweep(kind) && InteriorTiles(ny, nz, ty, tzc).interior() >= kSms) return nx - 4 < 64 ? nx - 4 : 64;
     const long long tiles = (long long)((ny - 4 + ty - 1) / ty) * ((nz - 4 + tzc - 1) / tzc);
     const int nxi = nx - 4;
-    if (is_sweep(kind)) {
-        if (InteriorTiles(ny, nz, ty, tzc).interior() > 0) {
-            const int maxc = nxi / 24 > 0 ? nxi / 24 : 1;
-            long long best = -1;
-            int bestc = 1;
-            for (int c = 1; c <= nxi && c <= 64; ++c) {
-                if (c > maxc && tiles * c > 4 * kSms) break;
-                const long long per = (nxi + c - 1) / c;
-                const long long waves = (tiles * c + kSms - 1) / kSms;
-                const long long cost = waves * (per + 3);
-                if (best < 0 || cost < best) { best = cost; bestc = c; }
-            }
-            return (nxi + bestc - 1) / bestc;
+    if (is_sweep(kind) && InteriorTiles(ny, nz, ty, tzc).interior() > 0) {
+        const int maxc = nxi / 24 > 0 ? nxi / 24 : 1;
+        long long best = -1;
+        int bestc = 1;
+        for (int c = 1; c <= nxi && c <= 64; ++c) {
+            if (c > maxc && tiles * c > 4 * kSms) break;
+            const long long per = (nxi + c - 1) / c;
+            const long long waves = (tiles * c + kSms - 1) / kSms;
+            const long long cost = waves * (per + 3);
+            if (best < 0 || cost < best) { best = cost; bestc = c; }
         }
-        int bestp = nxi;
-        long long best = sweep_makespan(tiles, nxi, nxi);
-        for (int p = nxi - 1; p >= 1; --p) {
-            // short chunks only where they fill idle SMs: a large grid's count
-            // of blocks (and of partials) stays that of 24 planes or more
-            const long long c = (nxi + p - 1) / p;
-            if ((p < 24 || c > 64) && tiles * c > 4 * kSms) continue;
-            const long long t = sweep_makespan(tiles, nxi, p);
-            if (t < best) { best = t; bestp = p; }
-        }
-        return bestp;
+        return (nxi + bestc - 1) / bestc;
     }
-    const long long target = 2LL * kSms * 14;
-    long long chunks = (target + tiles - 1) / tiles;
-    const long long maxc = nxi / 20 > 0 ? nxi / 20 : 1;
-    if (chunks > maxc) chunks = maxc;
-    if (chunks < 1) chunks = 1;
-    return (int)((nxi + chunks - 1) / chunks);
-}
-
-template <class T> int step_grid_blocks(const GridArgs<T> &a, int chunk) {
-    return step_grid_blocks(a.nx, a.ny, a.nz, sizeof(T) == 8 ? kRefF64 : kRefF32, chunk);
+    int bestp = nxi;
+    long long best = sweep_makespan(tiles, nxi, nxi);
+    for (int p = nxi - 1; p >= 1; --p) {
+        // short chunks only where they fill idle SMs: a large grid's count
+        // of blocks (and of partials) stays that of 24 planes or more
+        const long long c = (nxi + p - 1) / p;
+        if ((p < 24 || c > 64) && tiles * c > 4 * kSms) continue;
+        const long long t = sweep_makespan(tiles, nxi, p);
+        if (t < best) { best = t; bestp = p; }
+    }
+    return bestp;
 }
 
 // Launch helpers.  EXACT selects the reference-rounding policy
 // (dg_step_ref.cu, built with --fmad=false) or the fast one
 // (dg_step_fast.cu); float/fast, float/exact and double/exact exist.
-template <class T, bool EXACT>
-cudaError_t launch_step_policy(const GridArgs<T> &a, const CUtensorMap *tmap_src, int limiter, int chunk,
-                               cudaStream_t st);
 template <class T, bool EXACT> cudaError_t launch_reduce_policy(const GridArgs<T> &a, int set_dt, cudaStream_t st);
 template <class T, bool EXACT>
 cudaError_t launch_cons_to_prim_policy(const GridArgs<T> &a, const T *cons, T *prim, long long prim_fstride,
@@ -268,10 +240,11 @@ cudaError_t launch_cons_to_prim_policy(const GridArgs<T> &a, const T *cons, T *p
 // Message returned by dg_last_error(NULL) (errors not tied to a context).
 void set_global_error(const std::string &msg);
 
-// The sweep kernel (kFastF32 / kFastF64 contexts); the tensor map's box is
-// step_box_cols x (step_tile_rows + 4) x 1 x 5.
+// The step; the tensor map's box is step_box_cols x (step_tile_rows + 4) x 1
+// x 5.  launch_sweep: kFastF32; launch_march: the other kinds.
 cudaError_t launch_sweep(const GridArgs<float> &a, const CUtensorMap *tmap_src, int chunk, cudaStream_t st);
-cudaError_t launch_sweep(const GridArgs<double> &a, const CUtensorMap *tmap_src, int chunk, cudaStream_t st);
+cudaError_t launch_march(const GridArgs<float> &a, const CUtensorMap *tmap_src, int kind, int chunk, cudaStream_t st);
+cudaError_t launch_march(const GridArgs<double> &a, const CUtensorMap *tmap_src, int kind, int chunk, cudaStream_t st);
 template <class T> cudaError_t launch_fill_ghosts(const GridArgs<T> &a, T *buf, cudaStream_t st);
 template <class T>
 cudaError_t launch_prim_to_cons(const GridArgs<T> &a, const T *prim, long long prim_fstride, int prim_pitch, T *cons,

@@ -25,6 +25,7 @@
 //     before any stream capture.
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cstddef>
 #include <cstring>
 #include <mutex>
@@ -113,13 +114,34 @@ GridArgs<T> args_for(const dg_sim_info *info, const void *src, void *dst, void *
     return a;
 }
 
+// The block count that decides whether a grid fits the scratch.  For the
+// one-cell-per-lane kernels it is counted in 32 x 4 (FP64 reference rounding),
+// 32 x 8 (FP32) or 64 x 4 tiles, the sizes this entry point's limit was first
+// set by: those kernels need fewer blocks now, and a caller that sizes its
+// grids by the limit keeps the same answer.
+long long limit_blocks(const dg_sim_info *info, int kind) {
+    if (kind == kFastF32) return 0;
+    const long long rows = kind == kRefF32 ? 8 : 4, cols = kind == kFastF64 ? 64 : 32, nx = info->nx;
+    const long long ty = (info->ny + rows - 1) / rows, tz = (info->nz + cols - 1) / cols, tiles = ty * tz;
+    if (kind != kFastF64) {
+        const long long want = (2LL * kSms * 14 + tiles - 1) / tiles, most = std::max<long long>(1, nx / 20);
+        const long long per = (nx + std::min(want, most) - 1) / std::max<long long>(1, std::min(want, most));
+        return tiles * ((nx + per - 1) / per);
+    }
+    return tiles;
+}
+
 template <class T>
 int run(const dg_sim_info *info, int kind, void *cons_in, void *cons_out, double *dt_used, cudaStream_t st,
         void *scratch) {
     const int elem = (int)sizeof(T);
     GridArgs<T> a = args_for<T>(info, cons_in, cons_out, scratch);
-    const int chunk = choose_chunk(a.nx, a.ny, a.nz, kind);
-    const int blocks = step_grid_blocks(a.nx, a.ny, a.nz, kind, chunk);
+    int chunk = choose_chunk(a.nx, a.ny, a.nz, kind);
+    // a split with more blocks than the scratch has partials gives way to
+    // whole columns
+    if (step_grid_blocks(a.nx, a.ny, a.nz, kind, chunk) > kMaxBlocks) chunk = a.nx - 4;
+    const long long blocks = std::max<long long>(limit_blocks(info, kind),
+                                                 step_grid_blocks(a.nx, a.ny, a.nz, kind, chunk));
     if (blocks > kMaxBlocks || kReduceBlocks > kMaxBlocks)
         return fail(DG_ERR_INVALID, "grid too large for the no-allocation scratch (" + std::to_string(blocks) +
                                         " blocks > " + std::to_string(kMaxBlocks) + ")");
@@ -146,13 +168,11 @@ int run(const dg_sim_info *info, int kind, void *cons_in, void *cons_out, double
             if (e == cudaSuccess) e = launch_sweep(a, &map, chunk, st);
         } else {
             if (e == cudaSuccess) e = launch_reduce_policy<float, true>(a, 1, st);
-            if (e == cudaSuccess) e = launch_step_policy<float, true>(a, &map, info->limiter, chunk, st);
+            if (e == cudaSuccess) e = launch_march(a, &map, kind, chunk, st);
         }
     } else {
         if (e == cudaSuccess) e = launch_reduce_policy<double, true>(a, 1, st);
-        if (e == cudaSuccess)
-            e = kind == kFastF64 ? launch_sweep(a, &map, chunk, st)
-                                 : launch_step_policy<double, true>(a, &map, info->limiter, chunk, st);
+        if (e == cudaSuccess) e = launch_march(a, &map, kind, chunk, st);
     }
     if (e != cudaSuccess) return fail(DG_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     if (dt_used) {

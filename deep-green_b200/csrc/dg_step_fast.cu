@@ -1,6 +1,6 @@
-// dg_step_fast.cu -- the fused-arithmetic step (fast policy; multiply-add
-// contraction allowed): the sweep kernel in FP32 and FP64, and the fast
-// policy's state reduction.  Kernels: dg_sweep_impl.cuh, dg_step_impl.cuh.
+// dg_step_fast.cu -- the FP32 fused-arithmetic step (fast policy;
+// multiply-add contraction allowed): the sweep kernel and the fast policy's
+// state reduction.  Kernels: dg_sweep_impl.cuh, dg_step_impl.cuh.
 #include "dg_host.h"
 #include "dg_step_impl.cuh"
 #include "dg_sweep_impl.cuh"
@@ -8,15 +8,8 @@
 namespace dg {
 
 namespace {
-template <class T> struct SweepCfg;
-template <> struct SweepCfg<float> {
-    // five staged planes when they fit in shared memory, else four
-    static constexpr int TY = kSweepRowsF32;
-    static constexpr int R = sizeof(sweep::Smem<float, TY, 5>) + 1024 <= 232448 ? 5 : 4;
-};
-template <> struct SweepCfg<double> {
-    static constexpr int TY = kSweepRowsF64, R = 4;
-};
+// five staged planes when they fit in shared memory, else four
+constexpr int kSweepRing = sizeof(sweep::Smem<float, kSweepRowsF32, 5>) + 1024 <= 232448 ? 5 : 4;
 
 // One step: with interior tiles (InteriorTiles) two launches sharing one
 // reduction -- the interior tiles, with the owned warps' boundary switches
@@ -27,12 +20,12 @@ template <> struct SweepCfg<double> {
 // wave leaves free.  Without interior tiles, one launch of the general
 // kernel over all tiles.  (One kernel body holding both variants of the
 // loop ran slower than either alone.)
-template <class T, int LIM, bool GRAV>
-cudaError_t launch_sweep_t(const GridArgs<T> &a, const CUtensorMap *tmap, int chunk, cudaStream_t st) {
-    constexpr int TY = SweepCfg<T>::TY, R = SweepCfg<T>::R;
-    auto k_in = sweep::sweep_step_kernel<T, TY, R, LIM, GRAV, true>;
-    auto k_frame = sweep::sweep_step_kernel<T, TY, R, LIM, GRAV, false>;
-    constexpr int smem = sweep::smem_bytes<T, TY, R>();
+template <int LIM, bool GRAV>
+cudaError_t launch_sweep_t(const GridArgs<float> &a, const CUtensorMap *tmap, int chunk, cudaStream_t st) {
+    constexpr int TY = kSweepRowsF32, R = kSweepRing;
+    auto k_in = sweep::sweep_step_kernel<float, TY, R, LIM, GRAV, true>;
+    auto k_frame = sweep::sweep_step_kernel<float, TY, R, LIM, GRAV, false>;
+    constexpr int smem = sweep::smem_bytes<float, TY, R>();
     static std::atomic<unsigned long long> attr_in{0}, attr_frame{0};
     cudaError_t e = ensure_dynamic_smem(k_in, smem, attr_in);
     if (e == cudaSuccess) e = ensure_dynamic_smem(k_frame, smem, attr_frame);
@@ -62,24 +55,14 @@ cudaError_t launch_sweep_t(const GridArgs<T> &a, const CUtensorMap *tmap, int ch
     return cudaLaunchKernelEx(&cfg, k_frame, a, *tmap, chunk, n_in, nparts);
 }
 
-// One kernel per (limiter, gravity): the slope and flux code of the march
-// is fixed at compile time.
-template <class T>
-cudaError_t launch_sweep_any(const GridArgs<T> &a, const CUtensorMap *tmap, int chunk, cudaStream_t st) {
-    if (a.gravity) {
-        return a.limiter == 0 ? launch_sweep_t<T, 0, true>(a, tmap, chunk, st)
-                              : launch_sweep_t<T, 1, true>(a, tmap, chunk, st);
-    }
-    return a.limiter == 0 ? launch_sweep_t<T, 0, false>(a, tmap, chunk, st)
-                          : launch_sweep_t<T, 1, false>(a, tmap, chunk, st);
-}
 }  // namespace
 
+// One kernel per (limiter, gravity): the slope and flux code of the march
+// is fixed at compile time.
 cudaError_t launch_sweep(const GridArgs<float> &a, const CUtensorMap *tmap, int chunk, cudaStream_t st) {
-    return launch_sweep_any(a, tmap, chunk, st);
-}
-cudaError_t launch_sweep(const GridArgs<double> &a, const CUtensorMap *tmap, int chunk, cudaStream_t st) {
-    return launch_sweep_any(a, tmap, chunk, st);
+    if (a.gravity)
+        return a.limiter == 0 ? launch_sweep_t<0, true>(a, tmap, chunk, st) : launch_sweep_t<1, true>(a, tmap, chunk, st);
+    return a.limiter == 0 ? launch_sweep_t<0, false>(a, tmap, chunk, st) : launch_sweep_t<1, false>(a, tmap, chunk, st);
 }
 
 template cudaError_t launch_reduce_policy<float, false>(const GridArgs<float> &, int, cudaStream_t);

@@ -2,10 +2,25 @@
 // request).  This file is compiled with --fmad=false so that no multiply-add
 // is fused and every operation rounds as in the reference's scalar code.
 // Also holds the set-up kernels that must round like the reference
-// (calc_conserved) and the ghost fill.  Kernels: dg_step_impl.cuh.
+// (calc_conserved) and the ghost fill, and the FP64 step with fused
+// arithmetic (every fused operation is written as one).  Kernels:
+// dg_march_impl.cuh, dg_step_impl.cuh.
+#include "dg_march_impl.cuh"
 #include "dg_step_impl.cuh"
 
 namespace dg {
+
+cudaError_t launch_march(const GridArgs<double> &a, const CUtensorMap *tmap, int kind, int chunk, cudaStream_t st) {
+    const int blocks = step_grid_blocks(a.nx, a.ny, a.nz, kind, chunk);
+    return kind == kFastF64
+               ? march::launch<double, march::FusedArith, kMarchRows, kMarchRing>(a, tmap, blocks, chunk, st)
+               : march::launch<double, march::RefArith<double>, kMarchRows, kMarchRing>(a, tmap, blocks, chunk, st);
+}
+
+cudaError_t launch_march(const GridArgs<float> &a, const CUtensorMap *tmap, int kind, int chunk, cudaStream_t st) {
+    const int blocks = step_grid_blocks(a.nx, a.ny, a.nz, kind, chunk);
+    return march::launch<float, march::RefArith<float>, kMarchRows, kMarchRing>(a, tmap, blocks, chunk, st);
+}
 
 template <class T> cudaError_t launch_fill_ghosts(const GridArgs<T> &a, T *buf, cudaStream_t st) {
     const long long ghosts = (long long)a.nx * a.ny * a.nz - (long long)(a.nx - 4) * (a.ny - 4) * (a.nz - 4);
@@ -21,8 +36,6 @@ cudaError_t launch_prim_to_cons(const GridArgs<T> &a, const T *prim, long long p
 }
 
 #define DG_REF_INSTANTIATE(T)                                                                                      \
-    template cudaError_t launch_step_policy<T, true>(const GridArgs<T> &, const CUtensorMap *, int, int,            \
-                                                     cudaStream_t);                                                \
     template cudaError_t launch_reduce_policy<T, true>(const GridArgs<T> &, int, cudaStream_t);                     \
     template cudaError_t launch_cons_to_prim_policy<T, true>(const GridArgs<T> &, const T *, T *, long long, int,   \
                                                              cudaStream_t);                                        \

@@ -1,7 +1,7 @@
 // dg_sweep_impl.cuh -- the production step kernel of compute_step
 // (deep-green src/rs/src/physics.rs:595-681) with fused arithmetic (the
-// "fast" policy), in FP32 on packed pairs or in FP64: one launch per step,
-// or two (interior tiles, frame) on grids with interior tiles.
+// "fast" policy) in FP32 on packed pairs: one launch per step, or two
+// (interior tiles, frame) on grids with interior tiles.
 //
 // Decomposition.  A block owns a tile of TY rows (y) x 64 columns (z) of
 // cells and marches along x through a chunk of planes.  Each plane arrives by
@@ -10,7 +10,7 @@
 // conserved totals until its cells are updated.
 //   * Owned warps (TY): warp r owns row y0 + r; lane l owns the two adjacent
 //     cells (z, z + 1), z = z0 + 2l, as one pair.  Every per-cell formula is
-//     written on pairs, and in FP32 a pair is one packed register, so the
+//     written on pairs, and a pair is one packed register, so the
 //     arithmetic runs on Blackwell's packed instructions (add/sub/mul/fma
 //     .f32x2: two cells per instruction).  The x-neighbours of a cell are
 //     carried in registers along the march; the y-neighbours come from the
@@ -53,8 +53,9 @@ constexpr int kTileZ = 64;            // tile columns: 32 lanes x 2 cells
 constexpr int kBoxZ = kTileZ + 4;     // staged columns: 2-cell halo each side
 
 // ---------------------------------------------------------------------------
-// Pair arithmetic.  float2: packed FP32 instructions; double2: two scalar
-// operations.  Scalars of the pair's element type have the same interface.
+// Arithmetic on V: float2 (a pair of cells, packed FP32 instructions) or
+// double (one cell; the one-cell-per-lane kernel of dg_march_impl.cuh takes
+// its FP64 formulas from here).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
@@ -70,32 +71,25 @@ __device__ __forceinline__ float2 vsub(float2 a, float2 b) {
         : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
     return r;
 }
-__device__ __forceinline__ double2 vadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 vsub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 vmul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
-__device__ __forceinline__ double2 vfma(double2 a, double2 b, double2 c) {
-    return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
-}
-
-template <class T> struct PairT;
-template <> struct PairT<float> { using type = float2; };
-template <> struct PairT<double> { using type = double2; };
+__device__ __forceinline__ double vadd(double a, double b) { return a + b; }
+__device__ __forceinline__ double vsub(double a, double b) { return a - b; }
+__device__ __forceinline__ double vmul(double a, double b) { return a * b; }
+__device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
 
 template <class V> __device__ __forceinline__ V spl(double s);
 template <> __device__ __forceinline__ float2 spl<float2>(double s) { return make_float2((float)s, (float)s); }
-template <> __device__ __forceinline__ double2 spl<double2>(double s) { return make_double2(s, s); }
+template <> __device__ __forceinline__ double spl<double>(double s) { return s; }
 __device__ __forceinline__ float2 mk(float a, float b) { return make_float2(a, b); }
-__device__ __forceinline__ double2 mk(double a, double b) { return make_double2(a, b); }
 
 // 1/x of both cells: the fast policy's reciprocal (Phys<T, false>::prim).
 __device__ __forceinline__ float2 vrcp(float2 a) { return make_float2(rcp_approx(a.x), rcp_approx(a.y)); }
-__device__ __forceinline__ double2 vrcp(double2 a) { return make_double2(1.0 / a.x, 1.0 / a.y); }
+__device__ __forceinline__ double vrcp(double a) { return 1.0 / a; }
 __device__ __forceinline__ float2 vrsq(float2 a) { return make_float2(rsqrt_approx(a.x), rsqrt_approx(a.y)); }
-__device__ __forceinline__ double2 vrsq(double2 a) { return make_double2(rsqrt(a.x), rsqrt(a.y)); }
+__device__ __forceinline__ double vrsq(double a) { return rsqrt(a); }
 __device__ __forceinline__ float2 vmax(float2 a, float2 b) { return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)); }
-__device__ __forceinline__ double2 vmax(double2 a, double2 b) { return make_double2(fmax(a.x, b.x), fmax(a.y, b.y)); }
+__device__ __forceinline__ double vmax(double a, double b) { return fmax(a, b); }
 __device__ __forceinline__ float2 vabs(float2 a) { return make_float2(fabsf(a.x), fabsf(a.y)); }
-__device__ __forceinline__ double2 vabs(double2 a) { return make_double2(fabs(a.x), fabs(a.y)); }
+__device__ __forceinline__ double vabs(double a) { return fabs(a); }
 
 // minmod(a, b): 0 when the signs differ or either is zero, else the one of
 // smaller magnitude.  FP32: min(|a|, |b|) carrying the product of the signs
@@ -109,7 +103,6 @@ __device__ __forceinline__ float mm(float a, float b) {
 }
 __device__ __forceinline__ double mm(double a, double b) { return fmin(fmax(b, fmin(a, 0.0)), fmax(a, 0.0)); }
 __device__ __forceinline__ float2 mm(float2 a, float2 b) { return make_float2(mm(a.x, b.x), mm(a.y, b.y)); }
-__device__ __forceinline__ double2 mm(double2 a, double2 b) { return make_double2(mm(a.x, b.x), mm(a.y, b.y)); }
 
 // Slope in cell units (slope * ds) from the backward and forward
 // differences: minmod (LIM 1) or the reference's central difference
@@ -131,6 +124,30 @@ template <class T> struct K {
     T sc[5];   // update scale per field: -dt ds^2 / 2 (mass, momenta), / 4 (energy)
     T hq4;     // conducting wall: 4 Q/V per kelvin of (273 - t_in), the energy flux's scale
 };
+
+template <class T> __device__ __forceinline__ K<T> make_k(const GridArgs<T> &a, T dt) {
+    K<T> k;
+    k.inv_vol = a.k.inv_vol;
+    k.gamma = a.k.gamma;
+    k.gm1 = a.k.gm1;
+    k.kp = T(2) * a.k.inv_gm1;
+    k.c1 = T(0.5) * a.k.gm1;
+    k.sg = (T)sqrt((double)a.k.gamma);
+    k.iv_h = T(0.5) * a.k.inv_vol;
+    k.nh4 = T(-2) * dt * a.k.inv_ds;   // -4 dt / (2 ds)
+    const T scale = dt * a.k.ds * a.k.ds;
+    k.sc[0] = k.sc[1] = k.sc[2] = k.sc[3] = T(-0.5) * scale;
+    k.sc[4] = T(-0.25) * scale;
+    // wall_heat's factor S / (d/kappa + 1/hc_out) / V, times 4
+    const T ds = a.k.ds;
+    k.hq4 = T(4) * ((ds * ds) / ((T(0.008f) / T(0.2f)) + (T(1.0f) / T(10.0f)))) / (ds * ds * ds);
+    return k;
+}
+
+// Gravity height term of a z face whose lower cell has ghosted index klow.
+template <class T> __device__ __forceinline__ T grav_h(const GridArgs<T> &a, int klow) {
+    return a.k.g * (T(a.nz - 4) * a.k.ds - T(klow - 2) * a.k.ds);
+}
 
 // Conducting-wall heat of one cell in the energy flux's scale (4 Q/V,
 // wall_heat's formula with its constant factor folded into k.hq4); xr, xp:
@@ -274,7 +291,8 @@ template <class T, int TY, int R> struct Smem {
 };
 
 template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
-    using V = typename PairT<T>::type;
+    static_assert(sizeof(T) == 4, "pairs are packed FP32");
+    using V = float2;
     using Sm = Smem<T, TY, R>;
     static constexpr int W = TY + 2;      // warps: TY owned rows, A, B
     static constexpr int NT = 32 * W;
@@ -290,33 +308,17 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
 
     static __device__ __forceinline__ V mirror(V v, bool on) { return on ? vmul(v, spl<V>(-1.0)) : v; }
 
-    // Gravity height term of a z face whose lower cell has ghosted index klow.
-    static __device__ __forceinline__ T grav_h(const GridArgs<T> &a, int klow) {
-        return a.k.g * (T(a.nz - 4) * a.k.ds - T(klow - 2) * a.k.ds);
-    }
-
     // NaN-propagating maximum of wave speeds.
     static __device__ __forceinline__ float smax_of(float m, float v) { return max_nan(m, v); }
-    static __device__ __forceinline__ double smax_of(double m, double v) {
-        return (m != m || v != v) ? (m + v) : fmax(m, v);
-    }
 
     // Wave speeds c_s + |v| of the pair's cells in the updated state (the
-    // quantity whose maximum sets the next dt, physics.rs:186-190).  FP32:
-    // the state reduction's own scalar function (fast_speed), so that dt
-    // agrees bit for bit with it; the packed form of the same operations
-    // did not (one unit in the last place on some cells).  FP64: IEEE
-    // square roots.
+    // quantity whose maximum sets the next dt, physics.rs:186-190): the state
+    // reduction's own scalar function (fast_speed), so that dt agrees bit for
+    // bit with it; the packed form of the same operations did not (one unit
+    // in the last place on some cells).
     static __device__ __forceinline__ V speed_pair(const V q[5], const K<T> &k) {
-        if constexpr (sizeof(T) == 4) {
-            return mk(fast_speed(q[0].x, q[1].x, q[2].x, q[3].x, q[4].x, k.gamma),
-                      fast_speed(q[0].y, q[1].y, q[2].y, q[3].y, q[4].y, k.gamma));
-        } else {
-            auto one = [&](T r, T vx, T vy, T vz, T p) {
-                return sqrt(k.gamma * p / r) + sqrt(vx * vx + vy * vy + vz * vz);
-            };
-            return mk(one(q[0].x, q[1].x, q[2].x, q[3].x, q[4].x), one(q[0].y, q[1].y, q[2].y, q[3].y, q[4].y));
-        }
+        return mk(fast_speed(q[0].x, q[1].x, q[2].x, q[3].x, q[4].x, k.gamma),
+                  fast_speed(q[0].y, q[1].y, q[2].y, q[3].y, q[4].y, k.gamma));
     }
 
     // The ghost-cell images of one updated cell (all but the cell itself):
@@ -1012,22 +1014,7 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
 
         const unsigned step = (unsigned)a.ctl->step;
         const T dt = (T)a.ctl->dt[step & 1];
-        t.k.inv_vol = a.k.inv_vol;
-        t.k.gamma = a.k.gamma;
-        t.k.gm1 = a.k.gm1;
-        t.k.kp = T(2) * a.k.inv_gm1;
-        t.k.c1 = T(0.5) * a.k.gm1;
-        t.k.sg = (T)sqrt((double)a.k.gamma);
-        t.k.iv_h = T(0.5) * a.k.inv_vol;
-        t.k.nh4 = T(-2) * dt * a.k.inv_ds;   // -4 dt / (2 ds)
-        {
-            const T scale = dt * a.k.ds * a.k.ds;
-            t.k.sc[0] = t.k.sc[1] = t.k.sc[2] = t.k.sc[3] = T(-0.5) * scale;
-            t.k.sc[4] = T(-0.25) * scale;
-            // wall_heat's factor S / (d/kappa + 1/hc_out) / V, times 4
-            const T ds = a.k.ds;
-            t.k.hq4 = T(4) * ((ds * ds) / ((T(0.008f) / T(0.2f)) + (T(1.0f) / T(10.0f)))) / (ds * ds * ds);
-        }
+        t.k = make_k(a, dt);
         t.gh = t.ghe = spl<V>(0.0);
         if constexpr (GRAV) {
             t.gh = mk(grav_h(a, grav_klow(t.z0 + 2 * lane - 1, a.nz, a.bc[4])), grav_h(a, t.z0 + 2 * lane));
@@ -1074,9 +1061,7 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
             for (int i = 0; i < R; ++i) mbar_inval(&s.bar[i]);
         // min over cells of ds/speed = ds / max speed
         const unsigned nanf = smax != smax;
-        double wmin;
-        if constexpr (sizeof(T) == 4) wmin = nanf ? INFINITY : (double)__fdiv_rn(a.k.ds, smax);
-        else wmin = nanf ? INFINITY : a.k.ds / smax;
+        const double wmin = nanf ? INFINITY : (double)__fdiv_rn(a.k.ds, smax);
         double sum[5] = {0, 0, 0, 0, 0};
         if (block_partial(a, sum, wmin, nanf, tid, NT, s.red, &s.is_last, part_idx, nparts)) {
             __threadfence();
