@@ -10,6 +10,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstring>
 #include <mutex>
 #include <numeric>
@@ -41,7 +42,7 @@ struct GridSlot {
     long long fstride;
     size_t state_bytes;
     void *buf[2];
-    int nitems, item_off;
+    int nitems;
 };
 
 }  // namespace
@@ -52,8 +53,6 @@ struct dg_batch {
     std::vector<GridSlot> g;
     void *arena = nullptr;           // all state buffers
     DevCtl *ctl = nullptr;           // one control block per grid
-    Partial *part = nullptr;         // per work item (and set-up reductions)
-    size_t part_cap = 0;
     GridArgs<float> *d_args[2] = {nullptr, nullptr};   // [parity]: src = buf[parity]
     CUtensorMap *d_maps[2] = {nullptr, nullptr};
     BatchItem *d_items = nullptr;
@@ -127,7 +126,7 @@ GridArgs<float> args_of(const dg_batch *b, int i, int parity) {
     a.k.cfl = (float)s.info.cfl;
     a.k.g = (float)s.info.g;
     a.ctl = b->ctl + i;
-    a.part = b->part + s.item_off;
+    a.part = nullptr;
     return a;
 }
 
@@ -171,12 +170,10 @@ int rebuild(dg_batch *b) {
         GridSlot &s = b->g[i];
         const int tz_n = (s.nz - 4 + kTZs - 1) / kTZs, ty_n = (s.ny - 4 + ty - 1) / ty;
         const int cx_n = (s.nx - 4 + chunk - 1) / chunk;
-        s.item_off = off;
         s.nitems = tz_n * ty_n * cx_n;
-        int local = 0;
         for (int cx = 0; cx < cx_n; ++cx)
             for (int yy = 0; yy < ty_n; ++yy)
-                for (int zz = 0; zz < tz_n; ++zz) items.push_back(BatchItem{i, local++, zz, yy, cx});
+                for (int zz = 0; zz < tz_n; ++zz) items.push_back(BatchItem{i, zz, yy, cx});
         off += s.nitems;
         b->combo_off[combo_of(s.info) + 1] = off;
     }
@@ -186,11 +183,6 @@ int rebuild(dg_batch *b) {
         if (b->d_items) cudaFree(b->d_items);
         b->items_cap = (size_t)b->nitems;
         B_CUDA(b, cudaMalloc(&b->d_items, b->items_cap * sizeof(BatchItem)));
-    }
-    if ((size_t)std::max(b->nitems, kReduceBlocks) > b->part_cap) {
-        if (b->part) cudaFree(b->part);
-        b->part_cap = (size_t)std::max(b->nitems, kReduceBlocks);
-        B_CUDA(b, cudaMalloc(&b->part, b->part_cap * sizeof(Partial)));
     }
     B_CUDA(b, cudaMemcpyAsync(b->d_items, items.data(), items.size() * sizeof(BatchItem), cudaMemcpyHostToDevice,
                               b->stream));
@@ -324,58 +316,36 @@ void choose_orientation(const dg_sim_info &f, bool reorient, int perm[3]) {
     }
 }
 
-// Copies 5 fields between the caller's layout (dense, ghosted sizes cn,
-// velocity / momentum components along the caller's axes) and the stored
-// one (pitched, axes permuted by perm, components likewise).  TO_STORED:
-// caller -> stored; else stored -> caller.  One thread per destination cell.
-template <bool TO_STORED>
-__global__ void permute_fields(const float *src, float *dst, int cn0, int cn1, int cn2, int p0, int p1, int p2,
-                               int pitch, long long fstride) {
-    const int cn[3] = {cn0, cn1, cn2}, p[3] = {p0, p1, p2};
-    const long long ncaller = (long long)cn0 * cn1 * cn2;
-    const int sn0 = cn[p0], sn1 = cn[p1], sn2 = cn[p2];
-    const long long nstored = (long long)sn0 * sn1 * sn2;
-    const long long total = TO_STORED ? nstored : ncaller;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < 5 * total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int f = (int)(t / total);
-        const long long c = t % total;
-        int s[3], q[3];   // stored and caller coordinates
-        if (TO_STORED) {
-            s[2] = (int)(c % sn2);
-            s[1] = (int)(c / sn2 % sn1);
-            s[0] = (int)(c / ((long long)sn2 * sn1));
-            for (int d = 0; d < 3; ++d) q[p[d]] = s[d];
-        } else {
-            q[2] = (int)(c % cn2);
-            q[1] = (int)(c / cn2 % cn1);
-            q[0] = (int)(c / ((long long)cn2 * cn1));
-            for (int d = 0; d < 3; ++d) s[d] = q[p[d]];
-        }
-        // stored component 1 + d is the caller's component 1 + p[d]
-        const int fs = f, fc = (f >= 1 && f <= 3) ? 1 + p[f - 1] : f;
-        const long long ci = ((long long)q[0] * cn1 + q[1]) * cn2 + q[2];
-        const long long si = ((long long)s[0] * sn1 + s[1]) * pitch + s[2];
-        if (TO_STORED) dst[fs * fstride + si] = src[fc * ncaller + ci];
-        else dst[fc * ncaller + ci] = src[fs * fstride + si];
+// Grid s's fields in the caller's layout (dense, the caller's axes and vector
+// components) at base, seen along the stored axes: stored axis d is the
+// caller's perm[d], and stored component 1 + d the caller's 1 + perm[d].
+FieldView<const float> caller_view(const GridSlot &s, const float *base) {
+    const long long cells = (long long)s.cn[0] * s.cn[1] * s.cn[2];
+    const long long stride[3] = {(long long)s.cn[1] * s.cn[2], s.cn[2], 1};
+    FieldView<const float> v;
+    for (int f = 0; f < 5; ++f) v.f[f] = base + (f >= 1 && f <= 3 ? 1 + s.perm[f - 1] : f) * cells;
+    v.sx = stride[s.perm[0]];
+    v.sy = stride[s.perm[1]];
+    v.sz = stride[s.perm[2]];
+    return v;
+}
+
+// Grid s's stored state seen along the caller's axes and components.
+FieldView<const float> stored_view(const GridSlot &s, const float *buf) {
+    const long long stride[3] = {(long long)s.ny * s.pitch, s.pitch, 1};
+    long long c[3];
+    FieldView<const float> v;
+    v.f[0] = buf;
+    v.f[4] = buf + 4 * s.fstride;
+    for (int d = 0; d < 3; ++d) {
+        c[s.perm[d]] = stride[d];
+        v.f[1 + s.perm[d]] = buf + (1 + d) * s.fstride;
     }
+    v.sx = c[0];
+    v.sy = c[1];
+    v.sz = c[2];
+    return v;
 }
-
-int launch_permute(dg_batch *b, const GridSlot &s, bool to_stored, const float *src, float *dst) {
-    const long long cells = 5LL * s.cn[0] * s.cn[1] * s.cn[2];
-    const int threads = 256;
-    const int blocks = (int)std::min<long long>((cells + threads - 1) / threads, 148LL * 16);
-    if (to_stored)
-        permute_fields<true><<<blocks, threads, 0, b->stream>>>(src, dst, s.cn[0], s.cn[1], s.cn[2], s.perm[0],
-                                                                s.perm[1], s.perm[2], s.pitch, s.fstride);
-    else
-        permute_fields<false><<<blocks, threads, 0, b->stream>>>(src, dst, s.cn[0], s.cn[1], s.cn[2], s.perm[0],
-                                                                 s.perm[1], s.perm[2], s.pitch, s.fstride);
-    B_CUDA(b, cudaGetLastError());
-    return DG_OK;
-}
-
-bool identity(const GridSlot &s) { return s.perm[0] == 0 && s.perm[1] == 1 && s.perm[2] == 2; }
 
 }  // namespace
 
@@ -475,7 +445,6 @@ int32_t dg_batch_destroy(dg_batch *b) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
     if (b->arena) cudaFree(b->arena);
     if (b->ctl) cudaFree(b->ctl);
-    if (b->part) cudaFree(b->part);
     for (int p = 0; p < 2; ++p) {
         if (b->d_args[p]) cudaFree(b->d_args[p]);
         if (b->d_maps[p]) cudaFree(b->d_maps[p]);
@@ -494,35 +463,21 @@ int32_t dg_batch_set_primitives(dg_batch *b, int32_t i, const void *const prim[5
     B_CUDA(b, cudaSetDevice(b->device));
     GridSlot &s = b->g[i];
     const int cur = (int)(b->steps & 1);
-    void *stage = s.buf[1 - cur];
     for (int f = 0; f < 5; ++f)
         if (!prim[f]) return bfail(b, DG_ERR_INVALID, "null field");
-    if (identity(s)) {
-        const size_t row = (size_t)s.nz * 4;
-        for (int f = 0; f < 5; ++f)
-            B_CUDA(b, cudaMemcpy2DAsync(static_cast<char *>(stage) + (size_t)f * s.fstride * 4, (size_t)s.pitch * 4,
-                                        prim[f], row, row, (size_t)s.nx * s.ny, cudaMemcpyHostToDevice, b->stream));
-    } else {
-        // the caller's fields, dense, into the other buffer, then permuted
-        // into the stored layout
-        const size_t cells = (size_t)s.cn[0] * s.cn[1] * s.cn[2];
-        float *raw = static_cast<float *>(s.buf[cur]);
-        for (int f = 0; f < 5; ++f)
-            B_CUDA(b, cudaMemcpyAsync(raw + f * cells, prim[f], cells * 4, cudaMemcpyHostToDevice, b->stream));
-        const int r = launch_permute(b, s, true, raw, static_cast<float *>(stage));
-        if (r != DG_OK) return r;
-    }
+    // the caller's fields, dense and each in one contiguous copy, into the
+    // other buffer (row-by-row copies into the pitched layout ran at a fifth
+    // of the link's rate), then converted and permuted into the stored layout
+    const size_t cells = (size_t)s.cn[0] * s.cn[1] * s.cn[2];
+    float *stage = static_cast<float *>(s.buf[1 - cur]);
+    for (int f = 0; f < 5; ++f)
+        B_CUDA(b, cudaMemcpyAsync(stage + f * cells, prim[f], cells * 4, cudaMemcpyHostToDevice, b->stream));
     GridArgs<float> a = args_of(b, i, cur);
-    a.part = b->part;
-    B_CUDA(b, cudaMemsetAsync(a.ctl, 0, sizeof(DevCtl), b->stream));
+    a.dst = static_cast<float *>(s.buf[cur]);
+    B_CUDA(b, cudaMemsetAsync(a.ctl, 0, offsetof(DevCtl, hist), b->stream));
     // the grid's step counter must match the batch's parity: the kernels
     // read dt[step & 1]
-    const unsigned long long st = b->steps;
-    B_CUDA(b, cudaMemcpyAsync(&a.ctl->step, &st, sizeof(st), cudaMemcpyHostToDevice, b->stream));
-    B_CUDA(b, launch_prim_to_cons<float>(a, static_cast<const float *>(stage), s.fstride, s.pitch,
-                                         static_cast<float *>(s.buf[cur]), b->stream));
-    B_CUDA(b, launch_fill_ghosts<float>(a, static_cast<float *>(s.buf[cur]), b->stream));
-    B_CUDA(b, (launch_reduce_policy<float, false>(a, 1, b->stream)));
+    B_CUDA(b, launch_set_state<float>(a, caller_view(s, stage), true, false, b->steps, b->stream));
     B_CUDA(b, cudaStreamSynchronize(b->stream));
     return DG_OK;
 }
@@ -559,24 +514,18 @@ int32_t dg_batch_get_conserved(dg_batch *b, int32_t i, void *const cons[5]) {
     if (!b || !cons || i < 0 || i >= b->n) return bfail(b, DG_ERR_INVALID, "bad argument");
     B_CUDA(b, cudaSetDevice(b->device));
     const GridSlot &s = b->g[i];
-    const char *src = static_cast<const char *>(s.buf[b->steps & 1]);
     for (int f = 0; f < 5; ++f)
         if (!cons[f]) return bfail(b, DG_ERR_INVALID, "null field");
-    if (identity(s)) {
-        const size_t row = (size_t)s.nz * 4;
-        for (int f = 0; f < 5; ++f)
-            B_CUDA(b, cudaMemcpy2DAsync(cons[f], row, src + (size_t)f * s.fstride * 4, (size_t)s.pitch * 4, row,
-                                        (size_t)s.nx * s.ny, cudaMemcpyDeviceToHost, b->stream));
-    } else {
-        // permuted back into the caller's layout in the other buffer (which
-        // the next step overwrites), then copied out dense
-        const size_t cells = (size_t)s.cn[0] * s.cn[1] * s.cn[2];
-        float *raw = static_cast<float *>(s.buf[1 - (b->steps & 1)]);
-        const int r = launch_permute(b, s, false, reinterpret_cast<const float *>(src), raw);
-        if (r != DG_OK) return r;
-        for (int f = 0; f < 5; ++f)
-            B_CUDA(b, cudaMemcpyAsync(cons[f], raw + f * cells, cells * 4, cudaMemcpyDeviceToHost, b->stream));
-    }
+    // dense, in the caller's layout, in the other buffer (which the next step
+    // overwrites), then each field out in one contiguous copy
+    const size_t cells = (size_t)s.cn[0] * s.cn[1] * s.cn[2];
+    float *raw = static_cast<float *>(s.buf[1 - (b->steps & 1)]);
+    float *d[5];
+    for (int f = 0; f < 5; ++f) d[f] = raw + f * cells;
+    B_CUDA(b, launch_get_state<float>(stored_view(s, static_cast<const float *>(s.buf[b->steps & 1])), d, s.cn[0],
+                                      s.cn[1], s.cn[2], b->stream));
+    for (int f = 0; f < 5; ++f)
+        B_CUDA(b, cudaMemcpyAsync(cons[f], d[f], cells * 4, cudaMemcpyDeviceToHost, b->stream));
     B_CUDA(b, cudaStreamSynchronize(b->stream));
     return DG_OK;
 }

@@ -2,10 +2,11 @@
 //
 // A context owns two device copies of the ghosted state (the step reads one
 // and writes the other), the step control block (dt, sums, history) and
-// the per-block partials buffer, plus one TMA descriptor per state buffer.
+// the partials of the sum reduction, plus one TMA descriptor per state buffer.
 #include <cudaTypedefs.h>
 
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -63,95 +64,100 @@ int use_device(dg_ctx *c) {
     return DG_OK;
 }
 
-// Fill ghosts of the current state, then the dt / sums reduction.
-int finish_state(dg_ctx *c) {
-    cudaError_t e;
-    if (c->elem == 8) {
-        auto a = grid_args<double>(c, c->buf[c->cur], c->buf[c->cur]);
-        e = launch_fill_ghosts<double>(a, static_cast<double *>(c->buf[c->cur]), c->stream);
-        if (e == cudaSuccess) e = launch_reduce_policy<double, true>(a, 1, c->stream);
-    } else {
-        auto a = grid_args<float>(c, c->buf[c->cur], c->buf[c->cur]);
-        e = launch_fill_ghosts<float>(a, static_cast<float *>(c->buf[c->cur]), c->stream);
-        if (e == cudaSuccess)
-            e = c->exact ? launch_reduce_policy<float, true>(a, 1, c->stream)
-                         : launch_reduce_policy<float, false>(a, 1, c->stream);
-    }
-    if (e != cudaSuccess) return cuda_fail(c, e, "state set-up kernels");
+// The control fields before the dt history; a launch that timed out may
+// have left its counters half way.
+int reset_ctl(dg_ctx *c) {
+    DG_CUDA(c, cudaMemsetAsync(c->ctl, 0, offsetof(DevCtl, hist), c->stream));
+    return DG_OK;
+}
+
+// Five arrays of the ghosted extents, C order.
+template <class T> FieldView<T> dense_view(const dg_ctx *c, void *const f[5]) {
+    FieldView<T> v;
+    for (int i = 0; i < 5; ++i) v.f[i] = static_cast<T *>(f[i]);
+    v.sx = (long long)c->ny * c->nz;
+    v.sy = c->nz;
+    v.sz = 1;
+    return v;
+}
+
+// Five consecutive dense fields at base.
+struct Fields5 {
+    void *f[5];
+};
+Fields5 consecutive(const dg_ctx *c, const void *base) {
+    const size_t fb = (size_t)c->nx * c->ny * c->nz * c->elem;
+    Fields5 r;
+    for (int i = 0; i < 5; ++i) r.f[i] = const_cast<char *>(static_cast<const char *>(base)) + i * fb;
+    return r;
+}
+
+// A pitched state buffer seen through strides.
+template <class T> FieldView<T> pitched_view(const dg_ctx *c, const void *buf) {
+    FieldView<T> v;
+    for (int i = 0; i < 5; ++i) v.f[i] = const_cast<T *>(static_cast<const T *>(buf)) + i * c->fstride;
+    v.sx = (long long)c->ny * c->pitch;
+    v.sy = c->pitch;
+    v.sz = 1;
+    return v;
+}
+
+// The current state from the dense device fields `src` (NULL: from its own
+// interior), ghosts and the first dt included.
+template <class T> cudaError_t set_state(dg_ctx *c, void *const src[5], bool prims) {
+    const auto a = grid_args<T>(c, c->buf[c->cur], c->buf[c->cur]);
+    const FieldView<const T> v = src ? dense_view<const T>(c, src) : pitched_view<const T>(c, c->buf[c->cur]);
+    return launch_set_state<T>(a, v, prims, c->exact, 0, c->stream);
+}
+
+int finish_state(dg_ctx *c, void *const src[5] = nullptr, bool prims = false) {
+    const cudaError_t e = c->elem == 8 ? set_state<double>(c, src, prims) : set_state<float>(c, src, prims);
+    if (e != cudaSuccess) return cuda_fail(c, e, "state set-up kernel");
     c->has_state = true;
     c->steps = 0;
     return DG_OK;
 }
 
-int reset_ctl(dg_ctx *c) {
-    DG_CUDA(c, cudaMemsetAsync(c->ctl, 0, sizeof(DevCtl), c->stream));
-    return DG_OK;
-}
-
-// Copy 5 dense host/device fields (n^3 each) into the pitched buffer dst.
-int copy_in(dg_ctx *c, void *dst, const void *const src[5], cudaMemcpyKind kind) {
-    const size_t row = (size_t)c->nz * c->elem;
-    for (int f = 0; f < 5; ++f) {
-        if (!src[f]) return fail(c, DG_ERR_INVALID, "null field pointer");
-        char *d = static_cast<char *>(dst) + (size_t)f * c->fstride * c->elem;
-        DG_CUDA(c, cudaMemcpy2DAsync(d, (size_t)c->pitch * c->elem, src[f], row, row, (size_t)c->nx * c->ny, kind,
-                                     c->stream));
-    }
-    return DG_OK;
+bool null_field(const void *const f[5]) {
+    for (int i = 0; i < 5; ++i)
+        if (!f[i]) return true;
+    return false;
 }
 
 // Host transfers move each field as one contiguous copy (the copy engines'
 // fast case; row-by-row copies of the pitched layout from host memory run
-// at about half the rate) through a dense device copy of the fields; the
-// re-pitch between the dense and the pitched layout is a device-to-device
-// copy.
+// at about half the rate) through a dense device copy of the fields.
 size_t dense_field_bytes(const dg_ctx *c) { return (size_t)c->nx * c->ny * c->nz * c->elem; }
 
 int upload_dense(dg_ctx *c, void *dense, const void *const src[5]) {
     const size_t fb = dense_field_bytes(c);
-    for (int f = 0; f < 5; ++f) {
-        if (!src[f]) return fail(c, DG_ERR_INVALID, "null field pointer");
+    for (int f = 0; f < 5; ++f)
         DG_CUDA(c, cudaMemcpyAsync(static_cast<char *>(dense) + f * fb, src[f], fb, cudaMemcpyHostToDevice,
                                    c->stream));
-    }
     return DG_OK;
 }
 
 int download_dense(dg_ctx *c, void *const dst[5], const void *dense) {
     const size_t fb = dense_field_bytes(c);
-    for (int f = 0; f < 5; ++f) {
-        if (!dst[f]) return fail(c, DG_ERR_INVALID, "null field pointer");
+    for (int f = 0; f < 5; ++f)
         DG_CUDA(c, cudaMemcpyAsync(dst[f], static_cast<const char *>(dense) + f * fb, fb, cudaMemcpyDeviceToHost,
                                    c->stream));
-    }
     return DG_OK;
 }
 
-// dense <-> pitched, on the device
-int repitch(dg_ctx *c, void *dst, const void *src, bool to_pitched) {
-    const size_t row = (size_t)c->nz * c->elem, fb = dense_field_bytes(c);
-    const size_t pitched = (size_t)c->pitch * c->elem;
-    for (int f = 0; f < 5; ++f) {
-        const size_t po = (size_t)f * c->fstride * c->elem;
-        if (to_pitched)
-            DG_CUDA(c, cudaMemcpy2DAsync(static_cast<char *>(dst) + po, pitched, static_cast<const char *>(src) + f * fb,
-                                         row, row, (size_t)c->nx * c->ny, cudaMemcpyDeviceToDevice, c->stream));
-        else
-            DG_CUDA(c, cudaMemcpy2DAsync(static_cast<char *>(dst) + f * fb, row, static_cast<const char *>(src) + po,
-                                         pitched, row, (size_t)c->nx * c->ny, cudaMemcpyDeviceToDevice, c->stream));
+// The current state into dense device fields.
+int get_state(dg_ctx *c, void *const dst[5]) {
+    cudaError_t e;
+    if (c->elem == 8) {
+        double *d[5];
+        for (int f = 0; f < 5; ++f) d[f] = static_cast<double *>(dst[f]);
+        e = launch_get_state<double>(pitched_view<const double>(c, c->buf[c->cur]), d, c->nx, c->ny, c->nz, c->stream);
+    } else {
+        float *d[5];
+        for (int f = 0; f < 5; ++f) d[f] = static_cast<float *>(dst[f]);
+        e = launch_get_state<float>(pitched_view<const float>(c, c->buf[c->cur]), d, c->nx, c->ny, c->nz, c->stream);
     }
-    return DG_OK;
-}
-
-int copy_out(dg_ctx *c, void *const dst[5], const void *src, cudaMemcpyKind kind) {
-    const size_t row = (size_t)c->nz * c->elem;
-    for (int f = 0; f < 5; ++f) {
-        if (!dst[f]) return fail(c, DG_ERR_INVALID, "null field pointer");
-        const char *s = static_cast<const char *>(src) + (size_t)f * c->fstride * c->elem;
-        DG_CUDA(c, cudaMemcpy2DAsync(dst[f], row, s, (size_t)c->pitch * c->elem, row, (size_t)c->nx * c->ny, kind,
-                                     c->stream));
-    }
-    return DG_OK;
+    return e == cudaSuccess ? DG_OK : cuda_fail(c, e, "state copy kernel");
 }
 
 int check_flags(dg_ctx *c) {
@@ -285,19 +291,12 @@ int32_t dg_create(const dg_sim_info *info, dg_ctx **out) {
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMalloc(&c->buf[i], c->state_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&c->ctl, sizeof(DevCtl));
-    if (e == cudaSuccess) {
-        const int ty = step_tile_rows(c->kind), tzc = step_tile_cols(c->kind);
-        long long tiles = (long long)((c->ny - 4 + ty - 1) / ty) * ((c->nz - 4 + tzc - 1) / tzc);
-        long long cap = tiles * (c->nx - 4);   // chunk >= 1
-        if (cap < kReduceBlocks) cap = kReduceBlocks;
-        c->part_cap = (int)cap;
-        e = cudaMalloc(&c->part, (size_t)cap * sizeof(Partial));
-    }
+    if (e == cudaSuccess) e = cudaMalloc(&c->part, kReduceBlocks * sizeof(Partial));
     if (e != cudaSuccess) { c->err = std::string("device allocation: ") + cudaGetErrorString(e); return bail(DG_ERR_CUDA); }
     for (int i = 0; i < 2; ++i)
         if (encode_map(c, i) != DG_OK) return bail(DG_ERR_CUDA);
-    if (reset_ctl(c) != DG_OK) return bail(DG_ERR_CUDA);
-    if (cudaMemsetAsync(c->buf[0], 0, c->state_bytes, c->stream) != cudaSuccess ||
+    if (cudaMemsetAsync(c->ctl, 0, sizeof(DevCtl), c->stream) != cudaSuccess ||
+        cudaMemsetAsync(c->buf[0], 0, c->state_bytes, c->stream) != cudaSuccess ||
         cudaMemsetAsync(c->buf[1], 0, c->state_bytes, c->stream) != cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess) {
         c->err = "initial memset failed";
@@ -321,50 +320,39 @@ int32_t dg_destroy(dg_ctx *c) {
     return DG_OK;
 }
 
-int32_t dg_set_conserved(dg_ctx *c, const void *const cons[5]) {
-    if (!c || !cons) return fail(c, DG_ERR_INVALID, "null argument");
+// A state from host fields: the dense upload into the other state buffer,
+// then the set-up kernel from there.
+static int set_from_host(dg_ctx *c, const void *const src[5], bool prims) {
+    if (null_field(src)) return fail(c, DG_ERR_INVALID, "null field pointer");
     int r;
     if ((r = use_device(c)) != DG_OK) return r;
     if ((r = reset_ctl(c)) != DG_OK) return r;
-    // the other state buffer holds the dense upload
-    if ((r = upload_dense(c, c->buf[1 - c->cur], cons)) != DG_OK) return r;
-    if ((r = repitch(c, c->buf[c->cur], c->buf[1 - c->cur], true)) != DG_OK) return r;
-    if ((r = finish_state(c)) != DG_OK) return r;
+    void *stage = c->buf[1 - c->cur];
+    if ((r = upload_dense(c, stage, src)) != DG_OK) return r;
+    if ((r = finish_state(c, consecutive(c, stage).f, prims)) != DG_OK) return r;
     return check_flags(c);
+}
+
+int32_t dg_set_conserved(dg_ctx *c, const void *const cons[5]) {
+    if (!c || !cons) return fail(c, DG_ERR_INVALID, "null argument");
+    return set_from_host(c, cons, false);
 }
 
 int32_t dg_set_conserved_device(dg_ctx *c, const void *const cons[5]) {
     if (!c || !cons) return fail(c, DG_ERR_INVALID, "null argument");
+    if (null_field(cons)) return fail(c, DG_ERR_INVALID, "null field pointer");
     int r;
     if ((r = use_device(c)) != DG_OK) return r;
     if ((r = reset_ctl(c)) != DG_OK) return r;
-    if ((r = copy_in(c, c->buf[c->cur], cons, cudaMemcpyDeviceToDevice)) != DG_OK) return r;
-    if ((r = finish_state(c)) != DG_OK) return r;
+    void *src[5];
+    for (int f = 0; f < 5; ++f) src[f] = const_cast<void *>(cons[f]);
+    if ((r = finish_state(c, src)) != DG_OK) return r;
     return check_flags(c);
 }
 
 int32_t dg_set_primitives(dg_ctx *c, const void *const prim[5]) {
     if (!c || !prim) return fail(c, DG_ERR_INVALID, "null argument");
-    int r;
-    if ((r = use_device(c)) != DG_OK) return r;
-    if ((r = reset_ctl(c)) != DG_OK) return r;
-    // stage the primitives densely in the other state buffer, convert into the current one
-    void *stage = c->buf[1 - c->cur];
-    if ((r = upload_dense(c, stage, prim)) != DG_OK) return r;
-    const long long dfs = (long long)c->nx * c->ny * c->nz;
-    cudaError_t e;
-    if (c->elem == 8) {
-        auto a = grid_args<double>(c, stage, c->buf[c->cur]);
-        e = launch_prim_to_cons<double>(a, static_cast<const double *>(stage), dfs, c->nz,
-                                        static_cast<double *>(c->buf[c->cur]), c->stream);
-    } else {
-        auto a = grid_args<float>(c, stage, c->buf[c->cur]);
-        e = launch_prim_to_cons<float>(a, static_cast<const float *>(stage), dfs, c->nz,
-                                       static_cast<float *>(c->buf[c->cur]), c->stream);
-    }
-    if (e != cudaSuccess) return cuda_fail(c, e, "prim_to_cons");
-    if ((r = finish_state(c)) != DG_OK) return r;
-    return check_flags(c);
+    return set_from_host(c, prim, true);
 }
 
 int32_t dg_enqueue_steps(dg_ctx *c, int32_t nsteps) {
@@ -434,11 +422,12 @@ int32_t dg_compute_step_dt(dg_ctx *c, double dt) {
 
 int32_t dg_get_conserved(dg_ctx *c, void *const cons[5]) {
     if (!c || !cons) return fail(c, DG_ERR_INVALID, "null argument");
+    if (null_field(cons)) return fail(c, DG_ERR_INVALID, "null field pointer");
     if (!c->has_state) return fail(c, DG_ERR_NO_STATE, "no state set");
     int r;
     if ((r = use_device(c)) != DG_OK) return r;
     if (!c->prim_scratch) DG_CUDA(c, cudaMalloc(&c->prim_scratch, c->state_bytes));
-    if ((r = repitch(c, c->prim_scratch, c->buf[c->cur], false)) != DG_OK) return r;
+    if ((r = get_state(c, consecutive(c, c->prim_scratch).f)) != DG_OK) return r;
     if ((r = download_dense(c, cons, c->prim_scratch)) != DG_OK) return r;
     DG_CUDA(c, cudaStreamSynchronize(c->stream));
     return DG_OK;
@@ -446,10 +435,11 @@ int32_t dg_get_conserved(dg_ctx *c, void *const cons[5]) {
 
 int32_t dg_get_conserved_device(dg_ctx *c, void *const cons[5]) {
     if (!c || !cons) return fail(c, DG_ERR_INVALID, "null argument");
+    if (null_field(cons)) return fail(c, DG_ERR_INVALID, "null field pointer");
     if (!c->has_state) return fail(c, DG_ERR_NO_STATE, "no state set");
     int r;
     if ((r = use_device(c)) != DG_OK) return r;
-    if ((r = copy_out(c, cons, c->buf[c->cur], cudaMemcpyDeviceToDevice)) != DG_OK) return r;
+    if ((r = get_state(c, cons)) != DG_OK) return r;
     // the destination belongs to the caller's streams: return after the copies
     DG_CUDA(c, cudaStreamSynchronize(c->stream));
     return DG_OK;
@@ -457,6 +447,7 @@ int32_t dg_get_conserved_device(dg_ctx *c, void *const cons[5]) {
 
 int32_t dg_get_primitives(dg_ctx *c, void *const prim[5]) {
     if (!c || !prim) return fail(c, DG_ERR_INVALID, "null argument");
+    if (null_field(prim)) return fail(c, DG_ERR_INVALID, "null field pointer");
     if (!c->has_state) return fail(c, DG_ERR_NO_STATE, "no state set");
     int r;
     if ((r = use_device(c)) != DG_OK) return r;
@@ -490,14 +481,8 @@ int32_t dg_conservation_sums(dg_ctx *c, double out[5]) {
     int r;
     if ((r = use_device(c)) != DG_OK) return r;
     // FP64 sums of the current state, reduced on the device in a fixed order
-    cudaError_t e;
-    if (c->elem == 8) {
-        e = launch_reduce_policy<double, true>(grid_args<double>(c, c->buf[c->cur], nullptr), 0, c->stream);
-    } else {
-        auto a = grid_args<float>(c, c->buf[c->cur], nullptr);
-        e = c->exact ? launch_reduce_policy<float, true>(a, 0, c->stream)
-                     : launch_reduce_policy<float, false>(a, 0, c->stream);
-    }
+    const cudaError_t e = c->elem == 8 ? launch_sums(grid_args<double>(c, c->buf[c->cur], nullptr), c->stream)
+                                       : launch_sums(grid_args<float>(c, c->buf[c->cur], nullptr), c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "sum reduction");
     DG_CUDA(c, cudaMemcpyAsync(out, c->ctl->sums, 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     DG_CUDA(c, cudaStreamSynchronize(c->stream));

@@ -127,107 +127,65 @@ __host__ __device__ __forceinline__ int axis_source(int g, int n, int lo, int hi
     return g == n - 2 ? n - 3 : n - 4;
 }
 
-// Modes of final_reduce.
-enum ReduceMode { kSumsOnly = 0, kSetDt = 1, kAdvance = 2 };
-
-template <class T>
-__device__ void final_reduce(const GridArgs<T> &a, int tid, int nt, double *red, int mode, int nb);
-
-// Block-level reduction of (sums, min wave time, NaN flag) into
-// a.part[idx] in a fixed order.  Returns true, in every thread, in the last
-// of the nb blocks (work items) of this grid to finish.
-template <class T>
-__device__ bool block_partial(const GridArgs<T> &a, double sum[5], double wm, unsigned nanf, int tid, int nt,
-                              double *red, int *is_last, int idx, int nb) {
+// Wave speeds (>= 0, or NaN) as unsigned keys of the same order, NaN on top.
+__device__ __forceinline__ unsigned long long speed_key(float v) {
+    return v != v ? 0x7fffffffull : (unsigned long long)(__float_as_uint(v) & 0x7fffffffu);
+}
+__device__ __forceinline__ unsigned long long speed_key(double v) {
+    return v != v ? 0x7fffffffffffffffull : (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+__device__ __forceinline__ void key_speed(unsigned long long k, float &v) { v = __uint_as_float((unsigned)k); }
+__device__ __forceinline__ void key_speed(unsigned long long k, double &v) { v = __longlong_as_double((long long)k); }
+__device__ __forceinline__ unsigned long long warp_max(float v) {
+    return __reduce_max_sync(0xffffffffu, (unsigned)speed_key(v));
+}
+__device__ __forceinline__ unsigned long long warp_max(double v) {
+    unsigned long long k = speed_key(v);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int f = 0; f < 5; ++f) sum[f] += __shfl_xor_sync(0xffffffffu, sum[f], o);
-        wm = fmin(wm, __shfl_xor_sync(0xffffffffu, wm, o));
-        nanf |= __shfl_xor_sync(0xffffffffu, nanf, o);
+        const unsigned long long n = __shfl_xor_sync(0xffffffffu, k, o);
+        k = n > k ? n : k;
     }
-    const int warp = tid >> 5, lane = tid & 31;
-    if (lane == 0) {
-        for (int f = 0; f < 5; ++f) red[warp * 7 + f] = sum[f];
-        red[warp * 7 + 5] = wm;
-        red[warp * 7 + 6] = (double)nanf;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        Partial p;
-        for (int f = 0; f < 5; ++f) p.sums[f] = 0;
-        p.wmin = INFINITY;
-        p.nan = 0;
-        for (int w = 0; w < nt / 32; ++w) {
-            for (int f = 0; f < 5; ++f) p.sums[f] += red[w * 7 + f];
-            p.wmin = fmin(p.wmin, red[w * 7 + 5]);
-            p.nan |= red[w * 7 + 6] != 0.0;
-        }
-        p.pad = 0;
-        a.part[idx] = p;
-        __threadfence();
-        const unsigned ticket = atomicAdd(&a.ctl->counter, 1u);
-        *is_last = ticket == (unsigned)nb - 1;
-    }
-    __syncthreads();
-    return *is_last != 0;
+    return k;
 }
 
-// Fixed-order reduction of a launch's partials by its last block.
-// kAdvance: a step finished -> record its dt, set the next dt, step += 1;
-// kSetDt: a state was just set -> dt of the coming step; kSumsOnly: sums.
-template <class T>
-__device__ void final_reduce(const GridArgs<T> &a, int tid, int nt, double *red, int mode, int nb) {
-    double acc[5] = {0, 0, 0, 0, 0};
-    double wm = INFINITY;
-    unsigned nanf = 0;
-    for (int b = tid; b < nb; b += nt) {
-        const volatile Partial *p = a.part + b;
-        for (int f = 0; f < 5; ++f) acc[f] += p->sums[f];
-        wm = fmin(wm, p->wmin);
-        nanf |= p->nan;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int f = 0; f < 5; ++f) acc[f] += __shfl_xor_sync(0xffffffffu, acc[f], o);
-        wm = fmin(wm, __shfl_xor_sync(0xffffffffu, wm, o));
-        nanf |= __shfl_xor_sync(0xffffffffu, nanf, o);
-    }
-    const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
+// The launch's largest wave speed, and by its last block (of the nb of this
+// grid) the next dt: calc_timestep's CFL * min(ds / speed) is CFL * (ds / max
+// speed), division being monotone, or CFL * 1.0 when a NaN was seen
+// (physics.rs:191-195).  A maximum does not depend on its order, so one
+// atomic per warp in shared memory and one per block in the control block
+// replace partial results; s_max is zeroed before a barrier that precedes
+// the call.  ADVANCE: a step finished (record its dt, advance the counter);
+// else a state was set before step `step`.
+template <bool ADVANCE, class T>
+__device__ __forceinline__ void finish_speed(const GridArgs<T> &a, T smax, unsigned long long *s_max, int nb,
+                                             unsigned long long step = 0) {
+    const unsigned long long k = warp_max(smax);
+    if ((threadIdx.x & 31) == 0) atomicMax(s_max, k);
     __syncthreads();
-    if (lane == 0) {
-        for (int f = 0; f < 5; ++f) red[warp * 7 + f] = acc[f];
-        red[warp * 7 + 5] = wm;
-        red[warp * 7 + 6] = (double)nanf;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        double tot[5] = {0, 0, 0, 0, 0};
-        double w = INFINITY;
-        unsigned nn = 0;
-        for (int i = 0; i < nw; ++i) {
-            for (int f = 0; f < 5; ++f) tot[f] += red[i * 7 + f];
-            w = fmin(w, red[i * 7 + 5]);
-            nn |= red[i * 7 + 6] != 0.0;
-        }
-        DevCtl *c = a.ctl;
+    if (threadIdx.x != 0) return;
+    DevCtl *c = a.ctl;
+    atomicMax(&c->wmax, *s_max);
+    __threadfence();
+    if (atomicAdd(&c->counter, 1u) != (unsigned)nb - 1) return;
+    __threadfence();
+    T m;
+    key_speed(atomicExch(&c->wmax, 0ull), m);
+    const bool nan = m != m;
+    const T dtn = nan ? a.k.cfl * T(1.0) : a.k.cfl * (a.k.ds / m);
+    if constexpr (ADVANCE) {
         const unsigned long long st = c->step;
-        // calc_timestep: CFL * min, or CFL * 1.0 when a NaN was seen
-        // (physics.rs:191-195), evaluated in the step's precision.
-        const T dtn = nn ? (T)a.k.cfl * T(1.0) : (T)a.k.cfl * (T)w;
-        for (int f = 0; f < 5; ++f) c->sums[f] = tot[f];
-        if (mode != kSumsOnly && nn) c->flags |= kStatusNonFinite;
-        if (mode == kAdvance) {
-            c->hist[st % kHist] = c->dt[st & 1];
-            c->dt[(st + 1) & 1] = (double)dtn;
-            c->step = st + 1;
-        } else if (mode == kSetDt) {
-            c->dt[st & 1] = (double)dtn;
-        }
-        c->counter = 0;
-        __threadfence();
+        c->hist[st % kHist] = c->dt[st & 1];
+        c->dt[(st + 1) & 1] = (double)dtn;
+        c->step = st + 1;
+        if (nan) c->flags |= kStatusNonFinite;
+    } else {
+        c->dt[step & 1] = (double)dtn;
+        c->step = step;
+        c->flags = nan ? kStatusNonFinite : 0u;
     }
+    c->counter = 0;
+    __threadfence();
 }
 
 }  // namespace dg

@@ -19,7 +19,6 @@ struct dg_ctx {
     unsigned long long steps;  // steps since the state was set
     dg::DevCtl *ctl;
     dg::Partial *part;
-    int part_cap;
     void *prim_scratch;        // lazily allocated: dense primitives for dg_get_primitives
     CUtensorMap tmap[2];
     cudaStream_t stream;

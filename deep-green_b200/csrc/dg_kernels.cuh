@@ -24,18 +24,23 @@ struct DevCtl {
     unsigned long long step;   // steps completed since the state was set
     unsigned int counter;      // blocks of the running launch that finished
     unsigned int flags;        // sticky status bits (kStatus*)
+    unsigned long long wmax;   // largest wave speed of the running launch so far (bits; 0 between launches)
     double dt[2];
     double sums[5];            // FP64 interior sums of the current state
     double hist[kHist];        // dt used by step s at hist[s % kHist]
 };
 
-// Per-block partial results of a launch, reduced in a fixed order by the
-// launch's last block (deterministic sums).
+// Per-block partial sums, added in a fixed order by the launch's last block.
 struct Partial {
     double sums[5];
-    double wmin;               // min over the block's cells of ds/(c_s+|v|)
-    unsigned int nan;
-    unsigned int pad;
+};
+
+// Where the five fields of a state live outside the pitched buffers: base
+// pointers in the grid's field order and element strides along the grid's
+// axes.
+template <class T> struct FieldView {
+    T *f[5];
+    long long sx, sy, sz;
 };
 
 // Geometry and physics of one grid as the kernels see it.
@@ -53,7 +58,7 @@ template <class T> struct GridArgs {
     long long wait_budget;     // SM clocks a wait for a staged plane may take (kWaitBudget)
     Consts<T> k;
     DevCtl *ctl;
-    Partial *part;
+    Partial *part;             // conservation sums only (kReduceBlocks entries)
 };
 
 // Boundary types of dg_sim_info (DG_BC_*) into the kernels' form.  A
@@ -185,6 +190,23 @@ inline long long sweep_makespan(long long tiles, int nxi, int chunk) {
     return end;
 }
 
+// The split of x into chunks that minimises waves x (planes per block + 3
+// re-staged), at least 24 planes per block unless no more than `small` blocks
+// come of it.
+inline int waves_chunk(long long tiles, int nxi, long long small) {
+    const int maxc = nxi / 24 > 0 ? nxi / 24 : 1;
+    long long best = -1;
+    int bestc = 1;
+    for (int c = 1; c <= nxi && c <= 64; ++c) {
+        if (c > maxc && tiles * c > small) break;
+        const long long per = (nxi + c - 1) / c;
+        const long long waves = (tiles * c + kSms - 1) / kSms;
+        const long long cost = waves * (per + 3);
+        if (best < 0 || cost < best) { best = cost; bestc = c; }
+    }
+    return (nxi + bestc - 1) / bestc;
+}
+
 // Default x-planes per block (one block per SM).  The packed sweep with
 // interior tiles that fill the SMs: the frame launch's chunk (the interior
 // launch marches whole columns); with fewer interior tiles: the split of x that
@@ -205,17 +227,7 @@ inline int choose_chunk(int nx, int ny, int nz, int kind) {
     const long long tiles = (long long)((ny - 4 + ty - 1) / ty) * ((nz - 4 + tzc - 1) / tzc);
     const int nxi = nx - 4;
     if (is_sweep(kind) && InteriorTiles(ny, nz, ty, tzc).interior() > 0) {
-        const int maxc = nxi / 24 > 0 ? nxi / 24 : 1;
-        long long best = -1;
-        int bestc = 1;
-        for (int c = 1; c <= nxi && c <= 64; ++c) {
-            if (c > maxc && tiles * c > 4 * kSms) break;
-            const long long per = (nxi + c - 1) / c;
-            const long long waves = (tiles * c + kSms - 1) / kSms;
-            const long long cost = waves * (per + 3);
-            if (best < 0 || cost < best) { best = cost; bestc = c; }
-        }
-        return (nxi + bestc - 1) / bestc;
+        return waves_chunk(tiles, nxi, 4 * kSms);
     }
     int bestp = nxi;
     long long best = sweep_makespan(tiles, nxi, nxi);
@@ -233,7 +245,7 @@ inline int choose_chunk(int nx, int ny, int nz, int kind) {
 // Launch helpers.  EXACT selects the reference-rounding policy
 // (dg_step_ref.cu, built with --fmad=false) or the fast one
 // (dg_step_fast.cu); float/fast, float/exact and double/exact exist.
-template <class T, bool EXACT> cudaError_t launch_reduce_policy(const GridArgs<T> &a, int set_dt, cudaStream_t st);
+template <class T> cudaError_t launch_sums(const GridArgs<T> &a, cudaStream_t st);
 template <class T, bool EXACT>
 cudaError_t launch_cons_to_prim_policy(const GridArgs<T> &a, const T *cons, T *prim, long long prim_fstride,
                                        int prim_pitch, cudaStream_t st);
@@ -245,9 +257,16 @@ void set_global_error(const std::string &msg);
 cudaError_t launch_sweep(const GridArgs<float> &a, const CUtensorMap *tmap_src, int chunk, cudaStream_t st);
 cudaError_t launch_march(const GridArgs<float> &a, const CUtensorMap *tmap_src, int kind, int chunk, cudaStream_t st);
 cudaError_t launch_march(const GridArgs<double> &a, const CUtensorMap *tmap_src, int kind, int chunk, cudaStream_t st);
-template <class T> cudaError_t launch_fill_ghosts(const GridArgs<T> &a, T *buf, cudaStream_t st);
+// A state from src into a.dst with its ghosts, the dt of the coming step
+// (number `step`) and a fresh control block.  prims: src holds primitives;
+// exact: the wave speeds round like the reference (FP64 always does).  src
+// may be a.dst itself: then only the ghosts are written.
 template <class T>
-cudaError_t launch_prim_to_cons(const GridArgs<T> &a, const T *prim, long long prim_fstride, int prim_pitch, T *cons,
-                                cudaStream_t st);
+cudaError_t launch_set_state(const GridArgs<T> &a, const FieldView<const T> &src, bool prims, bool exact,
+                             unsigned long long step, cudaStream_t st);
+// The state at src (a's fields through the view's strides) as five dense
+// arrays of n0 x n1 x n2 cells.
+template <class T>
+cudaError_t launch_get_state(const FieldView<const T> &src, T *const dst[5], int n0, int n1, int n2, cudaStream_t st);
 
 }  // namespace dg

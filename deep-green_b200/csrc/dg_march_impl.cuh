@@ -318,10 +318,9 @@ template <class T, int TY, int R> struct Smem {
     T zex[2][TY][5];                                      // last column's xt (wall) or lower state (outflow)
     T fzr[2][TY][5];                                      // flux of the right edge face
     uint64_t bar[R];
-    double red[(TY + 2) * 7];
+    unsigned long long wmax;                              // finish_speed
     int abort_flag[2];                                    // by plane parity
     int skip;
-    int is_last;
 };
 
 template <class T, class P, int TY, int R, int LIM, bool GRAV> struct March {
@@ -825,6 +824,7 @@ template <class T, class P, int TY, int R, int LIM, bool GRAV> struct March {
         if (tid == 0) {
             s.skip = (*(volatile unsigned *)&a.ctl->flags & kStatusTimeout) != 0;
             s.abort_flag[0] = s.abort_flag[1] = 0;
+            s.wmax = 0;
             if (!s.skip) {
                 for (int i = 0; i < R; ++i) mbar_init(&s.bar[i], 1);
                 fence_mbar_init();
@@ -853,14 +853,7 @@ template <class T, class P, int TY, int R, int LIM, bool GRAV> struct March {
             }
             return;
         }
-        // min over cells of ds / speed = ds / max speed
-        const unsigned nanf = smax != smax;
-        const double wmin = nanf ? INFINITY : (double)(a.k.ds / smax);
-        double sum[5] = {0, 0, 0, 0, 0};
-        if (block_partial(a, sum, wmin, nanf, tid, NT, s.red, &s.is_last, blockIdx.x, gridDim.x)) {
-            __threadfence();
-            final_reduce<T>(a, tid, NT, s.red, kAdvance, gridDim.x);
-        }
+        finish_speed<true>(a, smax, &s.wmax, gridDim.x);
     }
 };
 

@@ -12,9 +12,8 @@
 // reductions) lives in a fixed-size array in the library's own device image.
 //
 // Limits and rules:
-//   * the scratch array holds the control block plus kMaxBlocks per-block
-//     partials (1 MiB in total); grids that need more blocks are rejected
-//     with DG_ERR_INVALID;
+//   * the scratch array is 1 MiB; grids that need more than kMaxBlocks
+//     blocks are rejected with DG_ERR_INVALID;
 //   * every GPU that loads the library holds this 1 MiB until the process
 //     exits;
 //   * all calls share the one array (per device): calls that overlap on the
@@ -39,7 +38,10 @@ namespace {
 
 constexpr size_t kNoAllocScratchBytes = 1u << 20;
 constexpr size_t kPartialOffset = (sizeof(DevCtl) + 255) / 256 * 256;
-constexpr int kMaxBlocks = (int)((kNoAllocScratchBytes - kPartialOffset) / sizeof(Partial));
+// Blocks a step may have: the scratch once held 64 bytes of partial results
+// per block, and the limit on a grid's size stays what that made it.
+constexpr int kMaxBlocks = (int)((kNoAllocScratchBytes - kPartialOffset) / 64);
+static_assert((kNoAllocScratchBytes - kPartialOffset) / sizeof(Partial) >= kReduceBlocks, "partials of the sums");
 
 // The scratch.  In host code this name is only a stand-in for the device
 // symbol: its device address comes from cudaGetSymbolAddress below.
@@ -114,21 +116,28 @@ GridArgs<T> args_for(const dg_sim_info *info, const void *src, void *dst, void *
     return a;
 }
 
-// The block count that decides whether a grid fits the scratch.  For the
-// one-cell-per-lane kernels it is counted in 32 x 4 (FP64 reference rounding),
-// 32 x 8 (FP32) or 64 x 4 tiles, the sizes this entry point's limit was first
-// set by: those kernels need fewer blocks now, and a caller that sizes its
-// grids by the limit keeps the same answer.
+// The block count that decides whether a grid fits the scratch: that of the
+// kernels and splits this entry point's limit was first set by (32 x 4 or 32
+// x 8 tiles with the reference's rounding, 64-column tiles of 14 or 4 rows
+// with fused arithmetic, at least 20 or 24 planes per block).  A step needs
+// no memory per block now; a caller that sizes its grids by the limit keeps
+// the same answer.
 long long limit_blocks(const dg_sim_info *info, int kind) {
-    if (kind == kFastF32) return 0;
-    const long long rows = kind == kRefF32 ? 8 : 4, cols = kind == kFastF64 ? 64 : 32, nx = info->nx;
-    const long long ty = (info->ny + rows - 1) / rows, tz = (info->nz + cols - 1) / cols, tiles = ty * tz;
-    if (kind != kFastF64) {
-        const long long want = (2LL * kSms * 14 + tiles - 1) / tiles, most = std::max<long long>(1, nx / 20);
-        const long long per = (nx + std::min(want, most) - 1) / std::max<long long>(1, std::min(want, most));
-        return tiles * ((nx + per - 1) / per);
+    const int nx = info->nx;
+    if (kind == kFastF32 || kind == kFastF64) {
+        const int rows = kind == kFastF32 ? 14 : 4;
+        const InteriorTiles it(info->ny + 4, info->nz + 4, rows, 64);
+        const long long tiles = (long long)it.tiles_y * it.tiles_z;
+        const bool columns = it.interior() >= kSms;
+        const int chunk = columns ? std::min(nx, 64) : waves_chunk(tiles, nx, 0);
+        const long long chunks = (nx + chunk - 1) / chunk;
+        return (long long)it.interior() * (columns ? 1 : chunks) + it.frame() * chunks;
     }
-    return tiles;
+    const long long rows = kind == kRefF32 ? 8 : 4;
+    const long long tiles = (info->ny + rows - 1) / rows * ((info->nz + 31) / 32);
+    const long long want = (2LL * kSms * 14 + tiles - 1) / tiles, most = std::max(1, nx / 20);
+    const long long chunks = std::min(want, most), per = (nx + chunks - 1) / chunks;
+    return tiles * ((nx + per - 1) / per);
 }
 
 template <class T>
@@ -136,13 +145,9 @@ int run(const dg_sim_info *info, int kind, void *cons_in, void *cons_out, double
         void *scratch) {
     const int elem = (int)sizeof(T);
     GridArgs<T> a = args_for<T>(info, cons_in, cons_out, scratch);
-    int chunk = choose_chunk(a.nx, a.ny, a.nz, kind);
-    // a split with more blocks than the scratch has partials gives way to
-    // whole columns
-    if (step_grid_blocks(a.nx, a.ny, a.nz, kind, chunk) > kMaxBlocks) chunk = a.nx - 4;
-    const long long blocks = std::max<long long>(limit_blocks(info, kind),
-                                                 step_grid_blocks(a.nx, a.ny, a.nz, kind, chunk));
-    if (blocks > kMaxBlocks || kReduceBlocks > kMaxBlocks)
+    const int chunk = choose_chunk(a.nx, a.ny, a.nz, kind);
+    const long long blocks = limit_blocks(info, kind);
+    if (blocks > kMaxBlocks)
         return fail(DG_ERR_INVALID, "grid too large for the no-allocation scratch (" + std::to_string(blocks) +
                                         " blocks > " + std::to_string(kMaxBlocks) + ")");
     auto fn = encode_fn();
@@ -161,30 +166,31 @@ int run(const dg_sim_info *info, int kind, void *cons_in, void *cons_out, double
 
     // the control fields of the scratch must start at zero on every call
     cudaError_t e = cudaMemsetAsync(scratch, 0, offsetof(DevCtl, hist), st);
-    if (e == cudaSuccess) e = launch_fill_ghosts<T>(a, static_cast<T *>(cons_in), st);
-    if constexpr (sizeof(T) == 4) {
-        if (kind == kFastF32) {
-            if (e == cudaSuccess) e = launch_reduce_policy<float, false>(a, 1, st);
-            if (e == cudaSuccess) e = launch_sweep(a, &map, chunk, st);
-        } else {
-            if (e == cudaSuccess) e = launch_reduce_policy<float, true>(a, 1, st);
-            if (e == cudaSuccess) e = launch_march(a, &map, kind, chunk, st);
-        }
-    } else {
-        if (e == cudaSuccess) e = launch_reduce_policy<double, true>(a, 1, st);
-        if (e == cudaSuccess) e = launch_march(a, &map, kind, chunk, st);
+    // ghosts of cons_in in place, and the step's dt
+    GridArgs<T> in = a;
+    in.dst = static_cast<T *>(cons_in);
+    FieldView<const T> v;
+    for (int f = 0; f < 5; ++f) v.f[f] = a.src + f * a.fstride;
+    v.sx = (long long)a.ny * a.nz;
+    v.sy = a.nz;
+    v.sz = 1;
+    if (e == cudaSuccess) e = launch_set_state<T>(in, v, false, kind == kRefF32, 0, st);
+    if (e == cudaSuccess) {
+        if constexpr (sizeof(T) == 4)
+            e = kind == kFastF32 ? launch_sweep(a, &map, chunk, st) : launch_march(a, &map, kind, chunk, st);
+        else e = launch_march(a, &map, kind, chunk, st);
     }
     if (e != cudaSuccess) return fail(DG_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     if (dt_used) {
-        // dt of the step = history entry 0 (step counter started at zero)
-        e = cudaMemcpyAsync(dt_used, static_cast<unsigned char *>(scratch) + offsetof(DevCtl, hist), sizeof(double),
-                            cudaMemcpyDeviceToHost, st);
-        unsigned flags = 0;
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(&flags, static_cast<unsigned char *>(scratch) + offsetof(DevCtl, flags),
-                                sizeof(flags), cudaMemcpyDeviceToHost, st);
+        // the control fields and, behind them, history entry 0: the step's dt
+        // (its counter started at zero), in one copy
+        unsigned char head[offsetof(DevCtl, hist) + sizeof(double)];
+        e = cudaMemcpyAsync(head, scratch, sizeof(head), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return fail(DG_ERR_CUDA, std::string("read-back: ") + cudaGetErrorString(e));
+        unsigned flags;
+        std::memcpy(&flags, head + offsetof(DevCtl, flags), sizeof(flags));
+        std::memcpy(dt_used, head + offsetof(DevCtl, hist), sizeof(double));
         if (flags & kStatusTimeout) return fail(DG_ERR_TIMEOUT, "a device-side wait timed out; output invalid");
     }
     return DG_OK;

@@ -1,6 +1,6 @@
 // dg_step_fast.cu -- the FP32 fused-arithmetic step (fast policy;
-// multiply-add contraction allowed): the sweep kernel and the fast policy's
-// state reduction.  Kernels: dg_sweep_impl.cuh, dg_step_impl.cuh.
+// multiply-add contraction allowed).  Kernels: dg_sweep_impl.cuh,
+// dg_step_impl.cuh.
 #include "dg_host.h"
 #include "dg_step_impl.cuh"
 #include "dg_sweep_impl.cuh"
@@ -34,12 +34,12 @@ cudaError_t launch_sweep_t(const GridArgs<float> &a, const CUtensorMap *tmap, in
     const int chunk_in = interior_chunk(a.nx, it, chunk);
     const int n_in = it.interior() * ((a.nx - 4 + chunk_in - 1) / chunk_in);
     const int n_fr = it.frame() * ((a.nx - 4 + chunk - 1) / chunk);
-    const int nparts = n_in + n_fr;   // = step_grid_blocks(): the partials' bound
+    const int nparts = n_in + n_fr;
     if (n_in == 0) {
-        k_frame<<<n_fr, 32 * (TY + 2), smem, st>>>(a, *tmap, chunk, 0, nparts);
+        k_frame<<<n_fr, 32 * (TY + 2), smem, st>>>(a, *tmap, chunk, nparts);
         return cudaGetLastError();
     }
-    k_in<<<n_in, 32 * (TY + 2), smem, st>>>(a, *tmap, chunk_in, n_in, nparts);
+    k_in<<<n_in, 32 * (TY + 2), smem, st>>>(a, *tmap, chunk_in, nparts);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
@@ -52,7 +52,7 @@ cudaError_t launch_sweep_t(const GridArgs<float> &a, const CUtensorMap *tmap, in
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_frame, a, *tmap, chunk, n_in, nparts);
+    return cudaLaunchKernelEx(&cfg, k_frame, a, *tmap, chunk, nparts);
 }
 
 }  // namespace
@@ -65,7 +65,6 @@ cudaError_t launch_sweep(const GridArgs<float> &a, const CUtensorMap *tmap, int 
     return a.limiter == 0 ? launch_sweep_t<0, false>(a, tmap, chunk, st) : launch_sweep_t<1, false>(a, tmap, chunk, st);
 }
 
-template cudaError_t launch_reduce_policy<float, false>(const GridArgs<float> &, int, cudaStream_t);
 template cudaError_t launch_cons_to_prim_policy<float, false>(const GridArgs<float> &, const float *, float *,
                                                               long long, int, cudaStream_t);
 }  // namespace dg

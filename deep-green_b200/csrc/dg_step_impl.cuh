@@ -16,18 +16,14 @@ namespace dg {
 // Helper kernels (set-up and read-back; not on the per-step path)
 // ---------------------------------------------------------------------------
 
-// Reduction of the current state (dt of the first step, conservation sums).
-template <class T, bool EXACT>
-__global__ void __launch_bounds__(256) reduce_kernel(const GridArgs<T> a, int set_dt) {
-    __shared__ double red[8 * 7];
+// FP64 sums of the conserved fields over the interior, in a fixed order.
+template <class T> __global__ void __launch_bounds__(256) sums_kernel(const GridArgs<T> a) {
+    __shared__ double red[8][5];
     __shared__ int is_last;
     const int tid = threadIdx.x;
     const long long nyi = a.ny - 4, nzi = a.nz - 4;
     const long long total = (long long)(a.nx - 4) * nyi * nzi;
     double sum[5] = {0, 0, 0, 0, 0};
-    double wm = INFINITY;
-    unsigned nanf = 0;
-    float smax = 0.0f;   // fast policy: max wave speed (NaN-propagating)
     // the cells c = blockIdx.x * 256 + tid + k * stride, with (x, y, z)
     // advanced by the stride's own decomposition (no division per cell)
     const long long stride = (long long)gridDim.x * 256;
@@ -41,120 +37,170 @@ __global__ void __launch_bounds__(256) reduce_kernel(const GridArgs<T> a, int se
         y += sy;
         if (y >= nyi) { y -= (int)nyi; ++x; }
         x += sx;
-        T u[5], w[5];
-        for (int f = 0; f < 5; ++f) u[f] = a.src[f * a.fstride + o];
-        Phys<T, EXACT>::prim(u, w, a.k);
-        if constexpr (EXACT) {
-            const T wd = Phys<T, EXACT>::wave_dt(w, a.k);
-            if (wd != wd) nanf = 1;
-            else wm = fmin(wm, (double)wd);
-        } else {
-            smax = max_nan(smax, fast_speed(w[0], w[1], w[2], w[3], w[4], a.k.gamma));
-        }
-        for (int f = 0; f < 5; ++f) sum[f] += (double)u[f];
+        for (int f = 0; f < 5; ++f) sum[f] += (double)a.src[f * a.fstride + o];
     }
-    if constexpr (!EXACT) {
-        if (smax != smax) nanf = 1;
-        else wm = (double)__fdiv_rn(a.k.ds, smax);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        for (int f = 0; f < 5; ++f) sum[f] += __shfl_xor_sync(0xffffffffu, sum[f], o);
-        wm = fmin(wm, __shfl_xor_sync(0xffffffffu, wm, o));
-        nanf |= __shfl_xor_sync(0xffffffffu, nanf, o);
-    }
-    if ((tid & 31) == 0) {
-        for (int f = 0; f < 5; ++f) red[(tid >> 5) * 7 + f] = sum[f];
-        red[(tid >> 5) * 7 + 5] = wm;
-        red[(tid >> 5) * 7 + 6] = (double)nanf;
-    }
-    __syncthreads();
+    auto block_sum = [&](int f) {
+        double t = 0;
+        for (int w = 0; w < 8; ++w) t += red[w][f];
+        return t;
+    };
+    auto warps_to_red = [&] {
+        for (int o = 16; o > 0; o >>= 1)
+            for (int f = 0; f < 5; ++f) sum[f] += __shfl_xor_sync(0xffffffffu, sum[f], o);
+        if ((tid & 31) == 0)
+            for (int f = 0; f < 5; ++f) red[tid >> 5][f] = sum[f];
+        __syncthreads();
+    };
+    warps_to_red();
     if (tid == 0) {
-        Partial p;
-        for (int f = 0; f < 5; ++f) p.sums[f] = 0;
-        p.wmin = INFINITY;
-        p.nan = 0;
-        for (int w = 0; w < 8; ++w) {
-            for (int f = 0; f < 5; ++f) p.sums[f] += red[w * 7 + f];
-            p.wmin = fmin(p.wmin, red[w * 7 + 5]);
-            p.nan |= red[w * 7 + 6] != 0.0;
-        }
-        p.pad = 0;
-        a.part[blockIdx.x] = p;
+        for (int f = 0; f < 5; ++f) a.part[blockIdx.x].sums[f] = block_sum(f);
         __threadfence();
         is_last = atomicAdd(&a.ctl->counter, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    final_reduce<T>(a, tid, 256, red, set_dt ? kSetDt : kSumsOnly, gridDim.x);
-}
-
-// Copy every ghost cell of buf from its interior source (boundary rules).
-// Ghost cell e (0 .. ghost_cells - 1) as ghosted coordinates: the two
-// layers of each x face (4 ny nz cells), then those of each y face over the
-// interior x (4 (nx-4) nz), then those of each z face over the interior x, y
-// (4 (nx-4)(ny-4)).
-__device__ __forceinline__ void ghost_cell(long long e, int nx, int ny, int nz, int &x, int &y, int &z) {
-    const long long fx = 4LL * ny * nz, fy = 4LL * (nx - 4) * nz;
-    if (e < fx) {
-        const int s = (int)(e / ((long long)ny * nz));
-        const long long r = e - (long long)s * ny * nz;
-        x = s < 2 ? s : nx - 4 + s;
-        y = (int)(r / nz);
-        z = (int)(r - (long long)y * nz);
-    } else if (e < fx + fy) {
-        e -= fx;
-        const int xi = (int)(e / (4LL * nz));
-        const int r = (int)(e - (long long)xi * 4 * nz);
-        const int s = r / nz;
-        x = xi + 2;
-        y = s < 2 ? s : ny - 4 + s;
-        z = r - s * nz;
-    } else {
-        e -= fx + fy;
-        const long long row = e >> 2;
-        const int s = (int)(e & 3);
-        x = (int)(row / (ny - 4)) + 2;
-        y = (int)(row - (long long)(x - 2) * (ny - 4)) + 2;
-        z = s < 2 ? s : nz - 4 + s;
+    for (int f = 0; f < 5; ++f) sum[f] = 0;
+    for (unsigned b = tid; b < gridDim.x; b += 256) {
+        const volatile Partial *p = a.part + b;
+        for (int f = 0; f < 5; ++f) sum[f] += p->sums[f];
+    }
+    warps_to_red();
+    if (tid == 0) {
+        for (int f = 0; f < 5; ++f) a.ctl->sums[f] = block_sum(f);
+        a.ctl->counter = 0;
+        __threadfence();
     }
 }
 
-template <class T> __global__ void fill_ghosts_kernel(const GridArgs<T> a, T *buf) {
-    const long long total = (long long)a.nx * a.ny * a.nz - (long long)(a.nx - 4) * (a.ny - 4) * (a.nz - 4);
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total;
-         c += (long long)gridDim.x * blockDim.x) {
-        int x, y, z;
-        ghost_cell(c, a.nx, a.ny, a.nz, x, y, z);
-        int fx, fy, fz;
+// V consecutive values; V > 1 is one 16-byte access.
+template <class T, int V> struct alignas(V * sizeof(T)) Quad {
+    T v[V];
+};
+template <class T> constexpr int kVec = 16 / (int)sizeof(T);
+
+// A state into the pitched layout: every ghosted cell from its interior
+// source (the boundary rules' composed per-axis sources), converted from
+// primitives if asked (calc_conserved, physics.rs:143-175), and the interior's
+// largest wave speed, i.e. the dt of the coming step.  Bound by memory: one
+// pass in place of a copy per field, a ghost fill and a reduction.  One warp
+// per row, V values per lane (V > 1: 16-byte accesses, for views whose rows
+// allow them).
+template <class T, bool EXACT, bool PRIM, int V>
+__global__ void __launch_bounds__(256) set_state_kernel(const GridArgs<T> a, const FieldView<const T> src,
+                                                        unsigned long long step) {
+    __shared__ unsigned long long s_max;
+    if (threadIdx.x == 0) s_max = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, nw = gridDim.x * 8;
+    const int rows = a.nx * a.ny;
+    const bool in_place = !PRIM && src.f[0] == a.dst;
+    T smax = T(0);
+    for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += nw) {
+        const int x = row / a.ny, y = row - x * a.ny;
+        int fx, fy;
         const int sx = axis_source(x, a.nx, a.bc[0], a.bc[1], &fx);
         const int sy = axis_source(y, a.ny, a.bc[2], a.bc[3], &fy);
-        const int sz = axis_source(z, a.nz, a.bc[4], a.bc[5], &fz);
-        const long long o = ((long long)x * a.ny + y) * a.pitch + z;
-        const long long so = ((long long)sx * a.ny + sy) * a.pitch + sz;
-        buf[o] = buf[so];
-        buf[a.fstride + o] = fx ? -buf[a.fstride + so] : buf[a.fstride + so];
-        buf[2 * a.fstride + o] = fy ? -buf[2 * a.fstride + so] : buf[2 * a.fstride + so];
-        buf[3 * a.fstride + o] = fz ? -buf[3 * a.fstride + so] : buf[3 * a.fstride + so];
-        buf[4 * a.fstride + o] = buf[4 * a.fstride + so];
+        const bool inner_row = sx == x && sy == y;
+        const long long so = sx * src.sx + sy * src.sy, o = (long long)row * a.pitch;
+        for (int z = lane * V; z < a.nz; z += 32 * V) {
+            Quad<T, V> u[5];
+            const bool inner_z = z >= 2 && z + V <= a.nz - 2;
+            bool fz[V];
+            if (V > 1 && inner_z) {
+#pragma unroll
+                for (int f = 0; f < 5; ++f) u[f] = *reinterpret_cast<const Quad<T, V> *>(src.f[f] + so + z);
+#pragma unroll
+                for (int i = 0; i < V; ++i) fz[i] = false;
+            } else {
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                    int flip;
+                    const int sz = axis_source(min(z + i, a.nz - 1), a.nz, a.bc[4], a.bc[5], &flip);
+                    fz[i] = flip != 0;
+#pragma unroll
+                    for (int f = 0; f < 5; ++f) u[f].v[i] = src.f[f][so + sz * src.sz];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                T w[5], c[5];
+#pragma unroll
+                for (int f = 0; f < 5; ++f) c[f] = u[f].v[i];
+                if constexpr (PRIM) {
+                    T q[5];
+#pragma unroll
+                    for (int f = 0; f < 5; ++f) q[f] = c[f];
+                    prim_to_cons(q, c, a.k.vol, a.k.gm1);
+                }
+                if (inner_row && z + i >= 2 && z + i < a.nz - 2) {
+                    T sp;
+                    Phys<T, EXACT>::prim(c, w, a.k);
+                    if constexpr (EXACT)
+                        sp = sqrt(a.k.gamma * w[4] / w[0]) + sqrt(w[1] * w[1] + w[2] * w[2] + w[3] * w[3]);
+                    else sp = fast_speed(w[0], w[1], w[2], w[3], w[4], a.k.gamma);
+                    smax = (smax != smax || sp != sp) ? smax + sp : (sp > smax ? sp : smax);
+                }
+                u[0].v[i] = c[0];
+                u[1].v[i] = fx ? -c[1] : c[1];
+                u[2].v[i] = fy ? -c[2] : c[2];
+                u[3].v[i] = fz[i] ? -c[3] : c[3];
+                u[4].v[i] = c[4];
+            }
+            if (in_place && inner_row && inner_z) continue;
+            if (z + V <= a.nz) {
+#pragma unroll
+                for (int f = 0; f < 5; ++f) *reinterpret_cast<Quad<T, V> *>(a.dst + f * a.fstride + o + z) = u[f];
+            } else {
+#pragma unroll
+                for (int f = 0; f < 5; ++f)
+#pragma unroll
+                    for (int i = 0; i < V; ++i)
+                        if (z + i < a.nz) a.dst[f * a.fstride + o + z + i] = u[f].v[i];
+            }
+        }
+    }
+    finish_speed<false>(a, smax, &s_max, gridDim.x, step);
+}
+
+// Five dense arrays of n0 x n1 x n2 cells from a state seen through strides;
+// one warp per row, field after field, so that the rows in flight lie
+// together (all five fields per row: 2.6 ms at 512^3 FP32).
+template <class T, int V>
+__global__ void __launch_bounds__(256) get_state_kernel(const FieldView<const T> src, const FieldView<T> dst, int n0,
+                                                        int n1, int n2) {
+    const int lane = threadIdx.x & 31, nw = gridDim.x * 8, rows = n0 * n1;
+    for (long long r = blockIdx.x * 8 + (threadIdx.x >> 5); r < 5LL * rows; r += nw) {
+        const int f = (int)(r / rows), row = (int)(r - (long long)f * rows);
+        const int i = row / n1, j = row - i * n1;
+        const T *s = src.f[0];
+        T *d = dst.f[0];
+#pragma unroll
+        for (int g = 1; g < 5; ++g)
+            if (f == g) {
+                s = src.f[g];
+                d = dst.f[g];
+            }
+        s += i * src.sx + j * src.sy;
+        d += (long long)row * n2;
+        if constexpr (V > 1) {
+#pragma unroll 4
+            for (int k = lane; k < n2 / V; k += 32)
+                reinterpret_cast<Quad<T, V> *>(d)[k] = reinterpret_cast<const Quad<T, V> *>(s)[k];
+        } else {
+#pragma unroll 4
+            for (int k = lane; k < n2; k += 32) d[k] = s[k * src.sz];
+        }
     }
 }
 
-// calc_conserved over the interior (physics.rs:143-175); prim is dense
-// with its own pitch/field stride.
-template <class T>
-__global__ void prim_to_cons_kernel(const GridArgs<T> a, const T *prim, long long pfs, int ppitch, T *cons) {
-    const long long total = (long long)a.nx * a.ny * a.nz;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total;
-         c += (long long)gridDim.x * blockDim.x) {
-        const long long xy = c / a.nz;
-        const int z = (int)(c % a.nz);
-        const long long po = xy * ppitch + z, co = xy * a.pitch + z;
-        T w[5], u[5];
-        for (int f = 0; f < 5; ++f) w[f] = prim[f * pfs + po];
-        prim_to_cons(w, u, a.k.vol, a.k.gm1);
-        for (int f = 0; f < 5; ++f) cons[f * a.fstride + co] = u[f];
-    }
+// Whether every row of the view, and of rows `n` values apart behind the other
+// pointers, starts on a 16-byte boundary and its values are adjacent.
+template <class T, class U> inline bool vector_rows(const FieldView<T> &v, U *const other[5], long long n) {
+    if (v.sz != 1 || v.sx % kVec<U> || v.sy % kVec<U> || n % kVec<U>) return false;
+    uintptr_t bits = 0;
+    for (int f = 0; f < 5; ++f) bits |= reinterpret_cast<uintptr_t>(v.f[f]) | reinterpret_cast<uintptr_t>(other[f]);
+    return (bits & 15) == 0;
 }
 
 // calc_primitives over every cell (ghosts included).
@@ -176,12 +222,18 @@ __global__ void cons_to_prim_kernel(const GridArgs<T> a, const T *cons, T *prim,
 // ---------------------------------------------------------------------------
 // Launch wrappers (instantiated per policy by the two translation units)
 // ---------------------------------------------------------------------------
-template <class T, bool EXACT> cudaError_t launch_reduce_policy(const GridArgs<T> &a, int set_dt, cudaStream_t st) {
+template <class T> cudaError_t launch_sums_kernel(const GridArgs<T> &a, cudaStream_t st) {
     const long long total = (long long)(a.nx - 4) * (a.ny - 4) * (a.nz - 4);
     long long blocks = (total + 255) / 256;
     if (blocks > kReduceBlocks) blocks = kReduceBlocks;
-    reduce_kernel<T, EXACT><<<(int)blocks, 256, 0, st>>>(a, set_dt);
+    sums_kernel<T><<<(int)blocks, 256, 0, st>>>(a);
     return cudaGetLastError();
+}
+
+// Blocks of the row kernels: one row per warp, 8 blocks of 8 warps per SM.
+inline int row_blocks(long long rows) {
+    const long long b = (rows + 7) / 8;
+    return (int)(b > kSms * 8 ? kSms * 8 : b);
 }
 
 inline int flat_blocks(long long total) {

@@ -281,13 +281,12 @@ template <class T, int TY, int R> struct Smem {
     T zex[2][TY][5];                                      // last column's xt (wall) or lower state (outflow)
     T fz[2][TY][5];                                       // flux of the right edge face (even width)
     uint64_t bar[R];
-    double red[(TY + 2) * 7];
+    unsigned long long wmax;                              // finish_speed
     // set when a wait gave up, read after the next barrier; two slots by
     // plane parity, so a warp already working on plane m + 1 cannot flag a
     // warp that is still between the barriers of plane m
     int abort_flag[2];
     int skip;
-    int is_last;
 };
 
 template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
@@ -987,13 +986,12 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
         }
     }
 
-    // One work item: tile (ty, tz) of grid `a`, x-planes of chunk cx.  Its
-    // partial result goes to a.part[part_idx]; the last of the grid's
-    // nparts items reduces them (next dt).  Returns false after a
+    // One work item: tile (ty, tz) of grid `a`, x-planes of chunk cx.  The last
+    // of the grid's nparts items to finish sets the next dt.  Returns false after a
     // device-side wait timed out (status flag set).
     template <bool IN>
     static __device__ bool run_tile(const GridArgs<T> &a, const CUtensorMap *tmap, int tz, int ty, int cx, int chunk,
-                                    int part_idx, int nparts, unsigned char *raw) {
+                                    int nparts, unsigned char *raw) {
         Sm &s = *reinterpret_cast<Sm *>(raw);
         const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
         Tile t;
@@ -1027,6 +1025,7 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
         if (tid == 0) {
             s.skip = (*(volatile unsigned *)&a.ctl->flags & kStatusTimeout) != 0;
             s.abort_flag[0] = s.abort_flag[1] = 0;
+            s.wmax = 0;
             if (!s.skip) {
                 for (int i = 0; i < R; ++i) mbar_init(&s.bar[i], 1);
                 fence_mbar_init();
@@ -1059,14 +1058,7 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
         // by the next work item of a persistent launch
         if (tid == 0)
             for (int i = 0; i < R; ++i) mbar_inval(&s.bar[i]);
-        // min over cells of ds/speed = ds / max speed
-        const unsigned nanf = smax != smax;
-        const double wmin = nanf ? INFINITY : (double)__fdiv_rn(a.k.ds, smax);
-        double sum[5] = {0, 0, 0, 0, 0};
-        if (block_partial(a, sum, wmin, nanf, tid, NT, s.red, &s.is_last, part_idx, nparts)) {
-            __threadfence();
-            final_reduce<T>(a, tid, NT, s.red, kAdvance, nparts);
-        }
+        finish_speed<true>(a, smax, &s.wmax, nparts);
         return true;
     }
 };
@@ -1091,15 +1083,14 @@ template <int TY> constexpr int sweep_max_regs() {
 // frame tiles x chunks), InteriorTiles.
 // The two touch disjoint tiles of the output and read only the input state,
 // so the frame launch may run beside the interior one (programmatic
-// dependent launch, launch_sweep).  They share one reduction: the interior
-// blocks hold partials [0, n_in), the frame blocks the rest, and whichever
-// block of either takes the last ticket advances dt (every block has read
-// the step's dt by then).  Without interior tiles the frame launch is the
-// whole step (n_in = 0).
+// dependent launch, launch_sweep).  They share one reduction over their
+// nparts blocks: whichever block of either takes the last ticket advances dt
+// (every block has read the step's dt by then).  Without interior tiles the
+// frame launch is the whole step.
 template <class T, int TY, int R, int LIM, bool GRAV, bool IN>
 __global__ void __maxnreg__(sweep_max_regs<TY>()) sweep_step_kernel(const GridArgs<T> a,
                                                                       const __grid_constant__ CUtensorMap tmap,
-                                                                      int chunk, int n_in, int nparts) {
+                                                                      int chunk, int nparts) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // the frame launch reads nothing this launch writes: let it start on the
     // SMs this launch leaves free
@@ -1116,8 +1107,7 @@ __global__ void __maxnreg__(sweep_max_regs<TY>()) sweep_step_kernel(const GridAr
         it.frame_tile(b % nf, ty, tz);
         b /= nf;
     }
-    const int part = IN ? (int)blockIdx.x : n_in + (int)blockIdx.x;
-    Sweep<T, TY, R, LIM, GRAV>::template run_tile<IN>(a, &tmap, tz, ty, b, chunk, part, nparts, smem_raw);
+    Sweep<T, TY, R, LIM, GRAV>::template run_tile<IN>(a, &tmap, tz, ty, b, chunk, nparts, smem_raw);
 }
 
 // Batched step: one persistent launch advances many independent grids by
@@ -1128,7 +1118,7 @@ __global__ void __maxnreg__(sweep_max_regs<TY>()) sweep_step_kernel(const GridAr
 // by the host before launch).  All grids of one launch share the limiter and
 // the gravity switch (the host launches one kernel per combination).
 struct BatchItem {
-    int g, local, tz, ty, cx;
+    int g, tz, ty, cx;
 };
 
 template <int TY, int R, int LIM, bool GRAV>
@@ -1151,8 +1141,8 @@ __global__ void __maxnreg__(sweep_max_regs<TY>()) sweep_batch_kernel(const GridA
             reinterpret_cast<int *>(&s_args)[i] = reinterpret_cast<const int *>(&args[bi.g])[i];
         __syncthreads();
         const GridArgs<float> ga = s_args;
-        const bool ok = Sweep<float, TY, R, LIM, GRAV>::template run_tile<false>(ga, &maps[bi.g], bi.tz, bi.ty, bi.cx, chunk,
-                                                                 bi.local, ga.nparts, smem_raw);
+        const bool ok = Sweep<float, TY, R, LIM, GRAV>::template run_tile<false>(ga, &maps[bi.g], bi.tz, bi.ty, bi.cx,
+                                                                                 chunk, ga.nparts, smem_raw);
         __syncthreads();
         if (!ok) return;
     }
