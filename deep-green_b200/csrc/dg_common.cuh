@@ -81,34 +81,34 @@ template <class A> __device__ __forceinline__ long long wait_budget_of(const A &
 }
 
 // ---------------------------------------------------------------------------
-// Ghost images: the set of cells (interior cell itself plus ghosts) that
-// hold a copy of interior coordinate c along one axis of extent n
-// (boundaries.rs / handle_walls source rules, inverted).  flip[i] = 1 when
-// the copy is a wall mirror (normal momentum negated).
+// Ghost images along one axis of extent n: bit g (0-3) is set when ghost index
+// 0, 1, n-2, n-1 holds an image of interior coordinate c (boundaries.rs /
+// handle_walls source rules, inverted), bit 4 + g when that image is a wall's
+// mirror (normal momentum negated).
 // ---------------------------------------------------------------------------
-__host__ __device__ __forceinline__ int axis_images(int c, int n, int lo, int hi, int out[4], int flip[4]) {
-    int m = 0;
-    out[m] = c; flip[m++] = 0;
+__host__ __device__ __forceinline__ unsigned image_bits(int c, int n, int lo, int hi) {
+    unsigned b = 0;
     if (lo == kPeriodic) {
-        if (c == n - 4) { out[m] = 0; flip[m++] = 0; }
-        if (c == n - 3) { out[m] = 1; flip[m++] = 0; }
+        if (c == n - 4) b |= 1u;
+        if (c == n - 3) b |= 2u;
     } else if (lo == kOutflow) {
-        if (c == 2) { out[m] = 0; flip[m++] = 0; out[m] = 1; flip[m++] = 0; }
+        if (c == 2) b |= 3u;
     } else {
-        if (c == 2) { out[m] = 1; flip[m++] = 1; }
-        if (c == 3) { out[m] = 0; flip[m++] = 1; }
+        if (c == 2) b |= 0x22u;
+        if (c == 3) b |= 0x11u;
     }
     if (hi == kPeriodic) {
-        if (c == 2 && m < 4) { out[m] = n - 2; flip[m++] = 0; }
-        if (c == 3 && m < 4) { out[m] = n - 1; flip[m++] = 0; }
+        if (c == 2) b |= 4u;
+        if (c == 3) b |= 8u;
     } else if (hi == kOutflow) {
-        if (c == n - 3 && m < 3) { out[m] = n - 2; flip[m++] = 0; out[m] = n - 1; flip[m++] = 0; }
+        if (c == n - 3) b |= 12u;
     } else {
-        if (c == n - 3 && m < 4) { out[m] = n - 2; flip[m++] = 1; }
-        if (c == n - 4 && m < 4) { out[m] = n - 1; flip[m++] = 1; }
+        if (c == n - 3) b |= 0x44u;
+        if (c == n - 4) b |= 0x88u;
     }
-    return m;
+    return b;
 }
+__host__ __device__ __forceinline__ int ghost_at(int g, int n) { return g < 2 ? g : n - 4 + g; }
 
 // Source interior coordinate of ghosted coordinate g along one axis, and
 // whether the copy is a wall mirror.

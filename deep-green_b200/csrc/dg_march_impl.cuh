@@ -396,20 +396,6 @@ template <class T, class P, int TY, int R, int LIM, bool GRAV> struct March {
         P::template slopes<LIM>(m, q, p, gz, a, k);
     }
 
-    // The four ghost indices 0, 1, n-2, n-1 of an axis that hold an image of
-    // interior cell c (bits 0-3) and which of them are mirrors (bits 4-7).
-    static __device__ __forceinline__ unsigned image_bits(int c, int n, int lo, int hi) {
-        int img[4], flp[4];
-        const int m = axis_images(c, n, lo, hi, img, flp);
-        unsigned b = 0;
-        for (int i = 1; i < m; ++i) {
-            const int g = img[i] < 2 ? img[i] : img[i] - n + 4;
-            b |= (1u << g) | (flp[i] ? 16u << g : 0u);
-        }
-        return b;
-    }
-    static __device__ __forceinline__ int ghost_at(int g, int n) { return g < 2 ? g : n - 4 + g; }
-
     // ---------------------------------------------------------------------
     // Owned warp: row y0 + r.
     // ---------------------------------------------------------------------

@@ -320,75 +320,80 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
                   fast_speed(q[0].y, q[1].y, q[2].y, q[3].y, q[4].y, k.gamma));
     }
 
-    // The ghost-cell images of one updated cell (all but the cell itself):
-    // the copies the reference's ghost fill makes of a cell next to a domain
-    // face (axis_images: periodic wrap, outflow copy, wall mirror with the
-    // normal momentum negated).  Rare: only cells within two of a face of a
-    // grid of odd width.  Inlined like xy_images (a call in the march costs
-    // more than the larger code).
-    static __device__ __forceinline__ void images(const GridArgs<T> &a, int x, int y, int z, T u0, T u1, T u2, T u3,
-                                               T u4) {
-        int ximg[4], xflp[4], yimg[4], yflp[4], zimg[4], zflp[4];
-        const int nxi = axis_images(x, a.nx, a.bc[0], a.bc[1], ximg, xflp);
-        const int nyi = axis_images(y, a.ny, a.bc[2], a.bc[3], yimg, yflp);
-        const int nzi = axis_images(z, a.nz, a.bc[4], a.bc[5], zimg, zflp);
-        for (int ix = 0; ix < nxi; ++ix)
-            for (int iy = 0; iy < nyi; ++iy)
-                for (int iz = 0; iz < nzi; ++iz) {
-                    if (ix == 0 && iy == 0 && iz == 0) continue;   // the cell itself
-                    const long long o = ((long long)ximg[ix] * a.ny + yimg[iy]) * a.pitch + zimg[iz];
-                    a.dst[o] = u0;
-                    a.dst[a.fstride + o] = xflp[ix] ? -u1 : u1;
-                    a.dst[2 * a.fstride + o] = yflp[iy] ? -u2 : u2;
-                    a.dst[3 * a.fstride + o] = zflp[iz] ? -u3 : u3;
-                    a.dst[4 * a.fstride + o] = u4;
-                }
-    }
+    // Ghost images along z of a lane's pair, fixed for the march.  With an
+    // even interior width every pair is aligned with the faces, and the
+    // images of a pair at a z face are one pair at zt: its cells (c0, c1 of
+    // the pair), the z momentum negated for a wall.  Odd widths (and width 2,
+    // where both faces share a pair) list each cell's ghost indices as bits:
+    // image_bits of the first cell, then of the second.
+    struct ZImages {
+        int zt = -1;
+        bool c0 = false, c1 = true, flip = false;
+        unsigned cells = 0;
+    };
 
-    // An updated pair (or its first cell) at (xq, yq, z), and for a lane at
-    // a z face of an even-width grid its z-image pair at zt (cells zc0, zc1
-    // of the pair; field 3 negated for a wall); fields 1 / 2 negated for a
-    // mirror along x / y.
+    // An updated pair (or its first cell) at (xq, yq, z) with its z images;
+    // fields 1 / 2 negated for a mirror along x / y.
     static __device__ __forceinline__ void put(const GridArgs<T> &a, int xq, int yq, int z, const V u[5], bool s0,
-                                               bool s1, bool fx, bool fy, int zt, int zc0, int zc1, bool zflip) {
-        const long long o = ((long long)xq * a.ny + yq) * a.pitch + z;
+                                               bool s1, bool fx, bool fy, const ZImages &zi) {
+        T *row = a.dst + ((long long)xq * a.ny + yq) * a.pitch;
         if (s1) {
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
                 const bool neg = (f == 1 && fx) || (f == 2 && fy);
-                stv(a.dst + f * a.fstride + o, neg ? vmul(u[f], spl<V>(-1.0)) : u[f]);
+                stv(row + f * a.fstride + z, neg ? vmul(u[f], spl<V>(-1.0)) : u[f]);
             }
-            if (zt >= 0) {
-                const long long oz = ((long long)xq * a.ny + yq) * a.pitch + zt;
+            if (zi.zt >= 0) {
 #pragma unroll
                 for (int f = 0; f < 5; ++f) {
-                    V v = mk(zc0 ? u[f].y : u[f].x, zc1 ? u[f].y : u[f].x);
-                    if ((f == 1 && fx) || (f == 2 && fy) || (f == 3 && zflip)) v = vmul(v, spl<V>(-1.0));
-                    stv(a.dst + f * a.fstride + oz, v);
+                    V v = mk(zi.c0 ? u[f].y : u[f].x, zi.c1 ? u[f].y : u[f].x);
+                    if ((f == 1 && fx) || (f == 2 && fy) || (f == 3 && zi.flip)) v = vmul(v, spl<V>(-1.0));
+                    stv(row + f * a.fstride + zi.zt, v);
                 }
             }
         } else if (s0) {
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
                 const bool neg = (f == 1 && fx) || (f == 2 && fy);
-                a.dst[f * a.fstride + o] = neg ? -u[f].x : u[f].x;
+                row[f * a.fstride + z] = neg ? -u[f].x : u[f].x;
+            }
+        }
+        if (zi.cells) {
+            for (int c = 0; c < 2; ++c) {
+                const unsigned bits = zi.cells >> (8 * c);
+                for (unsigned b = (c ? s1 : s0) ? bits & 15u : 0u; b; b &= b - 1) {
+                    const int g = __ffs(b) - 1, zg = ghost_at(g, a.nz);
+#pragma unroll
+                    for (int f = 0; f < 5; ++f) {
+                        const T v = c ? u[f].y : u[f].x;
+                        const bool neg = (f == 1 && fx) || (f == 2 && fy) || (f == 3 && ((bits >> (4 + g)) & 1u));
+                        row[f * a.fstride + zg] = neg ? -v : v;
+                    }
+                }
             }
         }
     }
 
     // The x / y ghost images of an updated pair next to an x or y face
     // (boundary planes and rows only): the pair again at every image plane
-    // and row, with its z images (put).  Inlined: a call in the march
-    // constrains the register allocation of the whole loop.
-    static __device__ __forceinline__ void xy_images(const GridArgs<T> &a, int xu, int y, int z, V u0, V u1, V u2, V u3,
-                                                  V u4, bool s0, bool s1, int zt, int zc0, int zc1, bool zflip) {
-        const V u[5] = {u0, u1, u2, u3, u4};
-        int ximg[4], xflp[4], yimg[4], yflp[4];
-        const int nxi = axis_images(xu, a.nx, a.bc[0], a.bc[1], ximg, xflp);
-        const int nyi = axis_images(y, a.ny, a.bc[2], a.bc[3], yimg, yflp);
-        for (int ix = 0; ix < nxi; ++ix)
-            for (int iy = 0; iy < nyi; ++iy)
-                if (ix || iy) put(a, ximg[ix], yimg[iy], z, u, s0, s1, xflp[ix] != 0, yflp[iy] != 0, zt, zc0, zc1, zflip);
+    // and row, with its z images (put).  The images are lists of bits, uniform
+    // over the warp: arrays of them lived in local memory, and the boundary
+    // rows that walked them held up their whole tile at the barrier.  Inlined:
+    // a call in the march constrains the register allocation of the whole
+    // loop.
+    static __device__ __forceinline__ void xy_images(const GridArgs<T> &a, int xu, int y, int z, const V u[5], bool s0,
+                                                     bool s1, unsigned xbits, unsigned ybits, const ZImages &zi) {
+        // bit 0: the cell's own plane / row; bit 1 + g: ghost index g
+        for (unsigned bx = ((xbits & 15u) << 1) | 1u; bx; bx &= bx - 1) {
+            const int gx = __ffs(bx) - 2;
+            const int xq = gx < 0 ? xu : ghost_at(gx, a.nx);
+            const bool fx = gx >= 0 && ((xbits >> (4 + gx)) & 1u);
+            for (unsigned by = ((ybits & 15u) << 1) | (gx >= 0 ? 1u : 0u); by; by &= by - 1) {
+                const int gy = __ffs(by) - 2;
+                put(a, xq, gy < 0 ? y : ghost_at(gy, a.ny), z, u, s0, s1, fx, gy >= 0 && ((ybits >> (4 + gy)) & 1u),
+                    zi);
+            }
+        }
     }
 
     // Load a pair of staged conserved values and convert it.
@@ -484,8 +489,7 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
         const bool yout = !IN && r == 0 && t.ylo == kOut;
         const bool zout = !IN && lane == 0 && t.zlo == kOut;
         const bool zheat = !IN && lane == 0 && t.zlo == kWallM && (a.heat & 4);
-        const bool img_y = !IN && (y <= 3 || y >= a.ny - 4);
-        const bool img_z = !IN && (z <= 3 || z + 1 >= a.nz - 4);
+        const unsigned ybits = !IN && active ? image_bits(y, a.ny, a.bc[2], a.bc[3]) : 0u;
         // carried along the march: lox, the lower state of the x face ahead
         // (xt + s/2 of the previous plane); nacc, the previous plane's flux
         // balance so far, negated (its lower faces' fluxes enter with a plus
@@ -515,37 +519,32 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
             prim(u, w, k);
             sp = speed_pair(w, k);
         };
-        // Ghost images along z of the lane's pair.  With an even interior
-        // width every pair is aligned with the faces, and the images of a
-        // pair at a z face are one pair at zt: (u[c0], u[c1]), the z
-        // momentum negated for a wall (axis_images' rules: periodic wrap,
-        // outflow copy of the first/last cell, wall mirror).  Odd widths and
-        // width 2 take the per-cell path (images()).
-        const bool even_z = ((a.nz - 4) & 1) == 0 && a.nz - 4 >= 4;   // (width 2: both faces on one pair)
-        int zt = -1, zc0 = 0, zc1 = 1;
-        bool zflip = false;
-        if (!IN && even_z && val1) {
-            if (z == 2) {
-                if (a.bc[4] == kPeriodic) { zt = a.nz - 2; }
-                else if (a.bc[4] == kOutflow) { zt = 0; zc1 = 0; }
-                else { zt = 0; zc0 = 1; zc1 = 0; zflip = true; }
-            } else if (z + 1 == a.nz - 3) {
-                if (a.bc[5] == kPeriodic) { zt = 0; }
-                else if (a.bc[5] == kOutflow) { zt = a.nz - 2; zc0 = 1; }
-                else { zt = a.nz - 2; zc0 = 1; zc1 = 0; zflip = true; }
+        ZImages zi;
+        if (!IN) {
+            if (((a.nz - 4) & 1) == 0 && a.nz - 4 >= 4) {
+                if (val1 && z == 2) {
+                    if (a.bc[4] == kPeriodic) { zi.zt = a.nz - 2; }
+                    else if (a.bc[4] == kOutflow) { zi.zt = 0; zi.c1 = false; }
+                    else { zi.zt = 0; zi.c0 = true; zi.c1 = false; zi.flip = true; }
+                } else if (val1 && z + 1 == a.nz - 3) {
+                    if (a.bc[5] == kPeriodic) { zi.zt = 0; }
+                    else if (a.bc[5] == kOutflow) { zi.zt = a.nz - 2; zi.c0 = true; }
+                    else { zi.zt = a.nz - 2; zi.c0 = true; zi.c1 = false; zi.flip = true; }
+                }
+            } else {
+                if (val0) zi.cells = image_bits(z, a.nz, a.bc[4], a.bc[5]);
+                if (val1) zi.cells |= image_bits(z + 1, a.nz, a.bc[4], a.bc[5]) << 8;
             }
         }
-        const bool zslow = !even_z && img_z;
         auto store = [&](int xu, const V u[5], const V &sp, bool on) {
             const bool s0 = on && val0, s1 = on && val1;
             if (s0) smax = smax_of(smax, sp.x);
             if (s1) smax = smax_of(smax, sp.y);
-            put(a, xu, y, z, u, s0, s1, false, false, zt, zc0, zc1, zflip);
+            put(a, xu, y, z, u, s0, s1, false, false, zi);
             const bool img_x = xu <= 3 || xu >= a.nx - 4;
-            if (on && (img_x || img_y)) xy_images(a, xu, y, z, u[0], u[1], u[2], u[3], u[4], s0, s1, zt, zc0, zc1, zflip);
-            if (on && zslow) {
-                if (s0) images(a, xu, y, z, u[0].x, u[1].x, u[2].x, u[3].x, u[4].x);
-                if (s1) images(a, xu, y, z + 1, u[0].y, u[1].y, u[2].y, u[3].y, u[4].y);
+            if (on && (img_x || ybits)) {
+                const unsigned xbits = img_x ? image_bits(xu, a.nx, a.bc[0], a.bc[1]) : 0u;
+                if (xbits | ybits) xy_images(a, xu, y, z, u, s0, s1, xbits, ybits, zi);
             }
         };
 
@@ -1140,9 +1139,8 @@ __global__ void __maxnreg__(sweep_max_regs<TY>()) sweep_batch_kernel(const GridA
         for (int i = tid; i < kWords; i += blockDim.x)
             reinterpret_cast<int *>(&s_args)[i] = reinterpret_cast<const int *>(&args[bi.g])[i];
         __syncthreads();
-        const GridArgs<float> ga = s_args;
-        const bool ok = Sweep<float, TY, R, LIM, GRAV>::template run_tile<false>(ga, &maps[bi.g], bi.tz, bi.ty, bi.cx,
-                                                                                 chunk, ga.nparts, smem_raw);
+        const bool ok = Sweep<float, TY, R, LIM, GRAV>::template run_tile<false>(s_args, &maps[bi.g], bi.tz, bi.ty,
+                                                                                 bi.cx, chunk, s_args.nparts, smem_raw);
         __syncthreads();
         if (!ok) return;
     }
