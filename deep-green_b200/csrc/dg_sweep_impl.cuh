@@ -6,8 +6,7 @@
 // Decomposition.  A block owns a tile of TY rows (y) x 64 columns (z) of
 // cells and marches along x through a chunk of planes.  Each plane arrives by
 // one 4-D TMA copy (68 columns x (TY + 4) rows x 5 fields: the tile and its
-// 2-cell halo, no multicast) in a ring of R slots, and stays there as
-// conserved totals until its cells are updated.
+// 2-cell halo, no multicast) in a ring of R slots.
 //   * Owned warps (TY): warp r owns row y0 + r; lane l owns the two adjacent
 //     cells (z, z + 1), z = z0 + 2l, as one pair.  Every per-cell formula is
 //     written on pairs, and a pair is one packed register, so the
@@ -501,11 +500,24 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
 #pragma unroll
         for (int f = 0; f < 5; ++f) lox[f] = nacc[f] = tu[f] = spl<V>(0.0);
 
-        // Update of plane xu (staged index sl_idx) with the term tu: the new
-        // state and its wave speeds (stores are left to the caller).
-        auto update = [&](int xu, int sl_idx, V u[5], V &sp) {
+        // The pair's conserved totals in plane xu (staged index sl).  Interior
+        // tiles read them again from the input state (L2), so that the ring
+        // holds only planes still to be converted and the copies run three
+        // planes ahead instead of one (512^3 outflow 3.44 -> 3.27 ms per
+        // step); the general loop has no registers for values in flight and
+        // keeps its planes staged until their update (with the same change 48
+        // uneven grids went from 1.17 to 1.26 ms).
+        const T *own = a.src + (long long)y * a.pitch + z;
+        auto load_own = [&](int xu, int sl, V u0[5]) {
+            const T *p = own + (long long)xu * a.ny * a.pitch;
+#pragma unroll
+            for (int f = 0; f < 5; ++f)
+                u0[f] = IN ? __ldg(reinterpret_cast<const V *>(p + f * a.fstride)) : ldv(&C(slot(s, sl), f, r + 2, col));
+        };
+        // Update of plane xu, totals u0, with the term tu: the new state and
+        // its wave speeds (stores are left to the caller).
+        auto update = [&](int xu, const V u0[5], V u[5], V &sp) {
             const int pp = xu & 1;
-            T *sl = slot(s, sl_idx);
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
                 V tt = tu[f];
@@ -513,7 +525,7 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
                 if (!yout) tt = vadd(tt, ldv(&s.fy[pp][r + 1][f][2 * lane]));
                 const T fe = s.fz[pp][r][f];
                 tt.y += edge_even ? fe : T(0);
-                u[f] = vfma(spl<V>(k.sc[f]), tt, ldv(&C(sl, f, r + 2, col)));
+                u[f] = vfma(spl<V>(k.sc[f]), tt, u0[f]);
             }
             V w[5];
             prim(u, w, k);
@@ -570,7 +582,11 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
             const int l = m - t.xs + 3;
             const int pm = m & 1;
             const bool upd = m >= t.xs && m < t.xe;
-            V sy[5], sz[5], xtc[5];
+            V sy[5], sz[5], xtc[5], u0[5];
+            // update of plane m-2 (from plane xs on; earlier iterations
+            // compute on a valid plane and store nothing)
+            const bool do_upd = m - 2 >= t.xs;
+            if (IN) load_own(do_upd ? m - 2 : t.xs, 0, u0);
             if (upper_stash(a, m)) barrier();
             if (!wait_plane(s, l, t.budget)) s.abort_flag[m & 1] = 1;
             if (active) {
@@ -584,10 +600,8 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
                 }
                 load_prim_pair(slot(s, l), r + 2, col, k, qn);
                 store_pb(s, pm ^ 1, r + 1, col, qn);
-                // update of plane m-2 (from plane xs on; earlier iterations
-                // compute on a valid slot and store nothing)
-                const bool do_upd = m - 2 >= t.xs;
-                update(m - 2, do_upd ? l - 3 : 0, u, sp);
+                if (!IN) load_own(0, do_upd ? l - 3 : 0, u0);
+                update(m - 2, u0, u, sp);
 #pragma unroll
                 for (int f = 0; f < 5; ++f) dn[f] = vsub(qn[f], q[f]);
                 slopes_adj(s, pm, r + 1, col, q, dq, dn, nullptr, nullptr, sx, sy, sz);
@@ -754,8 +768,9 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
         }
         // the last plane of the chunk: its fluxes arrived with the last barrier
         if (!aborted && active && t.xe - 1 >= t.xs) {
-            V u[5], sp;
-            update(t.xe - 1, t.xe - t.xs + 1, u, sp);
+            V u0[5], u[5], sp;
+            load_own(t.xe - 1, t.xe - t.xs + 1, u0);
+            update(t.xe - 1, u0, u, sp);
             store(t.xe - 1, u, sp, true);
         }
     }
@@ -767,6 +782,7 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
     // columns outside the lanes' pairs, and the TMA copies.  Returns the
     // number of planes it requested.
     // ---------------------------------------------------------------------
+    template <bool IN>
     static __device__ int run_a(Sm &s, const GridArgs<T> &a, const CUtensorMap *tmap, const Tile &t, int lane) {
         const K<T> &k = t.k;
         const int col = 2 + 2 * lane;
@@ -812,6 +828,20 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
         fence_proxy_async();
         barrier();
         if (s.abort_flag[t.xs & 1]) return issued;
+        // The barrier of plane m frees the slot of plane m+1, converted before
+        // it (interior tiles), or of plane m-2, updated before it.
+        auto stage = [&](int nl) {
+            if (nl >= t.np) return;
+            if (lane == 0) {
+                mbar_expect_tx(&s.bar[nl % R], Sm::kBoxBytes);
+                tma_load_4d(slot(s, nl), tmap, t.z0 - 2, t.y0 - 2, t.xs - 2 + nl, 0, &s.bar[nl % R]);
+            }
+            issued = nl + 1;
+        };
+        if (IN) {
+            stage(R);
+            stage(R + 1);
+        }
         for (int m = t.xs - 1; m <= t.xe; ++m) {
             const int l = m - t.xs + 3;
             const int pm = m & 1;
@@ -875,17 +905,8 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
             fence_proxy_async();
             barrier();
             if (s.abort_flag[m & 1]) break;
-            // from plane xs on, the barrier frees the slot of plane m-2
-            // (staged index m - xs): stage plane m-2+R there (the first R
-            // planes were staged before the march)
-            const int nl = m - t.xs + R;
-            if (m >= t.xs && nl < t.np) {
-                if (lane == 0) {
-                    mbar_expect_tx(&s.bar[nl % R], Sm::kBoxBytes);
-                    tma_load_4d(slot(s, nl), tmap, t.z0 - 2, t.y0 - 2, t.xs - 2 + nl, 0, &s.bar[nl % R]);
-                }
-                issued = nl + 1;
-            }
+            if (IN) stage(l + R);
+            else if (m >= t.xs) stage(m - t.xs + R);
         }
         return issued;
     }
@@ -1041,7 +1062,7 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
         T smax = T(0);
         int issued = 0;
         if (warp < TY) run_owned<IN>(s, a, t, warp, lane, smax);
-        else if (warp == WA) issued = run_a(s, a, tmap, t, lane);
+        else if (warp == WA) issued = run_a<IN>(s, a, tmap, t, lane);
         else run_b(s, a, t, lane);
         __syncthreads();
         if (s.abort_flag[0] | s.abort_flag[1]) {
