@@ -462,14 +462,14 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
     // ---------------------------------------------------------------------
     // Owned warp: row y0 + r, lane pair at buffer columns (col, col + 1).
     //
-    // Plane m's iteration, before the barrier: convert plane m+1; update
-    // plane m-2 (its last fluxes arrived with the barrier of plane m-1) and
-    // compute its wave speeds; slopes, prediction and the x-face flux
-    // between planes m-1 and m; publish the face states other warps need;
-    // store plane m-2.  After the barrier: the y- and z-face fluxes of plane
-    // m.  The update comes first and its stores last, so that one straight
-    // run of code interleaves its long dependency chain (loads, reciprocal,
-    // square roots) with the slopes and the prediction of plane m.
+    // Plane m's iteration, before the barrier: convert plane m+1; slopes,
+    // prediction and the x-face flux between planes m-1 and m; publish the face
+    // states other warps need.  After it: the y- and z-face fluxes of plane m
+    // and the update of plane m-1 (whose last fluxes arrived with the barrier)
+    // with its wave speeds and stores.  With the update before the barrier of
+    // plane m+1 instead, its term lived across the loop in ten more registers
+    // and the code stood a second time behind the loop: 4-8 % slower on every
+    // size.
     // ---------------------------------------------------------------------
     //
     // IN: the tile is interior (InteriorTiles): every row and column is
@@ -493,12 +493,11 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
         // (xt + s/2 of the previous plane); nacc, the previous plane's flux
         // balance so far, negated (its lower faces' fluxes enter with a plus
         // sign, so no flux is negated on its own; negation being exact, the
-        // sums round as the balance itself would); tu, the update term of the
-        // plane before it.  The own cell's primitives of the current and the
+        // sums round as the balance itself would).  The own cell's primitives of the current and the
         // previous plane are read back from the primitive buffer.
-        V lox[5], nacc[5], tu[5];
+        V lox[5], nacc[5];
 #pragma unroll
-        for (int f = 0; f < 5; ++f) lox[f] = nacc[f] = tu[f] = spl<V>(0.0);
+        for (int f = 0; f < 5; ++f) lox[f] = nacc[f] = spl<V>(0.0);
 
         // The pair's conserved totals in plane xu (staged index sl).  Interior
         // tiles read them again from the input state (L2), so that the ring
@@ -516,7 +515,7 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
         };
         // Update of plane xu, totals u0, with the term tu: the new state and
         // its wave speeds (stores are left to the caller).
-        auto update = [&](int xu, const V u0[5], V u[5], V &sp) {
+        auto update = [&](int xu, const V u0[5], const V tu[5], V u[5], V &sp) {
             const int pp = xu & 1;
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
@@ -577,20 +576,16 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
         fence_proxy_async();
         barrier();
         if (s.abort_flag[t.xs & 1]) return;
-        bool aborted = false;
         for (int m = t.xs - 1; m <= t.xe; ++m) {
             const int l = m - t.xs + 3;
             const int pm = m & 1;
             const bool upd = m >= t.xs && m < t.xe;
-            V sy[5], sz[5], xtc[5], u0[5];
-            // update of plane m-2 (from plane xs on; earlier iterations
-            // compute on a valid plane and store nothing)
-            const bool do_upd = m - 2 >= t.xs;
-            if (IN) load_own(do_upd ? m - 2 : t.xs, 0, u0);
+            V sy[5], sz[5], xtc[5], u0[5], tu[5];
+            const bool do_upd = m > t.xs;   // plane m-1 is this chunk's
             if (upper_stash(a, m)) barrier();
             if (!wait_plane(s, l, t.budget)) s.abort_flag[m & 1] = 1;
             if (active) {
-                V q[5], dq[5], qn[5], dn[5], sx[5], xt[5], u[5], sp;
+                V q[5], dq[5], qn[5], dn[5], sx[5], xt[5];
                 // the own cell at planes m and m-1 (this thread's entries), read
                 // before the conversion of plane m+1 replaces plane m-1's
 #pragma unroll
@@ -600,8 +595,6 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
                 }
                 load_prim_pair(slot(s, l), r + 2, col, k, qn);
                 store_pb(s, pm ^ 1, r + 1, col, qn);
-                if (!IN) load_own(0, do_upd ? l - 3 : 0, u0);
-                update(m - 2, u0, u, sp);
 #pragma unroll
                 for (int f = 0; f < 5; ++f) dn[f] = vsub(qn[f], q[f]);
                 slopes_adj(s, pm, r + 1, col, q, dq, dn, nullptr, nullptr, sx, sy, sz);
@@ -662,8 +655,7 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
                         }
                         face<1, false>(lo, up, spl<V>(0.0), k, fx);
                         // plane m-1 is complete but for its upper y flux and its
-                        // right edge flux (added at its update, two planes on); on
-                        // a lower outflow x face plane 2 sees no x divergence
+                        // right edge flux (added at its update); on a lower outflow x face plane 2 sees no x divergence
                         const bool xo_prev = m - 1 == 2 && a.bc[0] == kOutflow;
                         const bool xo = m == 2 && a.bc[0] == kOutflow;
     #pragma unroll
@@ -702,12 +694,13 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
                         }
                     }
                 }
-                store(m - 2, u, sp, do_upd);
             }
             fence_proxy_async();
             barrier();
-            if (s.abort_flag[m & 1]) { aborted = true; break; }
-            if (!active || !upd) continue;
+            if (s.abort_flag[m & 1]) return;
+            if (!active) continue;
+            if (IN && do_upd) load_own(m - 1, 0, u0);
+            if (upd) {
             // ================= after the barrier: y and z faces of plane m
             const V *xt = xtc;
             V ndy[5];   // the lower y face's flux (plus the heat of a conducting face)
@@ -741,37 +734,48 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
             for (int f = 0; f < 5; ++f) {
                 const V U = vadd(xt[f], sz[f]);
                 const V L = vsub(xt[f], sz[f]);
-                // the halo columns' states (broadcast loads, used by lane 0
-                // and, for an odd width, by the edge lane)
-                const T mx = f == 3 ? -xt[f].x : xt[f].x;   // wall mirror of the pair's first cell
-                T zlv = s.zl[pm][r][f];
-                if (!IN && t.zlo == kWallM) zlv += mx;
-                T zrv = s.zr[pm][r][f];
-                if (!IN && t.zhi == kWallM) zrv += mx;
-                if (!IN && t.zhi == kOut) zrv = L.x;
+                // the left halo column's state (a broadcast load, used by lane 0)
+                const T zlv = s.zl[pm][r][f];
                 const T left = __shfl_up_sync(full, U.y, 1);
                 lo[f] = mk(lane == 0 ? zlv : left, U.x);
-                // odd width: the edge lane's second cell is the right ghost column
-                up[f] = mk(L.x, !IN && edge && t.odd ? zrv : L.y);
+                up[f] = L;
+            }
+            if (!IN && t.zlo == kWallM) {
+                // the wall mirror of the pair's first cell + the ghost's half slope
+                if (lane == 0) {
+#pragma unroll
+                    for (int f = 0; f < 5; ++f) lo[f].x += f == 3 ? -xt[f].x : xt[f].x;
+                }
+            }
+            if (!IN && t.odd && t.zhi != kNormal) {
+                // odd width: the edge lane's second cell is the right ghost
+                // column, which only a face's rule makes differ from its own
+                // prediction
+                if (edge) {
+#pragma unroll
+                    for (int f = 0; f < 5; ++f)
+                        up[f].y = t.zhi == kOut ? up[f].x : s.zr[pm][r][f] + (f == 3 ? -xt[f].x : xt[f].x);
+                }
             }
             face<3, GRAV>(lo, up, t.gh, k, fzv);
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
                 T hi = __shfl_down_sync(full, fzv[f].x, 1);
-                if (edge_even) hi = T(0);   // right edge face: added at the update
+                if (edge) hi = T(0);   // right edge face: added at the update (even width)
                 V dz = vsub(mk(fzv[f].y, hi), fzv[f]);
-                if (zout) dz.x = T(0);
-                // conducting lower z face: the heat of the first column
-                if (f == 4 && zheat) dz.x -= heat4(xt[0].x, xt[4].x, k);
+                if (!IN && zout) dz.x = T(0);
                 nacc[f] = vadd(nacc[f], vsub(ndy[f], dz));
             }
-        }
-        // the last plane of the chunk: its fluxes arrived with the last barrier
-        if (!aborted && active && t.xe - 1 >= t.xs) {
-            V u0[5], u[5], sp;
-            load_own(t.xe - 1, t.xe - t.xs + 1, u0);
-            update(t.xe - 1, u0, u, sp);
-            store(t.xe - 1, u, sp, true);
+            // conducting lower z face: the heat of the first column
+            if (!IN && zheat) nacc[4].x += heat4(xt[0].x, xt[4].x, k);
+            }
+            if (do_upd) {
+                // update of plane m-1, whose last fluxes arrived with the barrier
+                V u[5], sp;
+                if (!IN) load_own(0, l - 2, u0);
+                update(m - 1, u0, tu, u, sp);
+                store(m - 1, u, sp, true);
+            }
         }
     }
 
