@@ -99,7 +99,7 @@ inline bool is_sweep(int kind) { return kind == kFastF32; }
 #endif
 constexpr int kSweepRowsF32 = DG_SWEEP_ROWS_F32;
 constexpr int kMarchRows = 14;   // 16 warps of 128 registers
-constexpr int kMarchRing = 3;    // staged planes
+constexpr int kMarchRing = 2;    // staged planes
 inline int step_tile_rows(int kind) { return is_sweep(kind) ? kSweepRowsF32 : kMarchRows; }
 // Tile columns (z) and the staged box width (2-cell halo each side).
 inline int step_tile_cols(int kind) { return is_sweep(kind) ? 64 : 32; }

@@ -15,13 +15,14 @@
 //   * Owned warps (TY): row y0 + r, lane l the cell z0 + l.
 //   * Halo warp A: the row below the tile, the halo columns left (lanes 0-15)
 //     and right (lanes 16-31) of it, and the TMA copies.
-//   * Halo warp B: the row above, the staged columns outside the lanes'
-//     (conversion only), the face above the tile's top row and the faces on
-//     its right edge.
-// One barrier per plane.  Iteration j, before it: convert plane j + 1; slopes
-// and prediction of plane j; the x face between planes j - 1 and j; publish
-// face states.  After it: update plane j - 1, whose six fluxes are now known,
-// in the reference's summation order; the y and z faces of plane j.
+//   * Halo warp B: the row above, the columns outside those (conversion
+//     only), the face above the tile's top row and the faces on its right
+//     edge.
+// All warps run one loop body (run_warp).  One barrier per plane.  Iteration
+// j, before it: convert plane j + 1; slopes and prediction of plane j; the x
+// face between planes j - 1 and j; publish face states.  After it: update
+// plane j - 1, whose six fluxes are now known, in the reference's summation
+// order; the y and z faces of plane j.
 //
 // What bounds it: the FP64 pipe (2 warp instructions per clock and SM) and,
 // in FP32 with the reference's rounding, issue; the divisions cost most.  The
@@ -96,6 +97,12 @@ struct KeyBounds {
     }
 };
 
+// The plain division of the rare paths, out of line: inlined, the dozens of
+// IEEE divisions behind the range tests made the march's code several times
+// larger than what runs, and its instruction fetches the leading stall.
+__device__ __noinline__ float plain_div(float a, float b) { return a / b; }
+__device__ __noinline__ double plain_div(double a, double b) { return a / b; }
+
 __device__ __forceinline__ float rcp_rn(float x) { return __frcp_rn(x); }
 __device__ __forceinline__ double rcp_rn(double x) { return __drcp_rn(x); }
 
@@ -132,7 +139,13 @@ template <class T> struct RefArith {
             w[3] = vz;
             w[4] = (div_shared(u[4], c.vol, c.inv_vol) - T(0.5) * r * (vx * vx + vy * vy + vz * vz)) * c.gm1;
         } else {
-            Ph::prim(u, w, c);
+            const T r1 = plain_div(u[0], c.vol), rv1 = r1 * c.vol;
+            const T vx = plain_div(u[1], rv1), vy = plain_div(u[2], rv1), vz = plain_div(u[3], rv1);
+            w[0] = r1;
+            w[1] = vx;
+            w[2] = vy;
+            w[3] = vz;
+            w[4] = (plain_div(u[4], c.vol) - T(0.5) * r1 * (vx * vx + vy * vy + vz * vz)) * c.gm1;
         }
     }
     // slopes of the five fields from the lower, own and upper value
@@ -171,7 +184,9 @@ template <class T> struct RefArith {
         }
         if (slow || !kb.safe<T>()) {
 #pragma unroll
-            for (int f = 0; f < 5; ++f) g[f] = Ph::template slope<LIM>(qm[f], q[f], qp[f], c);
+            for (int f = 0; f < 5; ++f)
+                g[f] = LIM == 0 ? plain_div(qp[f] - qm[f], c.two_ds)
+                                : minmod(plain_div(q[f] - qm[f], c.ds), plain_div(qp[f] - q[f], c.ds));
         }
     }
     static __device__ __forceinline__ void predict(const T q[5], const T gx[5], const T gy[5], const T gz[5],
@@ -213,13 +228,13 @@ template <class T> struct RefArith {
         T qk = div_shared(kin, rho_star, y), qxx = div_shared(xx, rho_star, y), qxy = div_shared(xy, rho_star, y),
           qxz = div_shared(xz, rho_star, y), qx = div_shared(mx, rho_star, y);
         if (!(k.safe && safe_divisor(rho_star) && kb.safe<T>())) {
-            el = pl / c.gm1;
-            er = pr / c.gm1;
-            qk = kin / rho_star;
-            qxx = xx / rho_star;
-            qxy = xy / rho_star;
-            qxz = xz / rho_star;
-            qx = mx / rho_star;
+            el = plain_div(pl, c.gm1);
+            er = plain_div(pr, c.gm1);
+            qk = plain_div(kin, rho_star);
+            qxx = plain_div(xx, rho_star);
+            qxy = plain_div(xy, rho_star);
+            qxz = plain_div(xz, rho_star);
+            qx = plain_div(mx, rho_star);
         }
         const T en_left = T(0.5) * (rl * (vxl * vxl + vyl * vyl + vzl * vzl)) + el;
         const T en_right = T(0.5) * (rr * (vxr * vxr + vyr * vyr + vzr * vzr)) + er;
@@ -305,12 +320,13 @@ template <class T, int TY, int R> struct Smem {
     static constexpr int kFieldElems = kRows * kBoxZ;
     static constexpr int kBoxBytes = 5 * kFieldElems * (int)sizeof(T);
     static constexpr int kSlotElems = ((kBoxBytes + 127) / 128) * 128 / (int)sizeof(T);
-    static constexpr int kPbRows = TY + 2;                // primitive rows y0-1 .. y0+TY
     T ring[R * kSlotElems];                               // conserved totals as staged
-    T pb[2][5][kPbRows][kBoxZ];                           // primitives, by plane parity
+    T pb[2][5][kRows][kBoxZ];                             // primitives of the staged cells, by plane parity
+    T colq[2][5][32];                                     // the halo columns' cells, by lane of warp A
     T ypl[2][TY + 1][5][kTileZ];                          // upper y state, rows y0-1 .. y0+TY-1
     T fy[2][TY + 1][5][kTileZ];                           // flux of the lower y face, rows y0 .. y0+TY
     T fz[TY][5][kTileZ + 2];                              // flux of the lower z face (own warp's rows only)
+    T fxl[TY][5][kTileZ];                                 // the lanes' flux of the x face behind
     T ytop[2][5][kTileZ];                                 // top row's xt (wall) or lower state (outflow)
     T zl[2][TY][5];                                       // left halo column: upper z state (wall: +hs)
     T zr[2][TY][5];                                       // right halo column: lower z state (wall: hs)
@@ -367,29 +383,19 @@ template <class T, class P, int TY, int R, int LIM, bool GRAV> struct March {
         for (int f = 0; f < 5; ++f) u[f] = sl[(f * Sm::kRows + ry) * kBoxZ + cz];
         P::prim(u, q, a, k);
     }
-    static __device__ __forceinline__ void store_pb(Sm &s, int par, int row, int col, const T q[5]) {
-#pragma unroll
-        for (int f = 0; f < 5; ++f) s.pb[par][f][row][col] = q[f];
-    }
     static __device__ __forceinline__ void load_pb(Sm &s, int par, int row, int col, T q[5]) {
 #pragma unroll
         for (int f = 0; f < 5; ++f) q[f] = s.pb[par][f][row][col];
     }
     // Slopes of the cell at (row, col) of plane parity par: x from qm, qn; y
-    // from the rows around it (or the given values), z from the columns.
+    // and z from the cells around it.
     static __device__ __forceinline__ void slopes_at(Sm &s, int par, int row, int col, const T qm[5], const T q[5],
-                                                     const T qn[5], const T *ym, const T *yp, const GridArgs<T> &a,
-                                                     const K &k, T gx[5], T gy[5], T gz[5]) {
+                                                     const T qn[5], const GridArgs<T> &a, const K &k, T gx[5], T gy[5],
+                                                     T gz[5]) {
         P::template slopes<LIM>(qm, q, qn, gx, a, k);
         T m[5], p[5];
-        if (ym) {
-#pragma unroll
-            for (int f = 0; f < 5; ++f) m[f] = ym[f];
-        } else load_pb(s, par, row - 1, col, m);
-        if (yp) {
-#pragma unroll
-            for (int f = 0; f < 5; ++f) p[f] = yp[f];
-        } else load_pb(s, par, row + 1, col, p);
+        load_pb(s, par, row - 1, col, m);
+        load_pb(s, par, row + 1, col, p);
         P::template slopes<LIM>(m, q, p, gy, a, k);
         load_pb(s, par, row, col - 1, m);
         load_pb(s, par, row, col + 1, p);
@@ -397,71 +403,114 @@ template <class T, class P, int TY, int R, int LIM, bool GRAV> struct March {
     }
 
     // ---------------------------------------------------------------------
-    // Owned warp: row y0 + r.
+    // The march of one warp.  All warps run the same code on cells of their
+    // own: warp r < TY the cells of row y0 + r, warp A those of the row below
+    // the tile and then those of the halo columns (lane l < 16: left of row l,
+    // else right of row l - 16), warp B those of the row above.  A and B also
+    // convert the staged cells nobody owns.  A loop per role made the kernels
+    // 145 (FP32) to 190 KB of code, and waiting for instructions their leading
+    // stall: 128^3 FP64 472 -> 374 us per step with this one, FP32 292 -> 247
+    // (reference rounding); fused FP64, 93 KB, lost some (251 -> 279 at
+    // 150x97x131).  What a lane carries from plane to plane beyond lox stays in
+    // shared memory for the registers' sake.  Returns the number of planes
+    // warp A requested.
     // ---------------------------------------------------------------------
-    static __device__ void run_owned(Sm &s, const GridArgs<T> &a, const Tile &t, int r, int lane, T &smax) {
+    static __device__ int run_warp(Sm &s, const GridArgs<T> &a, const CUtensorMap *tmap, const Tile &t, int w, int lane,
+                                   T &smax) {
         const unsigned full = 0xffffffffu;
         const K &k = t.k;
-        // lanes past the tile's last column work on its halo columns again,
-        // so that no lane computes on cells outside the grid
+        const bool isa = w == WA, isb = w == WB, own = w < TY, active = own && w < t.vy;
+        const int r = w;
+        // staged row of the warp's cells; the staged columns each lane converts
+        // and computes on: lanes past the tile's last column work on its halo
+        // columns again, so that no lane computes on cells outside the grid
+        const int prow = isa ? 1 : (isb ? t.vy + 2 : r + 2);
         const int ccol = 2 + min(lane, t.vz + 1), col = 2 + min(lane, t.vz);
-        const bool active = r < t.vy, valid = lane < t.vz;
-        const int y = t.y0 + r, z = t.z0 + min(lane, t.vz - 1);
-        const int edge = t.vz - 1;
-        const bool yout = r == 0 && t.ylo == sweep::kOut, ywall = r == 0 && t.ylo == sweep::kWallM;
-        const bool zout = lane == 0 && t.zlo == sweep::kOut;
+        const int crow = min(lane & 15, t.vy - 1), cz = lane < 16 ? 1 : t.vz + 2;   // warp A's halo column cell
+        const int y = t.y0 + r, z = t.z0 + min(lane, t.vz - 1), edge = t.vz - 1;
+        const bool valid = lane < t.vz;
+        const bool yout = own && r == 0 && t.ylo == sweep::kOut, ywall = own && r == 0 && t.ylo == sweep::kWallM;
+        const bool ytop = active && r == t.vy - 1 && t.yhi != sweep::kNormal;
         const bool zheat = lane == 0 && t.zlo == sweep::kWallM && (a.heat & 4);
-        const bool ytop = r == t.vy - 1 && t.yhi != sweep::kNormal;
         const unsigned ybits = active ? image_bits(y, a.ny, a.bc[2], a.bc[3]) : 0;
-        const unsigned zbits = valid ? image_bits(z, a.nz, a.bc[4], a.bc[5]) : 0;
+        const unsigned zbits = active && valid ? image_bits(z, a.nz, a.bc[4], a.bc[5]) : 0;
         const long long cell0 = (long long)y * a.pitch + z;
         const long long plane = (long long)a.ny * a.pitch;
-        // carried along the march: lox, the lower state of the x face ahead;
-        // fxl, the flux of the x face behind
-        T lox[5], fxl[5];
+        const int fidx = isb ? t.vy : r;   // the y face this warp computes
+        int issued = t.np < R ? t.np : R;
+        // carried along the march: lox, the lower state of the x face ahead
+        // (and s.fxl, the flux of the x face behind)
+        T lox[5];
 #pragma unroll
-        for (int f = 0; f < 5; ++f) lox[f] = fxl[f] = T(0);
+        for (int f = 0; f < 5; ++f) lox[f] = T(0);
 
-        bool ok = true;
-        for (int l = 0; l < 2; ++l) {
-            ok = ok && wait_plane(s, l, t.budget);
-            if (ok && active) {
-                T q[5];
-                load_prim(s, l, r + 2, ccol, a, k, q);
-                store_pb(s, (t.xs + l) & 1, r + 1, ccol, q);
-            }
-        }
-        if (!ok) s.abort_flag[t.xs & 1] = 1;
-        fence_proxy_async();
-        barrier();
-        if (s.abort_flag[t.xs & 1]) return;
-        for (int j = t.xs - 1; j <= t.xe; ++j) {
+        // iterations xs-3 and xs-2 only convert planes xs-2 and xs-1
+        for (int j = t.xs - 3; j <= t.xe; ++j) {
             const int l = j - t.xs + 3, pj = j & 1;
             const bool pub = j >= t.xs && j < t.xe;   // plane j's y and z faces belong to this chunk
-            T xt[5], hsy[5], hsz[5], d[5], u0[5];
+            T xt[5], hsx[5], hsy[5], hsz[5], d[5];
             if (upper_stash(a, j)) barrier();
             if (!wait_plane(s, l, t.budget)) s.abort_flag[pj] = 1;
-            if (active) {
-                // plane j-1's totals, for its update after the barrier
-                const T *src = a.src + (long long)(j - 1) * plane + cell0;
+            if (active || !own) {
+                // The cell at planes j and j-1, read before the conversion of
+                // plane j+1 takes plane j-1's place.  Slopes and prediction
+                // always, so that they interleave with the conversion: before
+                // plane xs-1, and for a ghost row of outflow, nothing uses them.
+                T q[5], qm[5], qn[5], gx[5], gy[5], gz[5];
+                load_pb(s, pj, prow, col, q);
+                load_pb(s, pj ^ 1, prow, col, qm);
+                load_prim(s, l, prow, ccol, a, k, qn);
 #pragma unroll
-                for (int f = 0; f < 5; ++f) u0[f] = src[f * a.fstride];
-                T hsx[5];
-                {
-                    T q[5], qm[5], qn[5], gx[5], gy[5], gz[5];
-                    load_pb(s, pj, r + 1, col, q);
-                    load_pb(s, pj ^ 1, r + 1, col, qm);
-                    load_prim(s, l, r + 2, ccol, a, k, qn);
-                    store_pb(s, pj ^ 1, r + 1, ccol, qn);
-                    slopes_at(s, pj, r + 1, col, qm, q, qn, nullptr, nullptr, a, k, gx, gy, gz);
-                    P::predict(q, gx, gy, gz, a, k, xt);
+                for (int f = 0; f < 5; ++f) s.pb[pj ^ 1][f][prow][ccol] = qn[f];
+                slopes_at(s, pj, prow, col, qm, q, qn, a, k, gx, gy, gz);
+                P::predict(q, gx, gy, gz, a, k, xt);
+#pragma unroll
+                for (int f = 0; f < 5; ++f) {
+                    hsx[f] = P::hs(gx[f], a);
+                    hsy[f] = P::hs(gy[f], a);
+                    hsz[f] = P::hs(gz[f], a);
+                }
+                if (!isb && pub) {
+                    const bool wall = isa && t.ylo == sweep::kWallM;   // a ghost row's own half slope
+#pragma unroll
+                    for (int f = 0; f < 5; ++f) s.ypl[pj][prow - 1][f][lane] = wall ? hsy[f] : xt[f] + hsy[f];
+                }
+            }
+            if (!own) {
+                // the staged cells nobody owns: the outermost row (A, B) and the
+                // columns outside the lanes' (B); A's halo column cells last
+#pragma unroll 1
+                for (int task = 1; task < (isa ? 3 : 4); ++task) {
+                    const bool cols = isa && task == 2;
+                    const int row = task == 1 ? (isa ? 0 : t.vy + 3) : (isa ? crow + 2 : 1 + min(lane >> 1, t.vy + 1));
+                    const int cc = task == 1 ? ccol : (isa ? cz : ((lane & 1) ? t.vz + 2 : 0) + task - 2);
+                    T cq[5], cm[5], cn[5];
 #pragma unroll
                     for (int f = 0; f < 5; ++f) {
-                        hsx[f] = P::hs(gx[f], a);
-                        hsy[f] = P::hs(gy[f], a);
-                        hsz[f] = P::hs(gz[f], a);
+                        cq[f] = s.colq[pj][f][lane];
+                        cm[f] = s.colq[pj ^ 1][f][lane];
+                    }
+                    load_prim(s, l, row, cc, a, k, cn);
+#pragma unroll
+                    for (int f = 0; f < 5; ++f) s.pb[pj ^ 1][f][row][cc] = cn[f];
+                    if (!cols) continue;
+#pragma unroll
+                    for (int f = 0; f < 5; ++f) s.colq[pj ^ 1][f][lane] = cn[f];
+                    if (!pub || (t.zlo == sweep::kOut && t.zhi == sweep::kOut)) continue;
+                    T gx[5], gy[5], gz[5], ct[5];
+                    slopes_at(s, pj, row, cc, cm, cq, cn, a, k, gx, gy, gz);
+                    P::predict(cq, gx, gy, gz, a, k, ct);
+                    if ((lane & 15) < t.vy) {
+#pragma unroll
+                        for (int f = 0; f < 5; ++f) {
+                            const T h = P::hs(gz[f], a);
+                            if (lane < 16) s.zl[pj][crow][f] = t.zlo == sweep::kWallM ? h : ct[f] + h;
+                            else s.zr[pj][crow][f] = t.zhi == sweep::kWallM ? h : ct[f] - h;
+                        }
                     }
                 }
+            }
+            if (active && j >= t.xs - 1) {
                 // a wall's ghost plane 1 keeps its own half slope for the
                 // face ahead; an upper ghost plane takes the last plane's
                 // operands, stashed one plane earlier
@@ -495,15 +544,13 @@ template <class T, class P, int TY, int R, int LIM, bool GRAV> struct March {
                     const bool xo = j - 1 == 2 && a.bc[0] == kOutflow;
 #pragma unroll
                     for (int f = 0; f < 5; ++f) {
-                        d[f] = fx[f] - (xo ? fx[f] : fxl[f]);
-                        fxl[f] = fx[f];
+                        d[f] = fx[f] - (xo ? fx[f] : s.fxl[r][f][lane]);
+                        s.fxl[r][f][lane] = fx[f];
                     }
                 }
 #pragma unroll
                 for (int f = 0; f < 5; ++f) lox[f] = j == 1 && wall_lo ? hsx[f] : xt[f] + hsx[f];
                 if (pub) {
-#pragma unroll
-                    for (int f = 0; f < 5; ++f) s.ypl[pj][r + 1][f][lane] = xt[f] + hsy[f];
                     if (ytop) {
 #pragma unroll
                         for (int f = 0; f < 5; ++f) s.ytop[pj][f][lane] = t.yhi == sweep::kOut ? xt[f] - hsy[f] : xt[f];
@@ -519,18 +566,33 @@ template <class T, class P, int TY, int R, int LIM, bool GRAV> struct March {
             }
             fence_proxy_async();
             barrier();
-            if (s.abort_flag[pj]) return;
-            if (!active) continue;
-            if (j > t.xs) {
-                // ---- update of plane j-1
+            if (s.abort_flag[pj]) break;
+            if (isa) {
+                // the barrier freed the slot converted before it
+                const int nl = l + R;
+                if (nl < t.np) {
+                    if (lane == 0) {
+                        mbar_expect_tx(&s.bar[nl % R], Sm::kBoxBytes);
+                        tma_load_4d(slot(s, nl), tmap, t.z0 - 2, t.y0 - 2, t.xs - 2 + nl, 0, &s.bar[nl % R]);
+                    }
+                    issued = nl + 1;
+                }
+                continue;
+            }
+            if (active && j > t.xs) {
+                // ---- update of plane j-1 (its totals loaded here: earlier, they
+                // cost registers that spilled, 400 against 374 us)
                 const int pp = pj ^ 1;
-                T u[5];
+                T u[5], u0[5];
+                const T *src = a.src + (long long)(j - 1) * plane + cell0;
+#pragma unroll
+                for (int f = 0; f < 5; ++f) u0[f] = src[f * a.fstride];
 #pragma unroll
                 for (int f = 0; f < 5; ++f) {
                     const T fyh = s.fy[pp][r + 1][f][lane];
                     const T fyl = yout ? fyh : s.fy[pp][r][f][lane];
                     const T fzh = lane >= edge ? s.fzr[pp][r][f] : s.fz[r][f][lane + 1];
-                    const T fzl = zout ? fzh : s.fz[r][f][lane];
+                    const T fzl = lane == 0 && t.zlo == sweep::kOut ? fzh : s.fz[r][f][lane];
                     u[f] = P::update(u0[f], d[f] + fyh - fyl + fzh - fzl, f, k);
                 }
                 __syncwarp();
@@ -543,18 +605,17 @@ template <class T, class P, int TY, int R, int LIM, bool GRAV> struct March {
                     const unsigned xbits = xu <= 3 || xu >= a.nx - 4 ? image_bits(xu, a.nx, a.bc[0], a.bc[1]) : 0;
                     if (xbits | ybits | zbits) {
                         // ghost images: every combination of the cell and its
-                        // images along the axes, but the cell itself
-                        for (int gx = -1; gx < 4; ++gx) {
-                            if (gx >= 0 && !((xbits >> gx) & 1)) continue;
-                            const int x = gx < 0 ? xu : ghost_at(gx, a.nx);
-                            for (int gy = -1; gy < 4; ++gy) {
-                                if (gy >= 0 && !((ybits >> gy) & 1)) continue;
-                                const int yy = gy < 0 ? y : ghost_at(gy, a.ny);
-                                for (int gz = -1; gz < 4; ++gz) {
-                                    if (gz >= 0 && !((zbits >> gz) & 1)) continue;
-                                    if (gx < 0 && gy < 0 && gz < 0) continue;
-                                    const int zz = gz < 0 ? z : ghost_at(gz, a.nz);
-                                    T *g = a.dst + ((long long)x * a.ny + yy) * a.pitch + zz;
+                        // images along the axes, but the cell itself (bit 0:
+                        // the cell's own index, bit 1 + g: ghost index g)
+                        for (unsigned bx = (xbits & 15u) << 1 | 1u; bx; bx &= bx - 1) {
+                            const int gx = __ffs(bx) - 2;
+                            for (unsigned by = (ybits & 15u) << 1 | 1u; by; by &= by - 1) {
+                                const int gy = __ffs(by) - 2;
+                                for (unsigned bz = (zbits & 15u) << 1 | (gx >= 0 || gy >= 0); bz; bz &= bz - 1) {
+                                    const int gz = __ffs(bz) - 2;
+                                    T *g = a.dst + ((long long)(gx < 0 ? xu : ghost_at(gx, a.nx)) * a.ny +
+                                                    (gy < 0 ? y : ghost_at(gy, a.ny))) * a.pitch +
+                                           (gz < 0 ? z : ghost_at(gz, a.nz));
                                     g[0] = u[0];
                                     g[a.fstride] = gx >= 0 && ((xbits >> (4 + gx)) & 1) ? -u[1] : u[1];
                                     g[2 * a.fstride] = gy >= 0 && ((ybits >> (4 + gy)) & 1) ? -u[2] : u[2];
@@ -567,215 +628,63 @@ template <class T, class P, int TY, int R, int LIM, bool GRAV> struct March {
                 }
                 __syncwarp();
             }
-            if (!pub) continue;
-            // ---- y and z faces of plane j
+            if (!pub || !(active || isb)) continue;
+            // ---- y and z faces of plane j: an owned row's lower y face and its
+            // cells' lower z faces; warp B the face above the top row and the
+            // right edge faces (one row per lane)
             T lo[5], up[5], F[5];
             if (!yout) {
 #pragma unroll
                 for (int f = 0; f < 5; ++f) {
-                    lo[f] = s.ypl[pj][r][f][lane];
+                    lo[f] = s.ypl[pj][fidx][f][lane];
                     // wall ghost row: mirrored prediction of this row + its own half slope
                     if (ywall) lo[f] = mirror(xt[f], f == 2) + lo[f];
                     up[f] = xt[f] - hsy[f];
                 }
+                if (isb && t.yhi != sweep::kNormal) {
+#pragma unroll
+                    for (int f = 0; f < 5; ++f) {
+                        const T x = s.ytop[pj][f][lane];
+                        up[f] = t.yhi == sweep::kOut ? x : mirror(x, f == 2) - hsy[f];
+                    }
+                }
                 P::template face<2, false>(lo, up, T(0), ywall && (a.heat & 2), xt, a, k, F);
 #pragma unroll
-                for (int f = 0; f < 5; ++f) s.fy[pj][r][f][lane] = F[f];
+                for (int f = 0; f < 5; ++f) s.fy[pj][fidx][f][lane] = F[f];
             }
-#pragma unroll
-            for (int f = 0; f < 5; ++f) {
-                const T left = __shfl_up_sync(full, xt[f] + hsz[f], 1);
-                T zlv = s.zl[pj][r][f];
-                if (t.zlo == sweep::kWallM) zlv = mirror(xt[f], f == 3) + zlv;
-                lo[f] = lane == 0 ? zlv : left;
-                up[f] = xt[f] - hsz[f];
-            }
-            P::template face<3, GRAV>(lo, up, t.gh, zheat, xt, a, k, F);
-#pragma unroll
-            for (int f = 0; f < 5; ++f) s.fz[r][f][lane] = F[f];
-            __syncwarp();
-        }
-    }
-
-    // ---------------------------------------------------------------------
-    // Halo warp A: the row below the tile (lanes as columns) and the halo
-    // columns (lane l < 16: left of row l, else right of row l - 16); issues
-    // the TMA copies.  Returns the number of planes it requested.
-    // ---------------------------------------------------------------------
-    static __device__ int run_a(Sm &s, const GridArgs<T> &a, const CUtensorMap *tmap, const Tile &t, int lane) {
-        const K &k = t.k;
-        const int ccol = 2 + min(lane, t.vz + 1), col = 2 + min(lane, t.vz);
-        const int crow = min(lane & 15, t.vy - 1);          // tile row of the lane's halo column cell
-        const int cz = lane < 16 ? 1 : t.vz + 2;            // its buffer column
-        const bool tl = (lane & 15) < t.vy;
-        int issued = t.np < R ? t.np : R;
-        T q2[5], c0[5], cm[5];   // row y0-2; the column cell at planes j and j-1
-        bool ok = true;
-        for (int l = 0; l < 2; ++l) {
-            ok = ok && wait_plane(s, l, t.budget);
-            if (!ok) break;
-            T q[5];
-            load_prim(s, l, 1, ccol, a, k, q);
-            store_pb(s, (t.xs + l) & 1, 0, ccol, q);
-            if (l == 0) load_prim(s, l, crow + 2, cz, a, k, cm);
-            else {
-                load_prim(s, l, crow + 2, cz, a, k, c0);
-                load_prim(s, l, 0, col, a, k, q2);
-            }
-        }
-        if (!ok) s.abort_flag[t.xs & 1] = 1;
-        fence_proxy_async();
-        barrier();
-        if (s.abort_flag[t.xs & 1]) return issued;
-        // a barrier frees the slots of the planes converted before it
-        auto stage = [&](int nl) {
-            if (nl >= t.np) return;
-            if (lane == 0) {
-                mbar_expect_tx(&s.bar[nl % R], Sm::kBoxBytes);
-                tma_load_4d(slot(s, nl), tmap, t.z0 - 2, t.y0 - 2, t.xs - 2 + nl, 0, &s.bar[nl % R]);
-            }
-            issued = nl + 1;
-        };
-        stage(R);
-        stage(R + 1);
-        for (int j = t.xs - 1; j <= t.xe; ++j) {
-            const int l = j - t.xs + 3, pj = j & 1;
-            const bool pub = j >= t.xs && j < t.xe;
-            if (upper_stash(a, j)) barrier();
-            if (!wait_plane(s, l, t.budget)) s.abort_flag[pj] = 1;
-            T qn[5], cn[5], gx[5], gy[5], gz[5], xt[5], qm[5], q[5];
-            load_pb(s, pj ^ 1, 0, col, qm);
-            load_pb(s, pj, 0, col, q);
-            load_prim(s, l, 1, ccol, a, k, qn);
-            store_pb(s, pj ^ 1, 0, ccol, qn);
-            if (pub && t.ylo != sweep::kOut) {
-                slopes_at(s, pj, 0, col, qm, q, qn, q2, nullptr, a, k, gx, gy, gz);
-                if (t.ylo == sweep::kNormal) {
-                    P::predict(q, gx, gy, gz, a, k, xt);
-#pragma unroll
-                    for (int f = 0; f < 5; ++f) s.ypl[pj][0][f][lane] = xt[f] + P::hs(gy[f], a);
-                } else {
-#pragma unroll
-                    for (int f = 0; f < 5; ++f) s.ypl[pj][0][f][lane] = P::hs(gy[f], a);
-                }
-            }
-            load_prim(s, l, 0, col, a, k, q2);
-            load_prim(s, l, crow + 2, cz, a, k, cn);
-            if (pub && !(t.zlo == sweep::kOut && t.zhi == sweep::kOut)) {
-                slopes_at(s, pj, crow + 1, cz, cm, c0, cn, nullptr, nullptr, a, k, gx, gy, gz);
-                P::predict(c0, gx, gy, gz, a, k, xt);
-                if (tl) {
-#pragma unroll
-                    for (int f = 0; f < 5; ++f) {
-                        const T h = P::hs(gz[f], a);
-                        if (lane < 16) s.zl[pj][crow][f] = t.zlo == sweep::kWallM ? h : xt[f] + h;
-                        else s.zr[pj][crow][f] = t.zhi == sweep::kWallM ? h : xt[f] - h;
-                    }
-                }
-            }
-#pragma unroll
-            for (int f = 0; f < 5; ++f) {
-                cm[f] = c0[f];
-                c0[f] = cn[f];
-            }
-            fence_proxy_async();
-            barrier();
-            if (s.abort_flag[pj]) break;
-            stage(l + R);
-        }
-        return issued;
-    }
-
-    // ---------------------------------------------------------------------
-    // Halo warp B: the row above the tile, the staged columns outside the
-    // lanes' columns, the face above the top row and the right edge faces
-    // (one row per lane).
-    // ---------------------------------------------------------------------
-    static __device__ void run_b(Sm &s, const GridArgs<T> &a, const Tile &t, int lane) {
-        const K &k = t.k;
-        const int ccol = 2 + min(lane, t.vz + 1), col = 2 + min(lane, t.vz);
-        const int br = t.vy + 1;   // buffer row of y0 + vy
-        const int orow = min(lane >> 1, br), ocol = (lane & 1) ? t.vz + 2 : 0;   // two outer cells per lane
-        const int erow = min(lane, t.vy - 1);
-        T q2[5], lb[5];
-        auto outer = [&](int l, int par) {
-            T q[5];
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                load_prim(s, l, orow + 1, ocol + c, a, k, q);
-                store_pb(s, par, orow, ocol + c, q);
-            }
-        };
-        bool ok = true;
-        for (int l = 0; l < 2; ++l) {
-            ok = ok && wait_plane(s, l, t.budget);
-            if (!ok) break;
-            T q[5];
-            load_prim(s, l, br + 1, ccol, a, k, q);
-            store_pb(s, (t.xs + l) & 1, br, ccol, q);
-            load_prim(s, l, br + 2, col, a, k, q2);
-            if (l == 1) outer(l, (t.xs + l) & 1);
-        }
-        if (!ok) s.abort_flag[t.xs & 1] = 1;
-        fence_proxy_async();
-        barrier();
-        if (s.abort_flag[t.xs & 1]) return;
-        for (int j = t.xs - 1; j <= t.xe; ++j) {
-            const int l = j - t.xs + 3, pj = j & 1;
-            const bool pub = j >= t.xs && j < t.xe;
-            if (upper_stash(a, j)) barrier();
-            if (!wait_plane(s, l, t.budget)) s.abort_flag[pj] = 1;
-            {
-                T q[5], qm[5], qn[5], gx[5], gy[5], gz[5], xt[5];
-                load_pb(s, pj ^ 1, br, col, qm);
-                load_pb(s, pj, br, col, q);
-                load_prim(s, l, br + 1, ccol, a, k, qn);
-                store_pb(s, pj ^ 1, br, ccol, qn);
-                outer(l, pj ^ 1);
-                if (pub && t.yhi != sweep::kOut) {
-                    slopes_at(s, pj, br, col, qm, q, qn, nullptr, q2, a, k, gx, gy, gz);
-                    if (t.yhi == sweep::kNormal) P::predict(q, gx, gy, gz, a, k, xt);
-#pragma unroll
-                    for (int f = 0; f < 5; ++f) {
-                        const T h = P::hs(gy[f], a);
-                        lb[f] = t.yhi == sweep::kNormal ? xt[f] - h : h;
-                    }
-                }
-                load_prim(s, l, br + 2, col, a, k, q2);
-            }
-            fence_proxy_async();
-            barrier();
-            if (s.abort_flag[pj]) break;
-            if (!pub) continue;
-            T lo[5], up[5], F[5];
-            {   // face (y0+vy-1 | y0+vy)
+            if (isb) {
+                const int er = min(lane, t.vy - 1);
 #pragma unroll
                 for (int f = 0; f < 5; ++f) {
-                    lo[f] = s.ypl[pj][t.vy][f][lane];
-                    if (t.yhi == sweep::kNormal) up[f] = lb[f];
-                    else {
-                        const T x = s.ytop[pj][f][lane];
-                        up[f] = t.yhi == sweep::kOut ? x : mirror(x, f == 2) - lb[f];
-                    }
-                }
-                P::template face<2, false>(lo, up, T(0), false, lo, a, k, F);
-#pragma unroll
-                for (int f = 0; f < 5; ++f) s.fy[pj][t.vy][f][lane] = F[f];
-            }
-            {   // right edge faces
-#pragma unroll
-                for (int f = 0; f < 5; ++f) {
-                    lo[f] = s.zeu[pj][erow][f];
-                    const T zr = s.zr[pj][erow][f], zx = s.zex[pj][erow][f];
+                    lo[f] = s.zeu[pj][er][f];
+                    const T zr = s.zr[pj][er][f], zx = s.zex[pj][er][f];
                     up[f] = t.zhi == sweep::kNormal ? zr : (t.zhi == sweep::kOut ? zx : mirror(zx, f == 3) - zr);
                 }
-                P::template face<3, GRAV>(lo, up, t.ghe, false, lo, a, k, F);
-                if (lane < t.vy) {
+            } else {
 #pragma unroll
-                    for (int f = 0; f < 5; ++f) s.fzr[pj][lane][f] = F[f];
+                for (int f = 0; f < 5; ++f) {
+                    const T left = __shfl_up_sync(full, xt[f] + hsz[f], 1);
+                    lo[f] = lane == 0 ? s.zl[pj][r][f] : left;
+                    up[f] = xt[f] - hsz[f];
+                }
+                if (t.zlo == sweep::kWallM) {
+                    if (lane == 0) {
+#pragma unroll
+                        for (int f = 0; f < 5; ++f) lo[f] = mirror(xt[f], f == 3) + lo[f];
+                    }
                 }
             }
+            P::template face<3, GRAV>(lo, up, isb ? t.ghe : t.gh, own && zheat, xt, a, k, F);
+            if (!isb) {
+#pragma unroll
+                for (int f = 0; f < 5; ++f) s.fz[r][f][lane] = F[f];
+            } else if (lane < t.vy) {
+#pragma unroll
+                for (int f = 0; f < 5; ++f) s.fzr[pj][lane][f] = F[f];
+            }
+            __syncwarp();
         }
+        return issued;
     }
 
     static __device__ void run(const GridArgs<T> &a, const CUtensorMap *tmap, int chunk, unsigned char *raw) {
@@ -825,10 +734,7 @@ template <class T, class P, int TY, int R, int LIM, bool GRAV> struct March {
             }
         }
         T smax = T(0);
-        int issued = 0;
-        if (warp < TY) run_owned(s, a, t, warp, lane, smax);
-        else if (warp == WA) issued = run_a(s, a, tmap, t, lane);
-        else run_b(s, a, t, lane);
+        const int issued = run_warp(s, a, tmap, t, warp, lane, smax);
         __syncthreads();
         if (s.abort_flag[0] | s.abort_flag[1]) {
             if (warp == WA && lane == 0) {

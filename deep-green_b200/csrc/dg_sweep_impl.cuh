@@ -100,7 +100,12 @@ __device__ __forceinline__ float mm(float a, float b) {
     r = fmaxf(r, 0.0f);
     return __int_as_float(__float_as_int(r) | (__float_as_int(a) & (int)0x80000000));
 }
-__device__ __forceinline__ double mm(double a, double b) { return fmin(fmax(b, fmin(a, 0.0)), fmax(a, 0.0)); }
+// FP64: the one of smaller magnitude where the sign bits agree (the clamp form
+// costs four compare-and-select pairs).
+__device__ __forceinline__ double mm(double a, double b) {
+    const double d = fabs(a) < fabs(b) ? a : b;
+    return (__double2hiint(a) ^ __double2hiint(b)) < 0 ? 0.0 : d;
+}
 __device__ __forceinline__ float2 mm(float2 a, float2 b) { return make_float2(mm(a.x, b.x), mm(a.y, b.y)); }
 
 // Slope in cell units (slope * ds) from the backward and forward
