@@ -18,8 +18,8 @@
 //     layout of the tensor cores; each (dy, dz) is that window at a start
 //     address dz rows further.  Positions with z >= Zin-2 wrap into the next
 //     row and are dropped by the epilogue (2 of every Zin positions).
-//   * a block walks along x through a column of tiles (fixed n and p range,
-//     x in a chunk).  Input plane P serves output planes P, P-1 and P-2 (taps
+//   * a block walks along x through columns of tiles (fixed n and p range), an
+//     equal share of all planes per block (Share).  Input plane P serves output planes P, P-1 and P-2 (taps
 //     dx = 0, 1, 2), so each (dy, dz, 16 channels) is ONE MMA with N = 3 COUT
 //     against the weights [W(dx=2) | W(dx=1) | W(dx=0)]: its three column
 //     blocks land in the TMEM accumulators of output planes P-2, P-1, P,
@@ -28,7 +28,7 @@
 //     drains its slot and zeroes it for reuse, so every MMA accumulates.
 //     Each input plane is read from shared memory once, by 9 x CIN/16 MMAs.
 //   * input planes arrive by TMA into a ring of shared-memory slots (3
-//     windows each); planes at the start of a chunk produce two partial
+//     windows each); planes at the start of a column or share produce two partial
 //     outputs that are drained and discarded.
 //   * all weights stay in shared memory, packed on the host as
 //     [dy, dz][dx' = 2-dx][co][ci] rows, swizzled like the windows.
@@ -36,9 +36,10 @@
 //     plane's MMAs (one thread each, descriptors advanced by constant
 //     offsets) into their own ring of accumulators -- a single thread's
 //     dependent issue loop, not the tensor core, would otherwise set the
-//     pace; warps 3-10 drain both rings (two warps per TMEM sub-partition,
-//     each half of the columns: sum, bias, GELU / GELU', BF16 or FP32
-//     stores) in a fixed order, so results do not depend on timing.
+//     pace; two groups of eight warps drain both rings in turn, a plane each
+//     (two warps per TMEM sub-partition, each half of the columns: sum, bias,
+//     GELU / GELU', BF16 or FP32 stores) in a fixed order, so results do not
+//     depend on timing.
 //   The input-gradient of a layer is the same kernel run on the output
 //   gradient zero-padded by 2 with the taps flipped and W transposed.
 //
@@ -69,7 +70,12 @@ constexpr int kBox = 3 * kWz * 16;         // one TMA box: 3 rows of kWz positio
 constexpr int kStages = 2;
 constexpr int kConvThreads = 192;          // weight gradient: 6 warps (TMA, MMA, 4 x epilogue)
 constexpr int kIssuers = 2;                // forward: MMA-issuing warps, each with its own accumulators
-constexpr int kFwdThreads = 32 * (1 + kIssuers + 8);   // forward: TMA, issuers, 8 x epilogue
+// Forward epilogue: warps in groups of 8 (two per TMEM sub-partition, each
+// half of the columns) that take the planes in turn.  One group spent the
+// whole period of a 16-channel layer on its chain of wait, TMEM load, GELU and
+// store.
+constexpr int kEpiGroups = 2;
+constexpr int kFwdThreads = 32 * (1 + kIssuers + 8 * kEpiGroups);   // forward: TMA, issuers, epilogue
 // Forward kernel: TMEM accumulator slots (output planes) of one issuer's ring;
 // the rings of all issuers fill the 512 TMEM columns.
 template <int COUT> constexpr int fwd_ring() { return 512 / (kIssuers * COUT); }
@@ -82,9 +88,7 @@ struct ConvArgs {
     int nb, xi, yi, zi;             // input extents
     int xo, yo, zo;                 // output extents (input - 2)
     int tpp;                        // tiles per (n, x) plane: ceil(yo * zi / kM)
-    int xchunk;                     // planes of x per work unit
-    int nxc;                        // x chunks: ceil(xo / xchunk)
-    int nunits;                     // work units nb * tpp * nxc: (n, p range, x chunk)
+    long long work;                 // output planes of all columns: nb * tpp * xo
     int ox, oy, oz, off;            // extents of the output buffer and offset of the output region in it
     const float *bias;              // [COUT] (kEpiGelu, kEpiLinear)
     __nv_bfloat16 *out_a;           // BF16 output: activation (kEpiGelu) or gradient (kEpiDGelu)
@@ -101,6 +105,48 @@ struct WgradArgs {
     int nunits;                     // work units (n, x, z segment, y chunk): nb * xo * nseg * nyc
     float *part;                    // per block: [COUT][CIN][27] weight partials then [COUT] bias partials
     unsigned *status;
+};
+
+// A block's share of the work: columns of `len` steps, `work` steps in all.
+// As many rounds of whole columns as every block gets one of, neighbouring
+// columns at neighbouring steps (each block starts a column a little further
+// in and wraps around), so that the rows they share come from L2 without all
+// blocks asking for one plane at once; then an equal range of the remaining
+// columns' steps.  next() gives a column, its first step and the count of
+// steps in it.  (Fixed chunks of 64 planes left a third of the SMs idle at the
+// end of a layer of 200^3, and half of them on columns a little longer than a
+// chunk, whose short remainders all fell to the odd blocks, as on training
+// crops.)  A column's outputs do not depend on the split.
+struct Share {
+    long long column, pos, end;
+    int len, rounds, shift;
+    bool wrapped = false;
+    __device__ __forceinline__ Share(long long work, int len_)
+        : column(blockIdx.x), len(len_), shift((int)((long long)len_ * blockIdx.x / gridDim.x)) {
+        const long long columns = work / len, whole = columns / gridDim.x * gridDim.x, rest = (columns - whole) * len;
+        rounds = (int)(columns / gridDim.x);
+        pos = whole * len + rest * blockIdx.x / gridDim.x;
+        end = whole * len + rest * (blockIdx.x + 1) / gridDim.x;
+    }
+    __device__ __forceinline__ bool next(long long &col, int &first, int &count) {
+        if (rounds > 0) {
+            col = column;
+            first = wrapped ? 0 : shift;
+            count = wrapped ? shift : len - shift;
+            if (wrapped || shift == 0) {
+                --rounds;
+                column += gridDim.x;
+                wrapped = false;
+            } else wrapped = true;
+            return true;
+        }
+        if (pos >= end) return false;
+        col = pos / len;
+        first = (int)(pos - col * len);
+        count = (int)min((long long)(len - first), end - pos);
+        pos += count;
+        return true;
+    }
 };
 
 __device__ __forceinline__ unsigned char *align128(unsigned char *p) {
@@ -124,9 +170,16 @@ __device__ __forceinline__ float tanh_approx(float x) {
 constexpr float kGeluC0 = 0.79788456080286536f;   // sqrt(2 / pi)
 constexpr float kGeluC1 = 0.044715f;
 
-__device__ __forceinline__ float gelu(float x) {
-    const float t = tanh_approx(kGeluC0 * (x + kGeluC1 * x * x * x));
-    return 0.5f * x * (1.0f + t);
+// Two values at once, the same operations in the same order on packed FP32
+// instructions: the epilogue's issue slots are what the MMA issuers compete
+// for (without its GELU a 32-channel layer of 260^3 takes 0.81 instead of 0.91
+// ms).
+__device__ __forceinline__ float2 gelu2(float2 x) {
+    auto splat = [](float v) { return make_float2(v, v); };
+    const float2 c = __fmul2_rn(__fmul2_rn(splat(kGeluC1), x), x);
+    const float2 a = __fmul2_rn(splat(kGeluC0), __ffma2_rn(c, x, x));
+    const float2 t = make_float2(tanh_approx(a.x), tanh_approx(a.y));
+    return __fmul2_rn(__fmul2_rn(splat(0.5f), x), __fadd2_rn(splat(1.0f), t));
 }
 
 __device__ __forceinline__ float gelu_grad(float x) {
@@ -209,7 +262,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     constexpr int R = fwd_ring<COUT>();          // slots of one issuer's ring
     constexpr int RING = R * COUT;               // TMEM columns of one issuer's ring
     constexpr uint32_t TCOLS = kIssuers * RING;  // 512
-    static_assert(TCOLS == 512 && R >= 8, "ring layout");
+    static_assert(TCOLS == 512 && R >= 8 && R % kEpiGroups == 0, "ring layout");
     constexpr uint32_t ID3 = tc::idesc_bf16(kM, 3 * COUT, 0, 0);
     constexpr uint32_t ID2 = tc::idesc_bf16(kM, 2 * COUT, 0, 0);
     constexpr uint32_t ID1 = tc::idesc_bf16(kM, COUT, 0, 0);
@@ -244,13 +297,14 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     tc::fence_after();
     const uint32_t tbase = *tslot;
     const int q = warp & 3;                      // epilogue: TMEM sub-partition (lanes 32q..32q+31)
-    const int c0 = ((warp - EPI0) >> 2) * NC;    // epilogue: first column of this warp's half
+    const int c0 = (((warp - EPI0) >> 2) & 1) * NC;   // epilogue: first column of this warp's half
+    const int grp = (warp - EPI0) >> 3;          // epilogue: takes the slots g with g % kEpiGroups == grp
     if (warp >= EPI0) {
         // every accumulator starts at zero: all MMAs accumulate
         float zero[NC];
 #pragma unroll
         for (int c = 0; c < NC; ++c) zero[c] = 0.0f;
-        for (int sl = 0; sl < kIssuers * R; ++sl) {
+        for (int sl = grp; sl < kIssuers * R; sl += kEpiGroups) {
             const uint32_t ta = tbase + ((uint32_t)(32 * q) << 16) + (uint32_t)(sl * COUT + c0);
             if constexpr (NC == 16) tc::tmem_st16(ta, zero);
             else tc::tmem_st8(ta, zero);
@@ -270,11 +324,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             mbar_expect_tx(wbar, L::WB);
             tc::bulk_load(wsm, wpack, L::WB, wbar);
             long long g = 0;                      // planes issued by this block
-            for (int unit = blockIdx.x; ok && unit < a.nunits; unit += gridDim.x) {
-                const int xc = unit % a.nxc, r = unit / a.nxc;
-                const int pt = r % a.tpp, b = r / a.tpp;
-                const int x0 = xc * a.xchunk, len = min(a.xchunk, a.xo - x0);
-                const int p0 = pt * kM;
+            Share share(a.work, a.xo);
+            long long column;
+            int x0, len;
+            while (ok && share.next(column, x0, len)) {
+                const int b = (int)(column / a.tpp), p0 = (int)(column - (long long)b * a.tpp) * kM;
                 for (int k = 0; k < len + 2; ++k, ++g) {
                     const int slot = (int)(g % kSlots);
                     const long long use = g / kSlots;
@@ -301,9 +355,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         long long g = 0;                      // input planes consumed = output slots completed
         const uint64_t b0 = tc::sdesc_sw(smem_u32(wsm), ROW);
         const uint32_t rbase = tbase + (uint32_t)(me * RING);
-        for (int unit = blockIdx.x; ok && unit < a.nunits; unit += gridDim.x) {
-            const int xc = unit % a.nxc;
-            const int len = min(a.xchunk, a.xo - xc * a.xchunk);
+        Share share(a.work, a.xo);
+        long long column;
+        int x0, len;
+        while (ok && share.next(column, x0, len)) {
             for (int k = 0; k < len + 2; ++k, ++g) {
                 const int ps = (int)(g % kSlots);
                 bool got = tc::mbar_sleep_wait(full + ps, (uint32_t)((g / kSlots) & 1), kWaitBudget);
@@ -366,14 +421,28 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         ok &= warp_wait(drain + me, 0);
     } else {
         long long g = 0;
-        for (int unit = blockIdx.x; ok && unit < a.nunits; unit += gridDim.x) {
-            const int xc = unit % a.nxc, r = unit / a.nxc;
-            const int pt = r % a.tpp, b = r / a.tpp;
-            const int x0 = xc * a.xchunk, len = min(a.xchunk, a.xo - x0);
-            const int p = pt * kM + 32 * q + lane;
+        Share share(a.work, a.xo);
+        long long column;
+        int x0, len;
+        while (ok && share.next(column, x0, len)) {
+            const int b = (int)(column / a.tpp);
+            const int p = (int)(column - (long long)b * a.tpp) * kM + 32 * q + lane;
             const int y = p / a.zi, z = p - y * a.zi;
             const bool valid = y < a.yo && z < a.zo;
+            auto add2 = [](float *s, const float *t) {
+#pragma unroll
+                for (int c = 0; c < NC; c += 2) {
+                    const float2 r = __fadd2_rn(make_float2(s[c], s[c + 1]), make_float2(t[c], t[c + 1]));
+                    s[c] = r.x;
+                    s[c + 1] = r.y;
+                }
+            };
+            // position of the column's plane 0 in the outputs
+            const long long o0 = ((((long long)b * a.ox + x0 + a.off) * a.oy + y + a.off) * a.oz + z + a.off) * COUT + c0;
+            const long long d0 = ((((long long)b * a.xo + x0) * a.yo + y) * a.zo + z) * COUT + c0;
+            const int ostep = a.oy * a.oz * COUT, dstep = a.yo * a.zo * COUT;
             for (int k = 0; k < len + 2; ++k, ++g) {
+                if ((int)(g % kEpiGroups) != grp) continue;
                 const int sl = (int)(g % R);
                 if (!warp_wait(tfull + sl, (uint32_t)((g / R) & 1))) {
                     ok = false;
@@ -404,30 +473,27 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                 // slot g holds output plane x0 + k - 2 of this chunk when k >= 2;
                 // the first two slots of a chunk mix planes of two chunks
                 if (k < 2 || !valid) continue;
-                if constexpr (kIssuers == 2)
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) v[c] += v2[c];
+                if constexpr (kIssuers == 2) add2(v, v2);
 
-                const int x = x0 + k - 2;
-                const long long o =
-                    ((((long long)b * a.ox + x + a.off) * a.oy + y + a.off) * a.oz + z + a.off) * COUT + c0;
-                const long long dn = ((((long long)b * a.xo + x) * a.yo + y) * a.zo + z) * COUT + c0;
+                const long long o = o0 + (long long)(k - 2) * ostep, dn = d0 + (long long)(k - 2) * dstep;
                 // one 32-byte store per lane and tensor where the columns allow
                 // (COUT 32: 16 BF16 columns; COUT 16: 8 FP32 columns)
                 if constexpr (EPI == kEpiGelu) {
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) v[c] += bias[c];
+                    add2(v, bias);
                     if (a.out_z) {
                         if constexpr (NC == 16) store16_bf16(a.out_z + dn, v);
                         else store_bf16(a.out_z + dn, v, NC);
                     }
 #pragma unroll
-                    for (int c = 0; c < NC; ++c) v[c] = gelu(v[c]);
+                    for (int c = 0; c < NC; c += 2) {
+                        const float2 g2 = gelu2(make_float2(v[c], v[c + 1]));
+                        v[c] = g2.x;
+                        v[c + 1] = g2.y;
+                    }
                     if constexpr (NC == 16) store16_bf16(a.out_a + o, v);
                     else store_bf16(a.out_a + o, v, NC);
                 } else if constexpr (EPI == kEpiLinear) {
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) v[c] += bias[c];
+                    add2(v, bias);
                     if constexpr (NC == 8) {
                         store8_f32(a.out_f + o, v);
                     } else {

@@ -370,23 +370,10 @@ cudaError_t launch_conv(dg_net *net, const void *in, int nb, int xi, int yi, int
     a.xi = xi; a.yi = yi; a.zi = zi;
     a.xo = xi - 2; a.yo = yi - 2; a.zo = zi - 2;
     a.tpp = (a.yo * zi + kM - 1) / kM;
-    // blocks holding all 512 TMEM columns cannot share an SM
-    const int per_sm = 1;
-    const int slots = per_sm * net->nsm;
-    // longest x chunk (fewest re-loaded planes) that still gives every block
-    // a few work units
-    a.xchunk = 8;
-    for (int len : {64, 32, 16}) {
-        const long long units = (long long)nb * a.tpp * ((a.xo + len - 1) / len);
-        if (units >= 4LL * slots) {
-            a.xchunk = len;
-            break;
-        }
-    }
-    a.nxc = (a.xo + a.xchunk - 1) / a.xchunk;
-    a.nunits = nb * a.tpp * a.nxc;
+    a.work = (long long)nb * a.tpp * a.xo;
     a.status = net->status;
-    const int grid = std::max(1, std::min(a.nunits, slots));
+    // one block per SM (a block holds all 512 TMEM columns)
+    const int grid = (int)std::min<long long>(a.work, net->nsm);
     kern<<<grid, kFwdThreads, L::BYTES, st>>>(m, w, a);
     return cudaGetLastError();
 }
@@ -405,7 +392,9 @@ cudaError_t launch_wgrad(dg_net *net, const void *x_in, const void *g_pad, int n
     WgradArgs a;
     a.nb = nb; a.xo = xo; a.yo = yo; a.zo = zo;
     a.nseg = (zo + kM - 1) / kM;
-    // columns along y split into chunks so that every block gets ~6 units
+    // columns along y split into chunks so that every block gets ~6 units.  The
+    // split decides which rows a block sums on its accumulators before the
+    // blocks' partials are added: another one changes the gradients by ~3e-4.
     const long long cols = (long long)nb * xo * a.nseg;
     const long long want = 6LL * net->nsm;
     int nyc = (int)std::min<long long>(yo, std::max<long long>(1, (want + cols - 1) / cols));
