@@ -128,37 +128,55 @@ bool map_wgrad(CUtensorMap *m, const void *base, int c, int n, int x, int y, int
 // Weight operand of the forward kernel: rows r = ((dy, dz), dx' = 2 - dx, co)
 // of kin channels (2 kin bytes), in the tensor cores' swizzled K-major layout:
 // the 16-byte chunk c of row r is stored at chunk c ^ ((r * row >> 7) &
-// (row/16 - 1)) (the shared-memory copy starts 1024-byte aligned).  `flip`
-// packs the input-gradient convolution instead, with cin' = cout, cout' =
-// cin and W'_t[co'][ci'] = W_{26-t}[ci'][co'] (taps flipped, channels
-// transposed).
-__global__ void pack_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ out, int cin, int cout,
-                            int flip) {
-    const int kin = flip ? cout : cin, kout = flip ? cin : cout;   // channels of the packed convolution
-    const int row = 2 * kin;
-    const int total = 27 * kin * kout;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const int r = i / kin, pos = i % kin;
-        const int mask = ((r * row) >> 7) & (row / 16 - 1);
-        const int ci = (((pos >> 3) ^ mask) << 3) | (pos & 7);     // logical channel stored here
-        const int n = r % (3 * kout), t9 = r / (3 * kout);
-        const int dx = 2 - n / kout, co = n % kout;
-        const int t = dx * 9 + t9;
-        const float v = flip ? w[((size_t)ci * cin + co) * 27 + (26 - t)] : w[((size_t)co * cin + ci) * 27 + t];
-        out[i] = __float2bfloat16_rn(v);
-    }
+// (row/16 - 1)) (the shared-memory copy starts 1024-byte aligned).  Index of
+// the value of tap t (dx, dy, dz), output channel co and input channel ci of
+// a convolution kin -> kout.
+__device__ __forceinline__ int packed_index(int t, int co, int ci, int kin, int kout) {
+    const int dx = t / 9, t9 = t - 9 * dx, row = 2 * kin;
+    const int r = t9 * 3 * kout + (2 - dx) * kout + co;
+    const int mask = ((r * row) >> 7) & (row / 16 - 1);
+    return r * kin + ((((ci >> 3) ^ mask) << 3) | (ci & 7));
 }
 
-// Fixed-order sum of the per-block weight-gradient partials.
-__global__ void wgrad_reduce_kernel(const float *__restrict__ part, int nblocks, int cin, int cout, float *gw,
-                                    float *gb) {
-    const int nw = cout * cin * 27, row = nw + cout;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < row; i += gridDim.x * blockDim.x) {
-        float s = 0.0f;
-        for (int k = 0; k < nblocks; ++k) s += part[(size_t)k * row + i];
-        if (i < nw) gw[i] = s;
-        else gb[i - nw] = s;
-    }
+// All parameters of the network, as the kernels that walk them see them.
+struct ParamTable {
+    float *p[8], *g[8], *m[8], *v[8];   // weights of layers 0-3, then biases
+    __nv_bfloat16 *wf[4], *wd[4];       // packings of the weights (wd of layer 0: none)
+    int cin[4], cout[4];
+    int first[9];                       // first value of each of the 8 arrays in the flat order
+};
+
+// A weight into the forward packing and into that of the input-gradient
+// convolution (cin' = cout, cout' = cin, taps flipped, channels transposed:
+// W'_t[co'][ci'] = W_{26-t}[ci'][co']).
+__device__ __forceinline__ void pack_weight(const ParamTable &t, int l, int i, float w) {
+    const int cin = t.cin[l], cout = t.cout[l], tap = i % 27, c = i / 27, ci = c % cin, co = c / cin;
+    const __nv_bfloat16 h = __float2bfloat16_rn(w);
+    t.wf[l][packed_index(tap, co, ci, cin, cout)] = h;
+    if (t.wd[l]) t.wd[l][packed_index(26 - tap, ci, co, cout, cin)] = h;
+}
+
+__global__ void __launch_bounds__(256) pack_kernel(ParamTable t) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= t.first[4]) return;
+    int l = 0;
+    while (i >= t.first[l + 1]) ++l;
+    pack_weight(t, l, i - t.first[l], t.p[l][i - t.first[l]]);
+}
+
+// Fixed-order sum of the per-block weight-gradient partials: one thread per
+// value, the blocks' rows in order, a quarter of 148 of them loaded ahead of
+// their additions (27,680 values x 148 blocks: 26 us with two values and one
+// load in flight per thread, 16 us with 8 loads, 11 us so).
+__global__ void __launch_bounds__(128) wgrad_reduce_kernel(const float *__restrict__ part, int nblocks, int cin,
+                                                           int cout, float *gw, float *gb) {
+    const int nw = cout * cin * 27, row = nw + cout, i = blockIdx.x * 128 + threadIdx.x;
+    if (i >= row) return;
+    float s = 0.0f;
+#pragma unroll 37
+    for (int k = 0; k < nblocks; ++k) s += part[(size_t)k * row + i];
+    if (i < nw) gw[i] = s;
+    else gb[i - nw] = s;
 }
 
 // Loss and its gradient w.r.t. the network output: L = mean (out - t)^2 over
@@ -270,14 +288,27 @@ __global__ void flux_residual_kernel(const float *__restrict__ out, const float 
         const int ix = r % s;
         const int b = (int)(r / s);
         const long long c0 = ((((long long)b * o + ix + 1) * o + iy + 1) * o + iz + 1) * kIO;
-        const long long lo[3] = {c0 - (long long)o * o * kIO, c0 - (long long)o * kIO, c0 - kIO};
+        // rows of 16 floats read in float4 / float2 pieces (both arrays start on
+        // 16 bytes: the workspace, and the entry point's check of the target);
+        // as scalars 8 crops of 64^3 took 140 us, so 61
+        const float4 *own = reinterpret_cast<const float4 *>(out + c0);
+        const float4 *px = reinterpret_cast<const float4 *>(out + c0 - (long long)o * o * kIO);
+        const float4 *py = reinterpret_cast<const float4 *>(out + c0 - (long long)o * kIO);
+        const float4 *pz = reinterpret_cast<const float4 *>(out + c0 - kIO);
+        const float4 *pt = reinterpret_cast<const float4 *>(tgt + (size_t)v * kIO);
+        const float4 f0 = own[0], f1 = own[1], f2 = own[2], f3 = own[3], x0 = px[0], y1 = py[1], z3 = pz[3], t0 = pt[0];
+        const float x4 = reinterpret_cast<const float *>(px)[4], t4 = reinterpret_cast<const float *>(pt)[4];
+        const float2 y8 = reinterpret_cast<const float2 *>(py)[4], z10 = reinterpret_cast<const float2 *>(pz)[5];
+        const float hi[15] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w, f2.x, f2.y, f2.z, f2.w, f3.x, f3.y, f3.z};
+        const float lo[15] = {x0.x, x0.y, x0.z, x0.w, x4, y1.y, y1.z, y1.w, y8.x, y8.y, z10.x, z10.y, z3.x, z3.y, z3.z};
+        const float tg[5] = {t0.x, t0.y, t0.z, t0.w, t4};
+        const float wb = wsample[b];
 #pragma unroll
         for (int c = 0; c < 5; ++c) {
             float du = 0.0f;
 #pragma unroll
-            for (int d = 0; d < 3; ++d) du += out[c0 + 5 * d + c] - out[lo[d] + 5 * d + c];
-            const float res = du - tgt[(size_t)v * kIO + c];
-            const float wb = wsample[b];
+            for (int d = 0; d < 3; ++d) du += hi[5 * d + c] - lo[5 * d + c];
+            const float res = du - tg[c];
             acc += (double)wb * res * res;
             gbuf[(size_t)v * 5 + c] = scale * wb * res;
         }
@@ -324,17 +355,24 @@ __global__ void flux_grad_kernel(const float *__restrict__ gbuf, int n, int s, _
     }
 }
 
-__global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
-                            float *__restrict__ v, int count, float lr, float b1, float b2, float eps, float c1,
-                            float c2) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * gi;
-        const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    }
+// Adam on every parameter, and the new weights straight into their packings
+// (one launch in place of eight updates and seven packings, ~3 us each).
+__global__ void __launch_bounds__(256) adam_kernel(ParamTable t, float lr, float b1, float b2, float eps, float c1,
+                                                   float c2) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= t.first[8]) return;
+    int l = 0;
+    while (i >= t.first[l + 1]) ++l;
+    const int k = i - t.first[l];
+    const float gi = t.g[l][k];
+    const float mi = b1 * t.m[l][k] + (1.0f - b1) * gi;
+    const float vi = b2 * t.v[l][k] + (1.0f - b2) * gi * gi;
+    t.m[l][k] = mi;
+    t.v[l][k] = vi;
+    float p = t.p[l][k];
+    p -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    t.p[l][k] = p;
+    if (l < 4) pack_weight(t, l, k, p);
 }
 
 // Unpadded copy of the interior of a BF16 tensor padded by 2 (test access).
@@ -386,12 +424,12 @@ cudaError_t launch_wgrad(dg_net *net, const void *x_in, const void *g_pad, int n
     static std::atomic<unsigned long long> attr_set{0};
     const cudaError_t attr_err = ensure_dynamic_smem(kern, L::BYTES, attr_set);
     if (attr_err != cudaSuccess) return attr_err;
-    CUtensorMap mx, mg;
-    if (!map_wgrad(&mx, x_in, CIN, nb, xo + 2, yo + 2, zo + 2, kWz, 1)) return cudaErrorInvalidValue;
-    if (!map_wgrad(&mg, g_pad, COUT, nb, xo + 4, yo + 4, zo + 4, kM, 1)) return cudaErrorInvalidValue;
     WgradArgs a;
     a.nb = nb; a.xo = xo; a.yo = yo; a.zo = zo;
     a.nseg = (zo + kM - 1) / kM;
+    CUtensorMap mx, mg;
+    if (!map_wgrad(&mx, x_in, CIN, nb, xo + 2, yo + 2, zo + 2, kWz, 1)) return cudaErrorInvalidValue;
+    if (!map_wgrad(&mg, g_pad, COUT, nb, xo + 4, yo + 4, zo + 4, kM, 1)) return cudaErrorInvalidValue;
     // columns along y split into chunks so that every block gets ~6 units.  The
     // split decides which rows a block sums on its accumulators before the
     // blocks' partials are added: another one changes the gradients by ~3e-4.
@@ -407,15 +445,32 @@ cudaError_t launch_wgrad(dg_net *net, const void *x_in, const void *g_pad, int n
     kern<<<grid, kConvThreads, L::BYTES, net->stream>>>(mx, mg, a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    wgrad_reduce_kernel<<<64, 256, 0, net->stream>>>(net->wpart, grid, CIN, COUT, gw, gb);
+    wgrad_reduce_kernel<<<(COUT * CIN * 27 + COUT + 127) / 128, 128, 0, net->stream>>>(net->wpart, grid, CIN, COUT, gw,
+                                                                                  gb);
     return cudaGetLastError();
 }
 
-int repack(dg_net *net) {
+ParamTable param_table(dg_net *net) {
+    ParamTable t;
+    t.first[0] = 0;
     for (int l = 0; l < 4; ++l) {
-        pack_kernel<<<64, 256, 0, net->stream>>>(net->w[l], net->wf[l], kCin[l], kCout[l], 0);
-        if (l > 0) pack_kernel<<<64, 256, 0, net->stream>>>(net->w[l], net->wd[l], kCin[l], kCout[l], 1);
+        float *const w[4] = {net->w[l], net->gw[l], net->mw[l], net->vw[l]};
+        float *const b[4] = {net->b[l], net->gb[l], net->mb[l], net->vb[l]};
+        t.p[l] = w[0]; t.g[l] = w[1]; t.m[l] = w[2]; t.v[l] = w[3];
+        t.p[4 + l] = b[0]; t.g[4 + l] = b[1]; t.m[4 + l] = b[2]; t.v[4 + l] = b[3];
+        t.wf[l] = net->wf[l];
+        t.wd[l] = net->wd[l];
+        t.cin[l] = kCin[l];
+        t.cout[l] = kCout[l];
+        t.first[l + 1] = t.first[l] + 27 * kCin[l] * kCout[l];
     }
+    for (int l = 0; l < 4; ++l) t.first[5 + l] = t.first[4 + l] + kCout[l];
+    return t;
+}
+
+int repack(dg_net *net) {
+    const ParamTable t = param_table(net);
+    pack_kernel<<<(t.first[4] + 255) / 256, 256, 0, net->stream>>>(t);
     NET_CUDA(net, cudaGetLastError());
     return DG_OK;
 }
@@ -807,15 +862,10 @@ int32_t dg_net_adam_step(dg_net *net, float lr, float beta1, float beta2, float 
     net->adam_t += 1;
     const float c1 = (float)(1.0 - std::pow((double)beta1, (double)net->adam_t));
     const float c2 = (float)(1.0 - std::pow((double)beta2, (double)net->adam_t));
-    for (int l = 0; l < 4; ++l) {
-        const int nw = 27 * kCin[l] * kCout[l];
-        adam_kernel<<<64, 256, 0, net->stream>>>(net->w[l], net->gw[l], net->mw[l], net->vw[l], nw, lr, beta1, beta2,
-                                                 eps, c1, c2);
-        adam_kernel<<<1, 64, 0, net->stream>>>(net->b[l], net->gb[l], net->mb[l], net->vb[l], kCout[l], lr, beta1,
-                                               beta2, eps, c1, c2);
-    }
+    const ParamTable t = param_table(net);
+    adam_kernel<<<(t.first[8] + 255) / 256, 256, 0, net->stream>>>(t, lr, beta1, beta2, eps, c1, c2);
     NET_CUDA(net, cudaGetLastError());
-    return repack(net);
+    return DG_OK;
 }
 
 int32_t dg_net_get_tensor(dg_net *net, int32_t layer, int32_t which, void *host, uint64_t bytes) {
