@@ -48,9 +48,15 @@
 // accumulators; the M rows are (dx in 0..3, ci) -- dx = 3 is a block of
 // ones, which turns its rows into the bias gradient sum_v dZ[v][co].  Both
 // operands are MN-major: K is the position along z, 16 bytes apart.  A block
-// walks a column of output rows along y (one tile = one row segment of kM
-// positions): the input rows y, y+1, y+2 that tile y reads sit in a ring of
-// 4 rows per (dx, channel group), so each tile brings one new input row.
+// walks a column of output rows along y (one tile = one row segment of at
+// most kM positions): the input rows y, y+1, y+2 that tile y reads sit in a
+// ring per (dx, channel group), so each tile brings one new input row.  With
+// 16 input channels M is 64.  Three warps issue the MMAs, each those of one
+// dy, into accumulators of their own: one warp's issue loop, not the operand
+// reads, had set the pace.  Layers of 8 crops of 64^3, per launch (32 -> 32,
+// 32 -> 16, 16 -> 32): 450, 396, 396 us with one issuer, 136-position copies
+// and four ring rows; 321, 282, 204 us so.  (The operand reads of the 32 -> 32
+// layer take ~245 us: 5 KB of shared memory per MMA.)
 //
 // Every wait is bounded (~2 s); a timeout sets a status bit and the block
 // drains its copies and MMAs and frees its TMEM before returning.
@@ -66,10 +72,11 @@ namespace net {
 
 constexpr int kM = 128;                    // positions per tile (MMA M)
 constexpr int kWz = 136;                   // window positions per row (>= kM + 2; 128-byte boxes)
-constexpr int kBox = 3 * kWz * 16;         // one TMA box: 3 rows of kWz positions x 8 channels (6528 B)
-constexpr int kStages = 2;
-constexpr int kConvThreads = 192;          // weight gradient: 6 warps (TMA, MMA, 4 x epilogue)
+constexpr int kMaxSmem = 227 * 1024;       // shared memory of one block
+constexpr int kMaxRows = 10;               // weight gradient: most input rows in a ring
 constexpr int kIssuers = 2;                // forward: MMA-issuing warps, each with its own accumulators
+constexpr int kWIssuers = 3;               // weight gradient: MMA-issuing warps, a third of the accumulators each
+constexpr int kConvThreads = 32 * (1 + kWIssuers + 4);  // weight gradient: TMA, issuers, epilogue
 // Forward epilogue: warps in groups of 8 (two per TMEM sub-partition, each
 // half of the columns) that take the planes in turn.  One group spent the
 // whole period of a 16-channel layer on its chain of wait, TMEM load, GELU and
@@ -101,6 +108,7 @@ struct ConvArgs {
 struct WgradArgs {
     int nb, xo, yo, zo;             // extents of the output-gradient region
     int nseg;                       // z segments of kM positions per row
+    int bz;                         // positions that a segment's K steps read: min(kM, zo rounded up to 16)
     int ych, nyc;                   // rows per work unit, units per column: ceil(yo / ych)
     int nunits;                     // work units (n, x, z segment, y chunk): nb * xo * nseg * nyc
     float *part;                    // per block: [COUT][CIN][27] weight partials then [COUT] bias partials
@@ -519,13 +527,22 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     if (warp == 1) tc::tmem_dealloc(tbase, TCOLS);
 }
 
+// Shared memory of the weight-gradient kernel for rows of bz positions: the
+// input rows of CIN / 2 groups (dx, 8 channels; dx = 3 holds ones), each a
+// ring of `rows` rows of bz + 8 positions, and rows - 2 output-gradient
+// segments.  The ring is as deep as fits: with four rows (two tiles ahead)
+// copies and MMAs waited on each other (a training step of 8 crops of 64^3
+// took 3.08 instead of 2.78 ms).
 template <int CIN, int COUT>
 struct WgradSmem {
-    static constexpr int ROWB = kWz * 16;                    // one input row of one group: [kWz][8 ch]
-    static constexpr int GROUP = 4 * ROWB;                   // a ring of 4 rows per group (the SBO of A)
-    static constexpr int XRING = 16 * GROUP;                 // 16 groups (dx, cg); dx = 3 holds ones
-    static constexpr int GSTAGE = (COUT / 8) * kM * 16;      // output gradient [co/8][kM][8]
-    static constexpr int BYTES = XRING + kStages * GSTAGE + 128 + 128;
+    static constexpr int kBars = 256, kGroups = CIN / 2;
+    int rowb, gseg, rows;
+    __host__ __device__ explicit WgradSmem(int bz)
+        : rowb((bz + 8) * 16), gseg((COUT / 8) * bz * 16),
+          rows((kMaxSmem - 128 - kBars + 2 * gseg) / (kGroups * rowb + gseg)) {
+        if (rows > kMaxRows) rows = kMaxRows;
+    }
+    __host__ __device__ int bytes() const { return rows * kGroups * rowb + (rows - 2) * gseg + kBars + 128; }
 };
 
 template <int CIN, int COUT>
@@ -533,36 +550,39 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     conv_wgrad_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap g_map,
                       WgradArgs a) {
     static_assert((CIN == 16 || CIN == 32) && (COUT == 16 || COUT == 32), "unsupported channel counts");
-    using L = WgradSmem<CIN, COUT>;
     constexpr int CG = CIN / 8, GG = COUT / 8;
     constexpr uint32_t NACC = 9 * COUT;
     constexpr uint32_t TCOLS = NACC <= 256 ? 256 : 512;
-    constexpr uint32_t IDESC = tc::idesc_bf16(kM, COUT, 1, 1);
-    constexpr uint32_t ROWTX = 3 * CG * L::ROWB;             // one new input row of every data group
-    constexpr uint32_t GTX = GG * kM * 16;                   // one tile's output-gradient segment
+    constexpr int ROWS = 4 * CIN;                              // rows of D: 64 or 128
+    constexpr uint32_t IDESC = tc::idesc_bf16(ROWS, COUT, 1, 1);
+    // Rows shorter than kM bring only the positions their K steps read, in 16-byte
+    // pieces of 8 channels each, which bound the copies.
+    const WgradSmem<CIN, COUT> L(a.bz);
+    const int rows = L.rows, stages = rows - 2, rowb = L.rowb, group = rows * rowb;
+    const uint32_t rowtx = 3 * CG * rowb;                      // one new input row of every data group
 
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = align128(smem_raw);
-    unsigned char *xr = smem;                                  // input-row rings [16 groups][4 rows]
-    unsigned char *gs = smem + L::XRING;                       // kStages x GSTAGE
-    uint64_t *bars = reinterpret_cast<uint64_t *>(gs + kStages * L::GSTAGE);
-    uint64_t *full = bars, *empty = bars + 2, *done = bars + 4;
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 6);
+    unsigned char *xr = smem;                                  // input-row rings [groups][rows]
+    unsigned char *gs = smem + L.kGroups * group;                     // output-gradient segments [stages]
+    uint64_t *bars = reinterpret_cast<uint64_t *>(gs + stages * L.gseg);
+    uint64_t *full = bars, *empty = bars + kMaxRows, *done = bars + 2 * kMaxRows;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // the dx = 3 groups hold ones in every ring row (bias gradient)
     {
         const uint4 ones = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
-        uint4 *p = reinterpret_cast<uint4 *>(xr + 3 * CG * L::GROUP);
-        for (int i = threadIdx.x; i < CG * L::GROUP / 16; i += blockDim.x) p[i] = ones;
+        uint4 *p = reinterpret_cast<uint4 *>(xr + 3 * CG * group);
+        for (int i = threadIdx.x; i < CG * group / 16; i += blockDim.x) p[i] = ones;
         fence_proxy_async();
     }
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < stages; ++i) {
             mbar_init(full + i, 1);
-            mbar_init(empty + i, 1);
+            mbar_init(empty + i, kWIssuers);
         }
-        mbar_init(done, 1);
+        mbar_init(done, kWIssuers);
         fence_mbar_init();
     }
     if (warp == 1) tc::tmem_alloc(tslot, TCOLS);
@@ -572,9 +592,14 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     const uint32_t tbase = *tslot;
     bool ok = true;
 
+    // Tile `it` reads ring rows it .. it+2 (mod rows), loads row it+2, and has
+    // stage it % stages.  A column is followed by two empty tiles, so that the
+    // next one finds its rows beside those still being read: copies do not
+    // wait for a column's last MMAs.
     if (warp == 0) {
         if (lane == 0) {
-            int it = 0;                                          // tiles of this block so far
+            int it = 0, row = 0, s = 0;
+            uint32_t ph = 0;
             for (int unit = blockIdx.x; ok && unit < a.nunits; unit += gridDim.x) {
                 int r = unit;
                 const int yc = r % a.nyc; r /= a.nyc;
@@ -582,41 +607,47 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 const int x = r % a.xo, b = r / a.xo;
                 const int y0 = yc * a.ych, ylen = min(a.ych, a.yo - y0);
                 const int z0 = seg * kM;
-                for (int j = 0; j < ylen; ++j, ++it) {
-                    const int s = it & 1, u = it >> 1;
-                    // tile it-2 done: its gradient stage and the ring row that
-                    // this tile's new row replaces are free
-                    if (u > 0 && !mbar_wait(empty + s, (u - 1) & 1, kWaitBudget)) {
+                for (int j = 0; j < ylen + 2; ++j, ++it) {
+                    // tile it - stages done: its gradient segment and the ring
+                    // row that this tile's new row replaces are free
+                    if (it >= stages && !mbar_wait(empty + s, ph ^ 1, kWaitBudget)) {
                         ok = false;
                         break;
                     }
-                    // a new column loads rows y0, y0+1 too, over the rows
-                    // that tile it-1 still reads
-                    if (j == 0 && it > 0 && !mbar_wait(empty + ((it - 1) & 1), ((it - 1) >> 1) & 1, kWaitBudget)) {
-                        ok = false;
-                        break;
+                    if (j < ylen) {
+                        const int first = j == 0 ? 0 : 2;            // new rows: j+first .. j+2
+                        mbar_expect_tx(full + s, (3 - first) * rowtx + L.gseg);
+                        for (int dr = first; dr < 3; ++dr) {
+                            const int slot = row + dr < rows ? row + dr : row + dr - rows;
+                            for (int dx = 0; dx < 3; ++dx)
+                                for (int cg = 0; cg < CG; ++cg)
+                                    tma_load_4d(xr + (dx * CG + cg) * group + slot * rowb, &x_map, cg * 8, z0,
+                                                y0 + j + dr, b * (a.xo + 2) + x + dx, full + s);
+                        }
+                        unsigned char *gd = gs + s * L.gseg;
+                        for (int g = 0; g < GG; ++g)
+                            tma_load_4d(gd + g * a.bz * 16, &g_map, g * 8, z0 + 2, y0 + j + 2,
+                                        b * (a.xo + 4) + x + 2, full + s);
+                    } else {
+                        tc::mbar_arrive(full + s);
                     }
-                    const int first = j == 0 ? 0 : 2;            // new rows: j+first .. j+2
-                    mbar_expect_tx(full + s, (3 - first) * ROWTX + GTX);
-                    for (int dr = first; dr < 3; ++dr) {
-                        const int slot = (it + dr) & 3;
-                        for (int dx = 0; dx < 3; ++dx)
-                            for (int cg = 0; cg < CG; ++cg)
-                                tma_load_4d(xr + (dx * CG + cg) * L::GROUP + slot * L::ROWB, &x_map, cg * 8, z0,
-                                            y0 + j + dr, b * (a.xo + 2) + x + dx, full + s);
-                    }
-                    unsigned char *gd = gs + s * L::GSTAGE;
-                    for (int g = 0; g < GG; ++g)
-                        tma_load_4d(gd + g * kM * 16, &g_map, g * 8, z0 + 2, y0 + j + 2, b * (a.xo + 4) + x + 2,
-                                    full + s);
+                    if (++row == rows) row = 0;
+                    if (++s == stages) s = 0, ph ^= 1;
                 }
             }
-            for (int j = it - 2 < 0 ? 0 : it - 2; j < it; ++j) ok &= mbar_wait(full + (j & 1), (j >> 1) & 1, kWaitBudget);
+            // copies still in flight must land before the block exits
+            for (int j = it - stages < 0 ? 0 : it - stages; j < it; ++j)
+                ok &= mbar_wait(full + j % stages, (j / stages) & 1, kWaitBudget);
         }
-    } else if (warp == 1) {
+    } else if (warp <= kWIssuers) {
         // the whole warp runs the issue loop; the elected lane issues each
         // tile's MMAs and its commit (see elect_one)
-        int it = 0;
+        constexpr int NT = 9 / kWIssuers;     // this issuer's (dy, dz) pairs
+        const int t9lo = (warp - 1) * NT;
+        int it = 0, row = 0, s = 0;
+        uint32_t ph = 0;
+        const uint64_t a0 = tc::sdesc(smem_u32(xr), 128, group);
+        const uint64_t b0 = tc::sdesc(smem_u32(gs), 128, a.bz * 16);
         for (int unit = blockIdx.x; ok && unit < a.nunits; unit += gridDim.x) {
             int r = unit;
             const int yc = r % a.nyc; r /= a.nyc;
@@ -624,39 +655,44 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             const int ylen = min(a.ych, a.yo - yc * a.ych);
             const int len = min(kM, a.zo - seg * kM);
             const int nk = (len + 15) >> 4;
-            for (int j = 0; j < ylen; ++j, ++it) {
-                const int s = it & 1, u = it >> 1;
-                if (!warp_wait(full + s, u & 1)) {
+            for (int j = 0; j < ylen + 2; ++j, ++it) {
+                if (!warp_wait(full + s, ph)) {
                     ok = false;
                     break;
                 }
                 tc::fence_after();
-                const uint32_t xa = smem_u32(xr);
-                const uint32_t ga = smem_u32(gs + s * L::GSTAGE);
+                // descriptors advance by (byte offset >> 4) in their address
+                // field; every address stays below 256 KB
+                uint64_t bd = b0 + (uint32_t)(s * L.gseg >> 4), ad[NT];
+#pragma unroll
+                for (int i = 0; i < NT; ++i) {
+                    const int t9 = t9lo + i, dy = t9 / 3, dz = t9 - 3 * dy;
+                    ad[i] = a0 + (uint32_t)(((row + dy < rows ? row + dy : row + dy - rows) * rowb + dz * 16) >> 4);
+                }
                 if (tc::elect_one()) {
 #pragma unroll 1
-                    for (int ks = 0; ks < nk; ++ks) {
-                        const uint64_t bd = tc::sdesc(ga + (uint32_t)(ks * 256), 128, kM * 16);
+                    for (int ks = 0; ks < (j < ylen ? nk : 0); ++ks) {
                         const uint32_t acc = (it | ks) != 0;
 #pragma unroll
-                        for (int t9 = 0; t9 < 9; ++t9) {
-                            const int dy = t9 / 3, dz = t9 % 3;
-                            const uint32_t aa =
-                                xa + (uint32_t)(((it + dy) & 3) * L::ROWB) + (uint32_t)((dz + 16 * ks) * 16);
-                            tc::mma_bf16(tbase + (uint32_t)(t9 * COUT), tc::sdesc(aa, 128, L::GROUP), bd, IDESC,
-                                         acc);
+                        for (int i = 0; i < NT; ++i) {
+                            tc::mma_bf16(tbase + (uint32_t)((t9lo + i) * COUT), ad[i], bd, IDESC, acc);
+                            ad[i] += 256 >> 4;
                         }
+                        bd += 256 >> 4;
                     }
                     tc::commit(empty + s);
                 }
                 __syncwarp();
+                if (++row == rows) row = 0;
+                if (++s == stages) s = 0, ph ^= 1;
             }
         }
         if (tc::elect_one()) tc::commit(done);
         __syncwarp();
     } else {
         const int q = warp & 3;
-        const int m = 32 * q + lane;            // TMEM lane = row of D
+        // row of D: TMEM lane of 128 rows; 64 rows take 16 lanes of each sub-partition
+        const int m = ROWS == 128 ? 32 * q + lane : 16 * q + (lane & 15);
         const int jgrp = m >> 3, ci_lo = m & 7;
         const int dx = jgrp / CG, cg = jgrp % CG;
         const bool have = blockIdx.x < a.nunits;
@@ -673,18 +709,20 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 #pragma unroll
                 for (int c = 0; c < COUT; ++c) v[c] = 0.0f;
             }
-            if (dx < 3) {
+            if (lane >= ROWS / 4) {
+                // no row of D
+            } else if (dx < 3) {
                 const int ci = cg * 8 + ci_lo;
                 const int t = dx * 9 + j;
 #pragma unroll
                 for (int co = 0; co < COUT; ++co) wpart[((size_t)co * CIN + ci) * 27 + t] = v[co];
-            } else if (dx == 3 && cg == 0 && ci_lo == 0 && j == 0) {
+            } else if (cg == 0 && ci_lo == 0 && j == 0) {
 #pragma unroll
                 for (int co = 0; co < COUT; ++co) wpart[COUT * CIN * 27 + co] = v[co];
             }
         }
     }
-    if (warp == 1 && lane == 0) ok &= mbar_wait(done, 0, kWaitBudget);
+    if (warp <= kWIssuers && warp > 0 && lane == 0) ok &= mbar_wait(done, 0, kWaitBudget);
     if (!ok) atomicOr(a.status, kNetTimeout);
     tc::fence_before();
     __syncthreads();

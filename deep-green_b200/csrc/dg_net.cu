@@ -419,17 +419,17 @@ cudaError_t launch_conv(dg_net *net, const void *in, int nb, int xi, int yi, int
 template <int CIN, int COUT>
 cudaError_t launch_wgrad(dg_net *net, const void *x_in, const void *g_pad, int nb, int xo, int yo, int zo, float *gw,
                          float *gb) {
-    using L = WgradSmem<CIN, COUT>;
     auto kern = conv_wgrad_kernel<CIN, COUT>;
     static std::atomic<unsigned long long> attr_set{0};
-    const cudaError_t attr_err = ensure_dynamic_smem(kern, L::BYTES, attr_set);
+    const cudaError_t attr_err = ensure_dynamic_smem(kern, kMaxSmem, attr_set);
     if (attr_err != cudaSuccess) return attr_err;
     WgradArgs a;
     a.nb = nb; a.xo = xo; a.yo = yo; a.zo = zo;
     a.nseg = (zo + kM - 1) / kM;
+    a.bz = std::min(kM, (zo + 15) / 16 * 16);
     CUtensorMap mx, mg;
-    if (!map_wgrad(&mx, x_in, CIN, nb, xo + 2, yo + 2, zo + 2, kWz, 1)) return cudaErrorInvalidValue;
-    if (!map_wgrad(&mg, g_pad, COUT, nb, xo + 4, yo + 4, zo + 4, kM, 1)) return cudaErrorInvalidValue;
+    if (!map_wgrad(&mx, x_in, CIN, nb, xo + 2, yo + 2, zo + 2, a.bz + 8, 1)) return cudaErrorInvalidValue;
+    if (!map_wgrad(&mg, g_pad, COUT, nb, xo + 4, yo + 4, zo + 4, a.bz, 1)) return cudaErrorInvalidValue;
     // columns along y split into chunks so that every block gets ~6 units.  The
     // split decides which rows a block sums on its accumulators before the
     // blocks' partials are added: another one changes the gradients by ~3e-4.
@@ -442,7 +442,7 @@ cudaError_t launch_wgrad(dg_net *net, const void *x_in, const void *g_pad, int n
     a.part = net->wpart;
     a.status = net->status;
     const int grid = std::max(1, std::min(a.nunits, net->nsm));
-    kern<<<grid, kConvThreads, L::BYTES, net->stream>>>(mx, mg, a);
+    kern<<<grid, kConvThreads, WgradSmem<CIN, COUT>(a.bz).bytes(), net->stream>>>(mx, mg, a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     wgrad_reduce_kernel<<<(COUT * CIN * 27 + COUT + 127) / 128, 128, 0, net->stream>>>(net->wpart, grid, CIN, COUT, gw,
