@@ -73,7 +73,7 @@ namespace net {
 constexpr int kM = 128;                    // positions per tile (MMA M)
 constexpr int kWz = 136;                   // window positions per row (>= kM + 2; 128-byte boxes)
 constexpr int kMaxSmem = 227 * 1024;       // shared memory of one block
-constexpr int kMaxRows = 10;               // weight gradient: most input rows in a ring
+constexpr int kMaxStages = 8;              // weight gradient: most stages
 constexpr int kIssuers = 2;                // forward: MMA-issuing warps, each with its own accumulators
 constexpr int kWIssuers = 3;               // weight gradient: MMA-issuing warps, a third of the accumulators each
 constexpr int kConvThreads = 32 * (1 + kWIssuers + 4);  // weight gradient: TMA, issuers, epilogue
@@ -527,22 +527,22 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     if (warp == 1) tc::tmem_dealloc(tbase, TCOLS);
 }
 
-// Shared memory of the weight-gradient kernel for rows of bz positions: the
-// input rows of CIN / 2 groups (dx, 8 channels; dx = 3 holds ones), each a
-// ring of `rows` rows of bz + 8 positions, and rows - 2 output-gradient
-// segments.  The ring is as deep as fits: with four rows (two tiles ahead)
-// copies and MMAs waited on each other (a training step of 8 crops of 64^3
-// took 3.08 instead of 2.78 ms).
+// Shared memory of the weight-gradient kernel for rows of bz positions:
+// `stages` input rows of CIN / 2 groups (dx, 8 channels; dx = 3 holds ones) of
+// bz + 8 positions, and a ring of stages + 2 output-gradient rows with copies
+// of its first two behind the last, so that any three rows in turn lie one
+// after the other.  As deep as fits: with two stages copies and MMAs waited
+// on each other.
 template <int CIN, int COUT>
 struct WgradSmem {
     static constexpr int kBars = 256, kGroups = CIN / 2;
-    int rowb, gseg, rows;
+    int rowb, gseg, stages;
     __host__ __device__ explicit WgradSmem(int bz)
         : rowb((bz + 8) * 16), gseg((COUT / 8) * bz * 16),
-          rows((kMaxSmem - 128 - kBars + 2 * gseg) / (kGroups * rowb + gseg)) {
-        if (rows > kMaxRows) rows = kMaxRows;
+          stages((kMaxSmem - 128 - kBars - 4 * gseg) / (kGroups * rowb + gseg)) {
+        if (stages > kMaxStages) stages = kMaxStages;
     }
-    __host__ __device__ int bytes() const { return rows * kGroups * rowb + (rows - 2) * gseg + kBars + 128; }
+    __host__ __device__ int bytes() const { return stages * kGroups * rowb + (stages + 4) * gseg + kBars + 128; }
 };
 
 template <int CIN, int COUT>
@@ -554,27 +554,30 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     constexpr uint32_t NACC = 9 * COUT;
     constexpr uint32_t TCOLS = NACC <= 256 ? 256 : 512;
     constexpr int ROWS = 4 * CIN;                              // rows of D: 64 or 128
-    constexpr uint32_t IDESC = tc::idesc_bf16(ROWS, COUT, 1, 1);
+    constexpr uint32_t ID1 = tc::idesc_bf16(ROWS, COUT, 1, 1), ID2 = tc::idesc_bf16(ROWS, 2 * COUT, 1, 1),
+                       ID3 = tc::idesc_bf16(ROWS, 3 * COUT, 1, 1);
     // Rows shorter than kM bring only the positions their K steps read, in 16-byte
     // pieces of 8 channels each, which bound the copies.
     const WgradSmem<CIN, COUT> L(a.bz);
-    const int rows = L.rows, stages = rows - 2, rowb = L.rowb, group = rows * rowb;
-    const uint32_t rowtx = 3 * CG * rowb;                      // one new input row of every data group
+    const int stages = L.stages, ring = stages + 2, rowb = L.rowb, xstage = L.kGroups * rowb;
 
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = align128(smem_raw);
-    unsigned char *xr = smem;                                  // input-row rings [groups][rows]
-    unsigned char *gs = smem + L.kGroups * group;                     // output-gradient segments [stages]
-    uint64_t *bars = reinterpret_cast<uint64_t *>(gs + stages * L.gseg);
-    uint64_t *full = bars, *empty = bars + kMaxRows, *done = bars + 2 * kMaxRows;
+    unsigned char *xs = smem;                                  // input rows [stages][groups]
+    unsigned char *gs = smem + stages * xstage;                // output-gradient rows [ring + 2]
+    uint64_t *bars = reinterpret_cast<uint64_t *>(gs + (ring + 2) * L.gseg);
+    uint64_t *full = bars, *empty = bars + kMaxStages, *done = bars + 2 * kMaxStages;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // the dx = 3 groups hold ones in every ring row (bias gradient)
+    const int q = warp & 3;                                    // epilogue: TMEM sub-partition
+    // the dx = 3 groups hold ones in every stage (bias gradient)
     {
         const uint4 ones = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
-        uint4 *p = reinterpret_cast<uint4 *>(xr + 3 * CG * group);
-        for (int i = threadIdx.x; i < CG * group / 16; i += blockDim.x) p[i] = ones;
+        for (int s = 0; s < stages; ++s) {
+            uint4 *p = reinterpret_cast<uint4 *>(xs + s * xstage + 3 * CG * rowb);
+            for (int i = threadIdx.x; i < CG * rowb / 16; i += blockDim.x) p[i] = ones;
+        }
         fence_proxy_async();
     }
     if (threadIdx.x == 0) {
@@ -590,15 +593,26 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     __syncthreads();
     tc::fence_after();
     const uint32_t tbase = *tslot;
+    if (warp > kWIssuers) {
+        // every accumulator starts at zero: all MMAs accumulate
+        float zero[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) zero[c] = 0.0f;
+        for (int c = 0; c < (int)NACC; c += 16) tc::tmem_st16(tbase + ((uint32_t)(32 * q) << 16) + c, zero);
+        tc::tmem_wait_st();
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
     bool ok = true;
 
-    // Tile `it` reads ring rows it .. it+2 (mod rows), loads row it+2, and has
-    // stage it % stages.  A column is followed by two empty tiles, so that the
-    // next one finds its rows beside those still being read: copies do not
-    // wait for a column's last MMAs.
+    // Step i of a column of ylen output rows takes input row y0 + i and the
+    // output-gradient rows i-2, i-1 and i that exist (dy = 2, 1, 0).  Gradient
+    // row i arrives with input row i, in ring slot `it mod ring` of the running
+    // step `it`; the column's last two steps bring none.
     if (warp == 0) {
         if (lane == 0) {
-            int it = 0, row = 0, s = 0;
+            int it = 0, slot = 0, s = 0;
             uint32_t ph = 0;
             for (int unit = blockIdx.x; ok && unit < a.nunits; unit += gridDim.x) {
                 int r = unit;
@@ -607,31 +621,24 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 const int x = r % a.xo, b = r / a.xo;
                 const int y0 = yc * a.ych, ylen = min(a.ych, a.yo - y0);
                 const int z0 = seg * kM;
-                for (int j = 0; j < ylen + 2; ++j, ++it) {
-                    // tile it - stages done: its gradient segment and the ring
-                    // row that this tile's new row replaces are free
+                for (int i = 0; i < ylen + 2; ++i, ++it) {
+                    // step it - stages done: its input row is free, and so is
+                    // the gradient row of step it - ring, which it read last
                     if (it >= stages && !mbar_wait(empty + s, ph ^ 1, kWaitBudget)) {
                         ok = false;
                         break;
                     }
-                    if (j < ylen) {
-                        const int first = j == 0 ? 0 : 2;            // new rows: j+first .. j+2
-                        mbar_expect_tx(full + s, (3 - first) * rowtx + L.gseg);
-                        for (int dr = first; dr < 3; ++dr) {
-                            const int slot = row + dr < rows ? row + dr : row + dr - rows;
-                            for (int dx = 0; dx < 3; ++dx)
-                                for (int cg = 0; cg < CG; ++cg)
-                                    tma_load_4d(xr + (dx * CG + cg) * group + slot * rowb, &x_map, cg * 8, z0,
-                                                y0 + j + dr, b * (a.xo + 2) + x + dx, full + s);
-                        }
-                        unsigned char *gd = gs + s * L.gseg;
+                    const int copies = i >= ylen ? 0 : slot < 2 ? 2 : 1;
+                    mbar_expect_tx(full + s, 3 * CG * rowb + copies * L.gseg);
+                    for (int dx = 0; dx < 3; ++dx)
+                        for (int cg = 0; cg < CG; ++cg)
+                            tma_load_4d(xs + s * xstage + (dx * CG + cg) * rowb, &x_map, cg * 8, z0, y0 + i,
+                                        b * (a.xo + 2) + x + dx, full + s);
+                    for (int c = 0; c < copies; ++c)
                         for (int g = 0; g < GG; ++g)
-                            tma_load_4d(gd + g * a.bz * 16, &g_map, g * 8, z0 + 2, y0 + j + 2,
-                                        b * (a.xo + 4) + x + 2, full + s);
-                    } else {
-                        tc::mbar_arrive(full + s);
-                    }
-                    if (++row == rows) row = 0;
+                            tma_load_4d(gs + (slot + c * ring) * L.gseg + g * a.bz * 16, &g_map, g * 8, z0 + 2,
+                                        y0 + i + 2, b * (a.xo + 4) + x + 2, full + s);
+                    if (++slot == ring) slot = 0;
                     if (++s == stages) s = 0, ph ^= 1;
                 }
             }
@@ -641,13 +648,13 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         }
     } else if (warp <= kWIssuers) {
         // the whole warp runs the issue loop; the elected lane issues each
-        // tile's MMAs and its commit (see elect_one)
-        constexpr int NT = 9 / kWIssuers;     // this issuer's (dy, dz) pairs
-        const int t9lo = (warp - 1) * NT;
-        int it = 0, row = 0, s = 0;
+        // step's MMAs and its commit (see elect_one).  Each warp takes one dz.
+        const int dz = warp - 1;
+        int it = 0, slot = 0, s = 0;
         uint32_t ph = 0;
-        const uint64_t a0 = tc::sdesc(smem_u32(xr), 128, group);
+        const uint64_t a0 = tc::sdesc(smem_u32(xs) + dz * 16, 128, rowb);
         const uint64_t b0 = tc::sdesc(smem_u32(gs), 128, a.bz * 16);
+        const uint32_t d0 = tbase + (uint32_t)(dz * 3 * COUT);
         for (int unit = blockIdx.x; ok && unit < a.nunits; unit += gridDim.x) {
             int r = unit;
             const int yc = r % a.nyc; r /= a.nyc;
@@ -655,42 +662,37 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             const int ylen = min(a.ych, a.yo - yc * a.ych);
             const int len = min(kM, a.zo - seg * kM);
             const int nk = (len + 15) >> 4;
-            for (int j = 0; j < ylen + 2; ++j, ++it) {
+            for (int i = 0; i < ylen + 2; ++i, ++it) {
                 if (!warp_wait(full + s, ph)) {
                     ok = false;
                     break;
                 }
                 tc::fence_after();
+                const int lo = max(0, i - 2), n = min(i, ylen - 1) - lo + 1;   // gradient rows lo .. lo+n-1
+                int first = slot - (i - lo);                                   // ring slot of row lo
+                if (first < 0) first += ring;
                 // descriptors advance by (byte offset >> 4) in their address
                 // field; every address stays below 256 KB
-                uint64_t bd = b0 + (uint32_t)(s * L.gseg >> 4), ad[NT];
-#pragma unroll
-                for (int i = 0; i < NT; ++i) {
-                    const int t9 = t9lo + i, dy = t9 / 3, dz = t9 - 3 * dy;
-                    ad[i] = a0 + (uint32_t)(((row + dy < rows ? row + dy : row + dy - rows) * rowb + dz * 16) >> 4);
-                }
+                uint64_t ad = a0 + (uint32_t)((s * xstage) >> 4), bd = b0 + (uint32_t)((first * L.gseg) >> 4);
+                const uint32_t d = d0 + (uint32_t)((2 - (i - lo)) * COUT);
+                const uint32_t id = n == 3 ? ID3 : n == 2 ? ID2 : ID1;
                 if (tc::elect_one()) {
 #pragma unroll 1
-                    for (int ks = 0; ks < (j < ylen ? nk : 0); ++ks) {
-                        const uint32_t acc = (it | ks) != 0;
-#pragma unroll
-                        for (int i = 0; i < NT; ++i) {
-                            tc::mma_bf16(tbase + (uint32_t)((t9lo + i) * COUT), ad[i], bd, IDESC, acc);
-                            ad[i] += 256 >> 4;
-                        }
+                    for (int ks = 0; ks < nk; ++ks) {
+                        tc::mma_bf16(d, ad, bd, id, 1u);
+                        ad += 256 >> 4;
                         bd += 256 >> 4;
                     }
                     tc::commit(empty + s);
                 }
                 __syncwarp();
-                if (++row == rows) row = 0;
+                if (++slot == ring) slot = 0;
                 if (++s == stages) s = 0, ph ^= 1;
             }
         }
         if (tc::elect_one()) tc::commit(done);
         __syncwarp();
     } else {
-        const int q = warp & 3;
         // row of D: TMEM lane of 128 rows; 64 rows take 16 lanes of each sub-partition
         const int m = ROWS == 128 ? 32 * q + lane : 16 * q + (lane & 15);
         const int jgrp = m >> 3, ci_lo = m & 7;
@@ -702,8 +704,9 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 #pragma unroll 1
         for (int j = 0; j < 9; ++j) {
             float v[COUT];
+            const uint32_t col = (uint32_t)(((j % 3) * 3 + 2 - j / 3) * COUT);   // tap (dy, dz) = (j / 3, j % 3)
 #pragma unroll
-            for (int c = 0; c < COUT; c += 16) tc::tmem_ld16(tbase + ((uint32_t)(32 * q) << 16) + j * COUT + c, v + c);
+            for (int c = 0; c < COUT; c += 16) tc::tmem_ld16(tbase + ((uint32_t)(32 * q) << 16) + col + c, v + c);
             tc::tmem_wait_ld();
             if (!have || !ok) {
 #pragma unroll
