@@ -44,19 +44,23 @@
 //   gradient zero-padded by 2 with the taps flipped and W transposed.
 //
 // Weight-gradient kernel: dW_t[co][ci] = sum_v dZ[v][co] X[v+t][ci] over
-// all output positions v.  D[M=128, N=COUT] per (dy, dz) pair, 9 TMEM
-// accumulators; the M rows are (dx in 0..3, ci) -- dx = 3 is a block of
-// ones, which turns its rows into the bias gradient sum_v dZ[v][co].  Both
-// operands are MN-major: K is the position along z, 16 bytes apart.  A block
-// walks a column of output rows along y (one tile = one row segment of at
-// most kM positions): the input rows y, y+1, y+2 that tile y reads sit in a
-// ring per (dx, channel group), so each tile brings one new input row.  With
-// 16 input channels M is 64.  Three warps issue the MMAs, each those of one
-// dy, into accumulators of their own: one warp's issue loop, not the operand
-// reads, had set the pace.  Layers of 8 crops of 64^3, per launch (32 -> 32,
-// 32 -> 16, 16 -> 32): 450, 396, 396 us with one issuer, 136-position copies
-// and four ring rows; 321, 282, 204 us so.  (The operand reads of the 32 -> 32
-// layer take ~245 us: 5 KB of shared memory per MMA.)
+// all output positions v.  K is the position along z, both operands are
+// MN-major: one row along z each, as it lies in memory (64 or 32 bytes per
+// position, the swizzled MN-major layout), and a shift by dz is a start dz
+// positions further.  M is (dx in 0..3, ci) -- dx = 3 is a row of ones, which
+// turns its rows of D into the bias gradient sum_v dZ[v][co].  N is (dy, co): a
+// block walks along y, and input row Y meets the gradient rows Y-2, Y-1, Y (dy
+// = 2, 1, 0), which lie one after the other in a ring.  Accumulators: 9 x COUT
+// columns.  Three warps issue the MMAs of one dz each.  Per launch on layers of
+// 8 crops of 64^3 (32 -> 32, 32 -> 16, 16 -> 32):
+//   450, 396, 396 us  one MMA per tap, one issuer, two stages, boxes of 8
+//                     channels x 136 positions (M = 128 for 16 channels too)
+//   321, 282, 204 us  three issuers (one warp's issue loop had set the pace),
+//                     more stages, boxes as long as the row, M = 64
+//   ~270 (32 -> 32)   dy in N: 7 KB of operands read per 96 columns, not 15 KB;
+//                     bound by the copies' 16-byte pieces (same time with a
+//                     fifth of the MMAs)
+//   176, 124, 145 us  whole rows of 64 or 32 bytes
 //
 // Every wait is bounded (~2 s); a timeout sets a status bit and the block
 // drains its copies and MMAs and frees its TMEM before returning.
@@ -156,11 +160,6 @@ struct Share {
         return true;
     }
 };
-
-__device__ __forceinline__ unsigned char *align128(unsigned char *p) {
-    const uint32_t s = smem_u32(p);
-    return p + ((128u - (s & 127u)) & 127u);
-}
 
 __device__ __forceinline__ unsigned char *align1024(unsigned char *p) {
     const uint32_t s = smem_u32(p);
@@ -528,21 +527,21 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
 }
 
 // Shared memory of the weight-gradient kernel for rows of bz positions:
-// `stages` input rows of CIN / 2 groups (dx, 8 channels; dx = 3 holds ones) of
-// bz + 8 positions, and a ring of stages + 2 output-gradient rows with copies
-// of its first two behind the last, so that any three rows in turn lie one
-// after the other.  As deep as fits: with two stages copies and MMAs waited
-// on each other.
+// `stages` times the input rows of the three dx (and a row of ones), of bz + 8
+// positions, and a ring of stages + 2 output-gradient rows with copies of its
+// first two behind the last, so that any three rows in turn lie one after the
+// other.  As deep as fits: with two stages copies and MMAs waited on each
+// other.
 template <int CIN, int COUT>
 struct WgradSmem {
-    static constexpr int kBars = 256, kGroups = CIN / 2;
-    int rowb, gseg, stages;
+    static constexpr int kBars = 256;
+    int xrow, grow, stages;                                  // bytes of a row, both multiples of the swizzle pattern
     __host__ __device__ explicit WgradSmem(int bz)
-        : rowb((bz + 8) * 16), gseg((COUT / 8) * bz * 16),
-          stages((kMaxSmem - 128 - kBars - 4 * gseg) / (kGroups * rowb + gseg)) {
+        : xrow((bz + 8) * CIN * 2), grow(bz * COUT * 2),
+          stages((kMaxSmem - 1024 - kBars - 4 * grow) / (4 * xrow + grow)) {
         if (stages > kMaxStages) stages = kMaxStages;
     }
-    __host__ __device__ int bytes() const { return stages * kGroups * rowb + (stages + 4) * gseg + kBars + 128; }
+    __host__ __device__ int bytes() const { return stages * 4 * xrow + (stages + 4) * grow + kBars + 1024; }
 };
 
 template <int CIN, int COUT>
@@ -550,33 +549,31 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     conv_wgrad_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap g_map,
                       WgradArgs a) {
     static_assert((CIN == 16 || CIN == 32) && (COUT == 16 || COUT == 32), "unsupported channel counts");
-    constexpr int CG = CIN / 8, GG = COUT / 8;
     constexpr uint32_t NACC = 9 * COUT;
     constexpr uint32_t TCOLS = NACC <= 256 ? 256 : 512;
     constexpr int ROWS = 4 * CIN;                              // rows of D: 64 or 128
     constexpr uint32_t ID1 = tc::idesc_bf16(ROWS, COUT, 1, 1), ID2 = tc::idesc_bf16(ROWS, 2 * COUT, 1, 1),
                        ID3 = tc::idesc_bf16(ROWS, 3 * COUT, 1, 1);
-    // Rows shorter than kM bring only the positions their K steps read, in 16-byte
-    // pieces of 8 channels each, which bound the copies.
+    // Rows shorter than kM bring only the positions their K steps read.
     const WgradSmem<CIN, COUT> L(a.bz);
-    const int stages = L.stages, ring = stages + 2, rowb = L.rowb, xstage = L.kGroups * rowb;
+    const int stages = L.stages, ring = stages + 2, xrow = L.xrow, xstage = 4 * xrow;
 
     extern __shared__ unsigned char smem_raw[];
-    unsigned char *smem = align128(smem_raw);
-    unsigned char *xs = smem;                                  // input rows [stages][groups]
+    unsigned char *smem = align1024(smem_raw);                 // swizzle patterns follow address bits
+    unsigned char *xs = smem;                                  // input rows [stages][dx]
     unsigned char *gs = smem + stages * xstage;                // output-gradient rows [ring + 2]
-    uint64_t *bars = reinterpret_cast<uint64_t *>(gs + (ring + 2) * L.gseg);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(gs + (ring + 2) * L.grow);
     uint64_t *full = bars, *empty = bars + kMaxStages, *done = bars + 2 * kMaxStages;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = warp & 3;                                    // epilogue: TMEM sub-partition
-    // the dx = 3 groups hold ones in every stage (bias gradient)
+    // the row of dx = 3 holds ones in every stage (bias gradient)
     {
         const uint4 ones = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
         for (int s = 0; s < stages; ++s) {
-            uint4 *p = reinterpret_cast<uint4 *>(xs + s * xstage + 3 * CG * rowb);
-            for (int i = threadIdx.x; i < CG * rowb / 16; i += blockDim.x) p[i] = ones;
+            uint4 *p = reinterpret_cast<uint4 *>(xs + s * xstage + 3 * xrow);
+            for (int i = threadIdx.x; i < xrow / 16; i += blockDim.x) p[i] = ones;
         }
         fence_proxy_async();
     }
@@ -629,15 +626,13 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                         break;
                     }
                     const int copies = i >= ylen ? 0 : slot < 2 ? 2 : 1;
-                    mbar_expect_tx(full + s, 3 * CG * rowb + copies * L.gseg);
+                    mbar_expect_tx(full + s, 3 * xrow + copies * L.grow);
                     for (int dx = 0; dx < 3; ++dx)
-                        for (int cg = 0; cg < CG; ++cg)
-                            tma_load_4d(xs + s * xstage + (dx * CG + cg) * rowb, &x_map, cg * 8, z0, y0 + i,
-                                        b * (a.xo + 2) + x + dx, full + s);
+                        tma_load_4d(xs + s * xstage + dx * xrow, &x_map, 0, z0, y0 + i, b * (a.xo + 2) + x + dx,
+                                    full + s);
                     for (int c = 0; c < copies; ++c)
-                        for (int g = 0; g < GG; ++g)
-                            tma_load_4d(gs + (slot + c * ring) * L.gseg + g * a.bz * 16, &g_map, g * 8, z0 + 2,
-                                        y0 + i + 2, b * (a.xo + 4) + x + 2, full + s);
+                        tma_load_4d(gs + (slot + c * ring) * L.grow, &g_map, 0, z0 + 2, y0 + i + 2,
+                                    b * (a.xo + 4) + x + 2, full + s);
                     if (++slot == ring) slot = 0;
                     if (++s == stages) s = 0, ph ^= 1;
                 }
@@ -652,8 +647,8 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         const int dz = warp - 1;
         int it = 0, slot = 0, s = 0;
         uint32_t ph = 0;
-        const uint64_t a0 = tc::sdesc(smem_u32(xs) + dz * 16, 128, rowb);
-        const uint64_t b0 = tc::sdesc(smem_u32(gs), 128, a.bz * 16);
+        const uint64_t a0 = tc::sdesc_sw_mn(smem_u32(xs) + dz * CIN * 2, CIN * 2, xrow);
+        const uint64_t b0 = tc::sdesc_sw_mn(smem_u32(gs), COUT * 2, L.grow);
         const uint32_t d0 = tbase + (uint32_t)(dz * 3 * COUT);
         for (int unit = blockIdx.x; ok && unit < a.nunits; unit += gridDim.x) {
             int r = unit;
@@ -673,15 +668,15 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                 if (first < 0) first += ring;
                 // descriptors advance by (byte offset >> 4) in their address
                 // field; every address stays below 256 KB
-                uint64_t ad = a0 + (uint32_t)((s * xstage) >> 4), bd = b0 + (uint32_t)((first * L.gseg) >> 4);
+                uint64_t ad = a0 + (uint32_t)((s * xstage) >> 4), bd = b0 + (uint32_t)((first * L.grow) >> 4);
                 const uint32_t d = d0 + (uint32_t)((2 - (i - lo)) * COUT);
                 const uint32_t id = n == 3 ? ID3 : n == 2 ? ID2 : ID1;
                 if (tc::elect_one()) {
 #pragma unroll 1
                     for (int ks = 0; ks < nk; ++ks) {
                         tc::mma_bf16(d, ad, bd, id, 1u);
-                        ad += 256 >> 4;
-                        bd += 256 >> 4;
+                        ad += (16 * CIN * 2) >> 4;
+                        bd += (16 * COUT * 2) >> 4;
                     }
                     tc::commit(empty + s);
                 }
@@ -695,8 +690,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     } else {
         // row of D: TMEM lane of 128 rows; 64 rows take 16 lanes of each sub-partition
         const int m = ROWS == 128 ? 32 * q + lane : 16 * q + (lane & 15);
-        const int jgrp = m >> 3, ci_lo = m & 7;
-        const int dx = jgrp / CG, cg = jgrp % CG;
+        const int dx = m / CIN, ci = m % CIN;
         const bool have = blockIdx.x < a.nunits;
         if (have && !warp_wait(done, 0)) ok = false;
         tc::fence_after();
@@ -715,11 +709,10 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             if (lane >= ROWS / 4) {
                 // no row of D
             } else if (dx < 3) {
-                const int ci = cg * 8 + ci_lo;
                 const int t = dx * 9 + j;
 #pragma unroll
                 for (int co = 0; co < COUT; ++co) wpart[((size_t)co * CIN + ci) * 27 + t] = v[co];
-            } else if (cg == 0 && ci_lo == 0 && j == 0) {
+            } else if (ci == 0 && j == 0) {
 #pragma unroll
                 for (int co = 0; co < COUT; ++co) wpart[COUT * CIN * 27 + co] = v[co];
             }

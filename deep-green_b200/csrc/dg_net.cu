@@ -106,19 +106,19 @@ bool map_conv_input(CUtensorMap *m, const void *base, int c, int n, int x, int y
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Weight-gradient operands: 4-D view (c, z, y, x + n * x_extent), box (8,
-// bz, by, 1): 8 channels of each position, no swizzle.
-bool map_wgrad(CUtensorMap *m, const void *base, int c, int n, int x, int y, int z, int bz, int by) {
+// Weight-gradient operands: 4-D view (c, z, y, x + n * x_extent), box (c, bz,
+// 1, 1) -- one row -- with the same swizzles.
+bool map_wgrad(CUtensorMap *m, const void *base, int c, int n, int x, int y, int z, int bz) {
     auto fn = encode_fn();
     if (!fn) return false;
     const cuuint64_t e = 2;
     cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)z, (cuuint64_t)y, (cuuint64_t)x * n};
     cuuint64_t strides[3] = {c * e, (cuuint64_t)z * c * e, (cuuint64_t)y * z * c * e};
-    cuuint32_t box[4] = {8, (cuuint32_t)bz, (cuuint32_t)by, 1};
+    cuuint32_t box[4] = {(cuuint32_t)c, (cuuint32_t)bz, 1, 1};
     cuuint32_t estr[4] = {1, 1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(base), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+              CU_TENSOR_MAP_INTERLEAVE_NONE, c == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // ---------------------------------------------------------------------------
@@ -428,8 +428,8 @@ cudaError_t launch_wgrad(dg_net *net, const void *x_in, const void *g_pad, int n
     a.nseg = (zo + kM - 1) / kM;
     a.bz = std::min(kM, (zo + 15) / 16 * 16);
     CUtensorMap mx, mg;
-    if (!map_wgrad(&mx, x_in, CIN, nb, xo + 2, yo + 2, zo + 2, a.bz + 8, 1)) return cudaErrorInvalidValue;
-    if (!map_wgrad(&mg, g_pad, COUT, nb, xo + 4, yo + 4, zo + 4, a.bz, 1)) return cudaErrorInvalidValue;
+    if (!map_wgrad(&mx, x_in, CIN, nb, xo + 2, yo + 2, zo + 2, a.bz + 8)) return cudaErrorInvalidValue;
+    if (!map_wgrad(&mg, g_pad, COUT, nb, xo + 4, yo + 4, zo + 4, a.bz)) return cudaErrorInvalidValue;
     // columns along y split into chunks so that every block gets ~6 units.  The
     // split decides which rows a block sums on its accumulators before the
     // blocks' partials are added: another one changes the gradients by ~3e-4.

@@ -1,16 +1,10 @@
 // dg_tc.cuh -- Blackwell tensor-core (tcgen05) and TMA wrappers for the
 // correction network's convolution kernels.
 //
-// Shared-memory matrix descriptors use the no-swizzle ("interleave")
-// canonical layouts of the 5th-generation tensor cores, in units of 16-byte
-// rows ("core matrix" = 8 such rows, 128 contiguous bytes):
-//   K-major : element (mn, k) of a core matrix at row mn, bytes 2*k;
-//             SBO = byte stride between 8-row groups along M/N,
-//             LBO = byte stride between 8-element groups along K.
-//   MN-major: element (mn, k) of a core matrix at row k, bytes 2*mn;
-//             SBO = byte stride between 8-element groups along M/N,
-//             LBO = byte stride between 8-row groups along K.
-// Accumulators live in tensor memory (TMEM): lane = row of D (M = 128),
+// Shared-memory matrix descriptors use the canonical swizzled layouts of the
+// 5th-generation tensor cores, with rows of 32 or 64 bytes.
+// Accumulators live in tensor memory (TMEM): lane = row of D (M = 128;
+// of M = 64, 16 rows in the first lanes of each 32),
 // column = column of D, 32-bit FP32 values.
 #pragma once
 #include <cuda.h>
@@ -22,13 +16,8 @@
 namespace dg {
 namespace tc {
 
-// 64-bit shared-memory matrix descriptor, no swizzle, version 1 (sm_100).
-__device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
-}
-
-// Descriptor of a K-major operand in one of the swizzled layouts: rows of
+// 64-bit shared-memory matrix descriptor (version 1, sm_100) of a K-major
+// operand in one of the swizzled layouts: rows of
 // `row` bytes (32 or 64), 8-row atoms of 8*row bytes whose 16-byte chunks are
 // permuted by address bits (chunk ^= (address >> 7) & (row/16 - 1)); SBO =
 // stride between atoms.  Layout codes: 6 = 32-byte swizzle, 4 = 64-byte.
@@ -39,6 +28,16 @@ __device__ __forceinline__ uint64_t sdesc_sw(uint32_t saddr, uint32_t row) {
     const uint64_t layout = row == 64 ? 4ull : 6ull;
     return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(((8 * row) >> 4) & 0x3FFFu) << 32) |
            (1ull << 46) | (layout << 61);
+}
+
+// Descriptor of an MN-major operand in a swizzled layout: atoms of `row` bytes
+// (16 or 32 elements along M/N) by 8 rows along K, permuted as above; atoms
+// follow one another along K, and LBO = stride between atoms along M/N.  A K
+// step of 16 rows, or a shift by any number of rows, advances the start.
+__device__ __forceinline__ uint64_t sdesc_sw_mn(uint32_t saddr, uint32_t row, uint32_t lbo) {
+    const uint64_t layout = row == 64 ? 4ull : 6ull;
+    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
+           ((uint64_t)(((8 * row) >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (layout << 61);
 }
 
 // 32-bit instruction descriptor of kind::f16: BF16 x BF16 -> FP32.
