@@ -189,9 +189,17 @@ __device__ __forceinline__ float2 gelu2(float2 x) {
     return __fmul2_rn(__fmul2_rn(splat(0.5f), x), __fadd2_rn(splat(1.0f), t));
 }
 
-__device__ __forceinline__ float gelu_grad(float x) {
-    const float t = tanh_approx(kGeluC0 * (x + kGeluC1 * x * x * x));
-    return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * kGeluC0 * (1.0f + 3.0f * kGeluC1 * x * x);
+// GELU' = (1 + t)/2 + x/2 (1 - t^2) sqrt(2/pi) (1 + 3 * 0.044715 x^2), likewise
+// (a training step on 8 crops of 64^3: 2.13 instead of 2.18 ms).
+__device__ __forceinline__ float2 gelu_grad2(float2 x) {
+    auto splat = [](float v) { return make_float2(v, v); };
+    const float2 c = __fmul2_rn(__fmul2_rn(splat(kGeluC1), x), x);
+    const float2 a = __fmul2_rn(splat(kGeluC0), __ffma2_rn(c, x, x));
+    const float2 t = make_float2(tanh_approx(a.x), tanh_approx(a.y));
+    const float2 s = __ffma2_rn(make_float2(-t.x, -t.y), t, splat(1.0f));
+    const float2 p = __fmul2_rn(__fmul2_rn(__fmul2_rn(splat(0.5f), x), s), splat(kGeluC0));
+    const float2 d = __ffma2_rn(__fmul2_rn(splat(3.0f * kGeluC1), x), x, splat(1.0f));
+    return __ffma2_rn(splat(0.5f), __fadd2_rn(splat(1.0f), t), __fmul2_rn(p, d));
 }
 
 // All lanes of the warp agree on a wait's outcome.
@@ -512,7 +520,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                     float zv[NC];
                     load_bf16(a.zsrc + dn, zv, NC);
 #pragma unroll
-                    for (int c = 0; c < NC; ++c) v[c] *= gelu_grad(zv[c]);
+                    for (int c = 0; c < NC; c += 2) {
+                        const float2 r =
+                            __fmul2_rn(make_float2(v[c], v[c + 1]), gelu_grad2(make_float2(zv[c], zv[c + 1])));
+                        v[c] = r.x;
+                        v[c + 1] = r.y;
+                    }
                     if constexpr (NC == 16) store16_bf16(a.out_a + o, v);
                     else store_bf16(a.out_a + o, v, NC);
                 }
