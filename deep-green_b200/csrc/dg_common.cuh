@@ -80,6 +80,13 @@ template <class A> __device__ __forceinline__ long long wait_budget_of(const A &
     return a.wait_budget != 0 ? a.wait_budget : kWaitBudget;
 }
 
+// 8 floats of read-only memory with one 32-byte load (p 32-byte aligned).
+__device__ __forceinline__ void load8_f32(const float *p, float *v) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+        : "l"(p));
+}
+
 // ---------------------------------------------------------------------------
 // Ghost images along one axis of extent n: bit g (0-3) is set when ghost index
 // 0, 1, n-2, n-1 holds an image of interior coordinate c (boundaries.rs /

@@ -251,24 +251,21 @@ __global__ void __launch_bounds__(kLearnThreads) correct_kernel(View u1, const f
         const int z = (int)(v - row * (unsigned)n), y = (int)(row % (unsigned)n), x = (int)(row / (unsigned)n);
         const long long i = vidx(u1, x, y, z);
         // divergence of the face fluxes (channel 5 d + c), periodic; rows of
-        // 16 floats read as float4 / float2 pieces
+        // 16 floats read in pieces of 32 bytes (of 16 bytes: 391 us at 256^3,
+        // so 330)
         const unsigned nn = (unsigned)n * n;
         const unsigned lx = (unsigned)(x == 0 ? n - 1 : x - 1) * nn + (unsigned)y * n + z;
         const unsigned ly = (unsigned)x * nn + (unsigned)(y == 0 ? n - 1 : y - 1) * n + z;
         const unsigned lz = (unsigned)x * nn + (unsigned)y * n + (z == 0 ? n - 1 : z - 1);
-        const float4 *own = reinterpret_cast<const float4 *>(out) + (size_t)v * 4;
-        const float4 f0 = own[0], f1 = own[1], f2 = own[2], f3 = own[3];
-        const float hi[15] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w,
-                              f2.x, f2.y, f2.z, f2.w, f3.x, f3.y, f3.z};
-        const float4 ax = reinterpret_cast<const float4 *>(out)[(size_t)lx * 4];
-        const float ax4 = out[(size_t)lx * 16 + 4];
+        float hi[16], lo_x[8], az[8];
+        load8_f32(out + (size_t)v * 16, hi);
+        load8_f32(out + (size_t)v * 16 + 8, hi + 8);
+        load8_f32(out + (size_t)lx * 16, lo_x);
+        load8_f32(out + (size_t)lz * 16 + 8, az);
         const float4 ay = reinterpret_cast<const float4 *>(out)[(size_t)ly * 4 + 1];
         const float2 ay8 = reinterpret_cast<const float2 *>(out)[(size_t)ly * 8 + 4];
-        const float2 az10 = reinterpret_cast<const float2 *>(out)[(size_t)lz * 8 + 5];
-        const float4 az12 = reinterpret_cast<const float4 *>(out)[(size_t)lz * 4 + 3];
-        const float lo_x[5] = {ax.x, ax.y, ax.z, ax.w, ax4};
         const float lo_y[5] = {ay.y, ay.z, ay.w, ay8.x, ay8.y};
-        const float lo_z[5] = {az10.x, az10.y, az12.x, az12.y, az12.z};
+        const float *lo_z = az + 2;
         float o[5];
 #pragma unroll
         for (int c = 0; c < 5; ++c)
@@ -385,8 +382,11 @@ __device__ __forceinline__ void store_quad(float *dst, const View &v, int x, int
 // pass 2: the corrected state into dst (interior and periodic ghosts),
 // conservation and positivity check, and the corrected state's dt (the
 // fast policy's CFL * ds / max(c_s + |v|), as the plain step's own
-// reduction computes it).  One thread per z-quad; n % 4 == 0.
-__global__ void __launch_bounds__(kLearnThreads) apply_kernel(View u1, float *__restrict__ dst,
+// reduction computes it).  One thread per z-quad; n % 4 == 0.  Bound by its
+// FP64 and 64-bit integer instructions at a few warps per SM: two blocks per
+// SM (128 registers; unbounded it took 130 and ran alone) are 283 us at 256^3
+// instead of 455, three (80 registers, spills) 458.
+__global__ void __launch_bounds__(kLearnThreads, 2) apply_kernel(View u1, float *__restrict__ dst,
                                                               const float *__restrict__ delta,
                                                               const uint8_t *__restrict__ mask, GridArgs<float> g,
                                                               double tol, double *part, CorrCtl *ctl) {

@@ -288,20 +288,20 @@ __global__ void flux_residual_kernel(const float *__restrict__ out, const float 
         const int ix = r % s;
         const int b = (int)(r / s);
         const long long c0 = ((((long long)b * o + ix + 1) * o + iy + 1) * o + iz + 1) * kIO;
-        // rows of 16 floats read in float4 / float2 pieces (both arrays start on
-        // 16 bytes: the workspace, and the entry point's check of the target);
-        // as scalars 8 crops of 64^3 took 140 us, so 61
-        const float4 *own = reinterpret_cast<const float4 *>(out + c0);
-        const float4 *px = reinterpret_cast<const float4 *>(out + c0 - (long long)o * o * kIO);
-        const float4 *py = reinterpret_cast<const float4 *>(out + c0 - (long long)o * kIO);
-        const float4 *pz = reinterpret_cast<const float4 *>(out + c0 - kIO);
-        const float4 *pt = reinterpret_cast<const float4 *>(tgt + (size_t)v * kIO);
-        const float4 f0 = own[0], f1 = own[1], f2 = own[2], f3 = own[3], x0 = px[0], y1 = py[1], z3 = pz[3], t0 = pt[0];
-        const float x4 = reinterpret_cast<const float *>(px)[4], t4 = reinterpret_cast<const float *>(pt)[4];
-        const float2 y8 = reinterpret_cast<const float2 *>(py)[4], z10 = reinterpret_cast<const float2 *>(pz)[5];
-        const float hi[15] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w, f2.x, f2.y, f2.z, f2.w, f3.x, f3.y, f3.z};
-        const float lo[15] = {x0.x, x0.y, x0.z, x0.w, x4, y1.y, y1.z, y1.w, y8.x, y8.y, z10.x, z10.y, z3.x, z3.y, z3.z};
-        const float tg[5] = {t0.x, t0.y, t0.z, t0.w, t4};
+        // rows of 16 floats read in pieces of 32 bytes, the target's of 16 (the
+        // entry point checks its alignment); as scalars 8 crops of 64^3 took 140
+        // us, in pieces of 16 bytes 61, so 54
+        float hi[16], x[8], z[8];
+        const float *py = out + c0 - (long long)o * kIO;
+        load8_f32(out + c0, hi);
+        load8_f32(out + c0 + 8, hi + 8);
+        load8_f32(out + c0 - (long long)o * o * kIO, x);
+        load8_f32(out + c0 - kIO + 8, z);
+        const float4 y = reinterpret_cast<const float4 *>(py)[1];
+        const float2 y8 = reinterpret_cast<const float2 *>(py)[4];
+        const float lo[15] = {x[0], x[1], x[2], x[3], x[4], y.y, y.z, y.w, y8.x, y8.y, z[2], z[3], z[4], z[5], z[6]};
+        const float4 t0 = *reinterpret_cast<const float4 *>(tgt + (size_t)v * kIO);
+        const float tg[5] = {t0.x, t0.y, t0.z, t0.w, tgt[(size_t)v * kIO + 4]};
         const float wb = wsample[b];
 #pragma unroll
         for (int c = 0; c < 5; ++c) {
