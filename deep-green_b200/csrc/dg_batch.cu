@@ -14,6 +14,7 @@
 #include <cstring>
 #include <mutex>
 #include <numeric>
+#include <queue>
 #include <string>
 #include <vector>
 
@@ -130,29 +131,68 @@ GridArgs<float> args_of(const dg_batch *b, int i, int parity) {
     return a;
 }
 
+// When the last of the blocks (one per SM) that take the batch's items in
+// queue order is done, in half planes, with x split into items of `chunk`
+// planes.  An item costs a plane and a half beside its own (it computes two
+// more, their copies run ahead of the item before).
+long long batch_makespan(const dg_batch *b, const std::vector<int> &order, int chunk) {
+    long long start = 0;
+    int combo = -1;
+    std::priority_queue<long long, std::vector<long long>, std::greater<long long>> sms;
+    long long end = 0;
+    for (int i : order) {
+        const GridSlot &s = b->g[i];
+        if (combo_of(s.info) != combo) {                     // another launch
+            combo = combo_of(s.info);
+            start = end;
+            sms = {};
+            for (int k = 0; k < kSms; ++k) sms.push(start);
+        }
+        const int nx = s.nx - 4;
+        const int tiles = ((s.nz - 4 + kTZs - 1) / kTZs) * ((s.ny - 4 + b->tile_rows - 1) / b->tile_rows);
+        for (int x = 0; x < nx; x += chunk)
+            for (int t = 0; t < tiles; ++t) {
+                const long long done = sms.top() + 2 * std::min(chunk, nx - x) + 3;
+                sms.pop();
+                sms.push(done);
+                end = std::max(end, done);
+            }
+    }
+    return end;
+}
+
+// Planes per item: of a few chunks, the one whose items end first.  Long items
+// are wanted where there are many, short ones in a small batch, whose time is
+// one item's planes after another.  Random batches, us per step with 64 planes
+// per item / 16 (the least that the cells per SM were given before) / this
+// rule: 1 grid of 24-40 cells an axis 203 / 98 / 26, 4 of 16-40 176 / 101 / 38,
+// 12 of 20-60 276 / 107 / 89, 12 of 32-90 351 / 181 / 177, 24 of 24-100 376 /
+// 297 / 297, 48 of 32-160 1463 / 1445 / 1432; within 1.5 % of the best in all.
+int auto_chunk(const dg_batch *b, const std::vector<int> &order) {
+    constexpr int cand[] = {64, 48, 40, 32, 28, 24, 20, 16, 12, 10, 8, 6, 5, 4, 3, 2, 1};
+    int best = cand[0];
+    long long t = -1;
+    for (int c : cand) {
+        long long items = 0;
+        for (const GridSlot &s : b->g)
+            items += (long long)((s.nz - 4 + kTZs - 1) / kTZs) * ((s.ny - 4 + b->tile_rows - 1) / b->tile_rows) *
+                     ((s.nx - 4 + c - 1) / c);
+        // more items than this gain nothing: the last of them is a small part
+        if (t >= 0 && items > 16 * kSms) break;
+        const long long m = batch_makespan(b, order, c);
+        if (t < 0 || m < t) {
+            t = m;
+            best = c;
+        }
+    }
+    return best;
+}
+
 // Work items, per-grid arguments and TMA descriptors for the current tiling.
 int rebuild(dg_batch *b) {
     auto fn = encode_fn();
     if (!fn) return bfail(b, DG_ERR_CUDA, "cuTensorMapEncodeTiled not available from the driver");
     const int ty = b->tile_rows;
-    // x-planes per item: as for one grid, sized on the batch's total tiles
-    long long tiles_total = 0;
-    int min_nx = 1 << 30;
-    for (auto &s : b->g) {
-        tiles_total += (long long)((s.ny - 4 + ty - 1) / ty) * ((s.nz - 4 + kTZs - 1) / kTZs);
-        min_nx = std::min(min_nx, s.nx - 4);
-    }
-    int chunk = b->chunk;
-    if (chunk <= 0) {
-        long long cells = 0;
-        for (auto &s : b->g) cells += (long long)(s.nx - 4) * (s.ny - 4) * (s.nz - 4);
-        // ~8 waves of one block per SM worth of items, at least 16 planes
-        const long long items_target = (long long)kSms * 8;
-        const long long tile_cells = (long long)ty * kTZs;
-        long long c = cells / std::max<long long>(1, items_target * tile_cells);
-        chunk = (int)std::max<long long>(16, c);
-    }
-    b->chunk_used = chunk;
     // items: grouped by (limiter, gravity), largest grids first, each grid's
     // items contiguous
     std::vector<int> order(b->n);
@@ -163,6 +203,8 @@ int rebuild(dg_batch *b) {
         auto sz = [&](int i) { return (long long)b->g[i].nx * b->g[i].ny * b->g[i].nz; };
         return sz(x) > sz(y);
     });
+    const int chunk = b->chunk > 0 ? b->chunk : auto_chunk(b, order);
+    b->chunk_used = chunk;
     std::vector<BatchItem> items;
     int off = 0;
     for (int c = 0; c <= kCombos; ++c) b->combo_off[c] = 0;
