@@ -178,11 +178,11 @@ int enqueue(dg_ctx *c, int nsteps) {
         cudaError_t e;
         if (c->elem == 8) {
             auto a = grid_args<double>(c, c->buf[src], c->buf[dst]);
-            e = launch_march(a, &c->tmap[src], c->kind, chunk, c->stream);
+            e = launch_march(a, &c->tmap[src], c->kind, chunk, c->stream, s > 0);
         } else {
             auto a = grid_args<float>(c, c->buf[src], c->buf[dst]);
-            e = c->exact ? launch_march(a, &c->tmap[src], c->kind, chunk, c->stream)
-                         : launch_sweep(a, &c->tmap[src], chunk, c->stream);
+            e = c->exact ? launch_march(a, &c->tmap[src], c->kind, chunk, c->stream, s > 0)
+                         : launch_sweep(a, &c->tmap[src], chunk, c->stream, s > 0);
         }
         if (e != cudaSuccess) return cuda_fail(c, e, "step kernel launch");
         c->cur = dst;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <utility>
 
 namespace dg {
 
@@ -21,6 +22,25 @@ inline cudaError_t ensure_dynamic_smem(Kernel kern, int bytes, std::atomic<unsig
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
     return e;
+}
+
+// A launch that may begin while the one before it in the stream (`overlap`)
+// is still running: that one lets its dependents go, and the kernel itself
+// waits for it where it has to.
+template <class... Params, class... Args>
+inline cudaError_t launch_after(void (*kern)(Params...), int blocks, int threads, int smem, cudaStream_t st,
+                                bool overlap, Args &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
 }  // namespace dg

@@ -254,9 +254,13 @@ void set_global_error(const std::string &msg);
 
 // The step; the tensor map's box is step_box_cols x (step_tile_rows + 4) x 1
 // x 5.  launch_sweep: kFastF32; launch_march: the other kinds.
-cudaError_t launch_sweep(const GridArgs<float> &a, const CUtensorMap *tmap_src, int chunk, cudaStream_t st);
-cudaError_t launch_march(const GridArgs<float> &a, const CUtensorMap *tmap_src, int kind, int chunk, cudaStream_t st);
-cudaError_t launch_march(const GridArgs<double> &a, const CUtensorMap *tmap_src, int kind, int chunk, cudaStream_t st);
+// follows: the launch before it in the stream is a step of the same grid.
+cudaError_t launch_sweep(const GridArgs<float> &a, const CUtensorMap *tmap_src, int chunk, cudaStream_t st,
+                         bool follows = false);
+cudaError_t launch_march(const GridArgs<float> &a, const CUtensorMap *tmap_src, int kind, int chunk, cudaStream_t st,
+                         bool follows = false);
+cudaError_t launch_march(const GridArgs<double> &a, const CUtensorMap *tmap_src, int kind, int chunk, cudaStream_t st,
+                         bool follows = false);
 // A state from src into a.dst with its ghosts, the dt of the coming step
 // (number `step`) and a fresh control block.  prims: src holds primitives;
 // exact: the wave speeds round like the reference (FP64 always does).  src
