@@ -175,14 +175,17 @@ int enqueue(dg_ctx *c, int nsteps) {
     const int chunk = auto_chunk(c);
     for (int s = 0; s < nsteps; ++s) {
         const int src = c->cur, dst = 1 - c->cur;
+        const int chain = (s > 0 ? kChainWait : 0) | (s + 1 < nsteps ? kChainLet : 0);
         cudaError_t e;
         if (c->elem == 8) {
             auto a = grid_args<double>(c, c->buf[src], c->buf[dst]);
-            e = launch_march(a, &c->tmap[src], c->kind, chunk, c->stream, s > 0);
+            a.chain = chain;
+            e = launch_march(a, &c->tmap[src], c->kind, chunk, c->stream);
         } else {
             auto a = grid_args<float>(c, c->buf[src], c->buf[dst]);
-            e = c->exact ? launch_march(a, &c->tmap[src], c->kind, chunk, c->stream, s > 0)
-                         : launch_sweep(a, &c->tmap[src], chunk, c->stream, s > 0);
+            a.chain = chain;
+            e = c->exact ? launch_march(a, &c->tmap[src], c->kind, chunk, c->stream)
+                         : launch_sweep(a, &c->tmap[src], chunk, c->stream);
         }
         if (e != cudaSuccess) return cuda_fail(c, e, "step kernel launch");
         c->cur = dst;

@@ -60,6 +60,7 @@ template <class T> inline GridArgs<T> grid_args(const dg_ctx *c, const void *src
     a.gravity = c->info.gravity;
     a.limiter = c->info.limiter;
     a.nparts = 0;
+    a.chain = 0;
     a.wait_budget = c->wait_budget;
     const T ds = (T)c->info.ds;
     a.k.ds = ds;

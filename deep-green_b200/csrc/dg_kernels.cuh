@@ -56,10 +56,15 @@ template <class T> struct GridArgs {
     int limiter;               // 0 central slopes, 1 minmod
     int nparts;                // work items of this grid in a batched launch
     long long wait_budget;     // SM clocks a wait for a staged plane may take (kWaitBudget)
+    int chain;                 // kChain*: this step among the steps of one call
     Consts<T> k;
     DevCtl *ctl;
     Partial *part;             // conservation sums only (kReduceBlocks entries)
 };
+
+// GridArgs::chain.  Wait: the launch before is the step before, which lets this
+// one start early; Let: the launch after is a step that waits.
+enum : int { kChainWait = 1, kChainLet = 2 };
 
 // Boundary types of dg_sim_info (DG_BC_*) into the kernels' form.  A
 // conducting wall (DG_BC_CONDUCTING_WALL = 3, the reference CUDA variant's
@@ -254,13 +259,9 @@ void set_global_error(const std::string &msg);
 
 // The step; the tensor map's box is step_box_cols x (step_tile_rows + 4) x 1
 // x 5.  launch_sweep: kFastF32; launch_march: the other kinds.
-// follows: the launch before it in the stream is a step of the same grid.
-cudaError_t launch_sweep(const GridArgs<float> &a, const CUtensorMap *tmap_src, int chunk, cudaStream_t st,
-                         bool follows = false);
-cudaError_t launch_march(const GridArgs<float> &a, const CUtensorMap *tmap_src, int kind, int chunk, cudaStream_t st,
-                         bool follows = false);
-cudaError_t launch_march(const GridArgs<double> &a, const CUtensorMap *tmap_src, int kind, int chunk, cudaStream_t st,
-                         bool follows = false);
+cudaError_t launch_sweep(const GridArgs<float> &a, const CUtensorMap *tmap_src, int chunk, cudaStream_t st);
+cudaError_t launch_march(const GridArgs<float> &a, const CUtensorMap *tmap_src, int kind, int chunk, cudaStream_t st);
+cudaError_t launch_march(const GridArgs<double> &a, const CUtensorMap *tmap_src, int kind, int chunk, cudaStream_t st);
 // A state from src into a.dst with its ghosts, the dt of the coming step
 // (number `step`) and a fresh control block.  prims: src holds primitives;
 // exact: the wave speeds round like the reference (FP64 always does).  src

@@ -745,8 +745,7 @@ template <class T, class P, int TY, int R, int LIM, bool GRAV> struct March {
             }
             return;
         }
-        // the next step's blocks may take the SMs that this one's leave
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        if (a.chain & kChainLet) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         finish_speed<true>(a, smax, &s.wmax, gridDim.x);
     }
 };
@@ -758,31 +757,29 @@ template <class T, int TY, int R> constexpr int smem_bytes() {
 
 template <class T, class P, int TY, int R, int LIM, bool GRAV>
 __global__ void __launch_bounds__(32 * (TY + 2), 1)
-    march_step_kernel(const GridArgs<T> a, const __grid_constant__ CUtensorMap tmap, int chunk, int follows) {
+    march_step_kernel(const GridArgs<T> a, const __grid_constant__ CUtensorMap tmap, int chunk) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    if (follows) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (a.chain & kChainWait) asm volatile("griddepcontrol.wait;" ::: "memory");
     March<T, P, TY, R, LIM, GRAV>::run(a, &tmap, chunk, smem_raw);
 }
 
 template <class T, class P, int TY, int R, int LIM, bool GRAV>
-cudaError_t launch_one(const GridArgs<T> &a, const CUtensorMap *tmap, int blocks, int chunk, cudaStream_t st,
-                       bool follows) {
+cudaError_t launch_one(const GridArgs<T> &a, const CUtensorMap *tmap, int blocks, int chunk, cudaStream_t st) {
     auto kern = march_step_kernel<T, P, TY, R, LIM, GRAV>;
     constexpr int smem = smem_bytes<T, TY, R>();
     static std::atomic<unsigned long long> attr_set{0};
     const cudaError_t e = ensure_dynamic_smem(kern, smem, attr_set);
     if (e != cudaSuccess) return e;
-    return launch_after(kern, blocks, 32 * (TY + 2), smem, st, follows, a, *tmap, chunk, follows ? 1 : 0);
+    return launch_after(kern, blocks, 32 * (TY + 2), smem, st, (a.chain & kChainWait) != 0, a, *tmap, chunk);
 }
 
 template <class T, class P, int TY, int R>
-cudaError_t launch(const GridArgs<T> &a, const CUtensorMap *tmap, int blocks, int chunk, cudaStream_t st,
-                   bool follows) {
+cudaError_t launch(const GridArgs<T> &a, const CUtensorMap *tmap, int blocks, int chunk, cudaStream_t st) {
     if (a.gravity)
-        return a.limiter == 0 ? launch_one<T, P, TY, R, 0, true>(a, tmap, blocks, chunk, st, follows)
-                              : launch_one<T, P, TY, R, 1, true>(a, tmap, blocks, chunk, st, follows);
-    return a.limiter == 0 ? launch_one<T, P, TY, R, 0, false>(a, tmap, blocks, chunk, st, follows)
-                          : launch_one<T, P, TY, R, 1, false>(a, tmap, blocks, chunk, st, follows);
+        return a.limiter == 0 ? launch_one<T, P, TY, R, 0, true>(a, tmap, blocks, chunk, st)
+                              : launch_one<T, P, TY, R, 1, true>(a, tmap, blocks, chunk, st);
+    return a.limiter == 0 ? launch_one<T, P, TY, R, 0, false>(a, tmap, blocks, chunk, st)
+                          : launch_one<T, P, TY, R, 1, false>(a, tmap, blocks, chunk, st);
 }
 
 }  // namespace march

@@ -97,6 +97,7 @@ GridArgs<T> args_for(const dg_sim_info *info, const void *src, void *dst, void *
     a.gravity = info->gravity;
     a.limiter = info->limiter;
     a.nparts = 0;
+    a.chain = 0;
     a.wait_budget = 0;
     const T ds = (T)info->ds;
     a.k.ds = ds;

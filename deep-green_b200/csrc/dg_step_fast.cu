@@ -21,7 +21,7 @@ constexpr int kSweepRing = sizeof(sweep::Smem<float, kSweepRowsF32, 5>) + 1024 <
 // kernel over all tiles.  (One kernel body holding both variants of the
 // loop ran slower than either alone.)
 template <int LIM, bool GRAV>
-cudaError_t launch_sweep_t(const GridArgs<float> &a, const CUtensorMap *tmap, int chunk, cudaStream_t st, bool follows) {
+cudaError_t launch_sweep_t(const GridArgs<float> &a, const CUtensorMap *tmap, int chunk, cudaStream_t st) {
     constexpr int TY = kSweepRowsF32, R = kSweepRing;
     auto k_in = sweep::sweep_step_kernel<float, TY, R, LIM, GRAV, true>;
     auto k_frame = sweep::sweep_step_kernel<float, TY, R, LIM, GRAV, false>;
@@ -36,25 +36,22 @@ cudaError_t launch_sweep_t(const GridArgs<float> &a, const CUtensorMap *tmap, in
     const int n_fr = it.frame() * ((a.nx - 4 + chunk - 1) / chunk);
     const int nparts = n_in + n_fr;
     if (n_in > 0) {
-        k_in<<<n_in, 32 * (TY + 2), smem, st>>>(a, *tmap, chunk_in, nparts, 0);
+        k_in<<<n_in, 32 * (TY + 2), smem, st>>>(a, *tmap, chunk_in, nparts);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    // `follows` concerns the launch before this step: the frame waits for it
-    // only where it is the whole step
-    return launch_after(k_frame, n_fr, 32 * (TY + 2), smem, st, n_in > 0 || follows, a, *tmap, chunk, nparts,
-                        n_in == 0 && follows ? 1 : 0);
+    return launch_after(k_frame, n_fr, 32 * (TY + 2), smem, st, n_in > 0 || (a.chain & kChainWait), a, *tmap, chunk,
+                        nparts);
 }
 
 }  // namespace
 
 // One kernel per (limiter, gravity): the slope and flux code of the march
 // is fixed at compile time.
-cudaError_t launch_sweep(const GridArgs<float> &a, const CUtensorMap *tmap, int chunk, cudaStream_t st,
-                         bool follows) {
+cudaError_t launch_sweep(const GridArgs<float> &a, const CUtensorMap *tmap, int chunk, cudaStream_t st) {
     if (a.gravity)
-        return a.limiter == 0 ? launch_sweep_t<0, true>(a, tmap, chunk, st, follows) : launch_sweep_t<1, true>(a, tmap, chunk, st, follows);
-    return a.limiter == 0 ? launch_sweep_t<0, false>(a, tmap, chunk, st, follows) : launch_sweep_t<1, false>(a, tmap, chunk, st, follows);
+        return a.limiter == 0 ? launch_sweep_t<0, true>(a, tmap, chunk, st) : launch_sweep_t<1, true>(a, tmap, chunk, st);
+    return a.limiter == 0 ? launch_sweep_t<0, false>(a, tmap, chunk, st) : launch_sweep_t<1, false>(a, tmap, chunk, st);
 }
 
 template cudaError_t launch_cons_to_prim_policy<float, false>(const GridArgs<float> &, const float *, float *,

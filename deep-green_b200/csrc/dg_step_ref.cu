@@ -10,18 +10,16 @@
 
 namespace dg {
 
-cudaError_t launch_march(const GridArgs<double> &a, const CUtensorMap *tmap, int kind, int chunk, cudaStream_t st,
-                         bool follows) {
+cudaError_t launch_march(const GridArgs<double> &a, const CUtensorMap *tmap, int kind, int chunk, cudaStream_t st) {
     const int blocks = step_grid_blocks(a.nx, a.ny, a.nz, kind, chunk);
     return kind == kFastF64
-               ? march::launch<double, march::FusedArith, kMarchRows, kMarchRing>(a, tmap, blocks, chunk, st, follows)
-               : march::launch<double, march::RefArith<double>, kMarchRows, kMarchRing>(a, tmap, blocks, chunk, st, follows);
+               ? march::launch<double, march::FusedArith, kMarchRows, kMarchRing>(a, tmap, blocks, chunk, st)
+               : march::launch<double, march::RefArith<double>, kMarchRows, kMarchRing>(a, tmap, blocks, chunk, st);
 }
 
-cudaError_t launch_march(const GridArgs<float> &a, const CUtensorMap *tmap, int kind, int chunk, cudaStream_t st,
-                         bool follows) {
+cudaError_t launch_march(const GridArgs<float> &a, const CUtensorMap *tmap, int kind, int chunk, cudaStream_t st) {
     const int blocks = step_grid_blocks(a.nx, a.ny, a.nz, kind, chunk);
-    return march::launch<float, march::RefArith<float>, kMarchRows, kMarchRing>(a, tmap, blocks, chunk, st, follows);
+    return march::launch<float, march::RefArith<float>, kMarchRows, kMarchRing>(a, tmap, blocks, chunk, st);
 }
 
 template <class T, bool EXACT, bool PRIM>

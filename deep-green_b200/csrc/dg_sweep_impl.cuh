@@ -1088,7 +1088,7 @@ template <class T, int TY, int R, int LIM, bool GRAV> struct Sweep {
         if (tid == 0)
             for (int i = 0; i < R; ++i) mbar_inval(&s.bar[i]);
         if constexpr (!IN)
-            if (nparts == (int)gridDim.x) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+            if (a.chain & kChainLet) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         finish_speed<true>(a, smax, &s.wmax, nparts);
         return true;
     }
@@ -1117,23 +1117,22 @@ template <int TY> constexpr int sweep_max_regs() {
 // dependent launch, launch_sweep).  They share one reduction over their
 // nparts blocks: whichever block of either takes the last ticket advances dt
 // (every block has read the step's dt by then).  Without interior tiles the
-// frame launch is the whole step; with `follows` the launch before it in the
-// stream is such a step too, and its blocks take the SMs as that one's blocks
-// leave them, then wait for all of it (64^3: 22.4 instead of 24.7 us per step,
-// 128x112x128 64.5 instead of 65.9; with the dependents let go at the start of
-// a block instead of before its last reduction 22.8 and 67.1).
+// frame launch is the whole step, and within one call (a.chain) a step's blocks
+// take the SMs as those of the step before leave them, then wait for all of it
+// (64^3: 23.5 instead of 24.7 us per step, 128x112x128 64.6 instead of 66.3;
+// with the dependents let go at the start of a block instead of before its last
+// reduction 22.8 and 67.1).
 template <class T, int TY, int R, int LIM, bool GRAV, bool IN>
 __global__ void __maxnreg__(sweep_max_regs<TY>()) sweep_step_kernel(const GridArgs<T> a,
                                                                       const __grid_constant__ CUtensorMap tmap,
-                                                                      int chunk, int nparts, int follows) {
+                                                                      int chunk, int nparts) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    if constexpr (!IN) {
-        if (follows) asm volatile("griddepcontrol.wait;" ::: "memory");
-    }
+    const InteriorTiles it(a.ny, a.nz, TY, kTileZ);
+    if constexpr (!IN)
+        if ((a.chain & kChainWait) && it.interior() == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
     // the frame launch reads nothing this launch writes: let it start on the
     // SMs this launch leaves free
     if constexpr (IN) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const InteriorTiles it(a.ny, a.nz, TY, kTileZ);
     int b = blockIdx.x, ty, tz;
     if constexpr (IN) {
         tz = 1 + b % it.nz;
