@@ -44,6 +44,7 @@ struct dg_net {
     int device = 0;
     int inputs = 0, outputs = 0;
     cudaStream_t stream = nullptr;
+    cudaEvent_t ready = nullptr;       // the caller's work on the default stream (after_default_stream)
     float *w[4] = {}, *b[4] = {};
     float *gw[4] = {}, *gb[4] = {};
     float *mw[4] = {}, *vw[4] = {}, *mb[4] = {}, *vb[4] = {};
@@ -574,6 +575,17 @@ int forward(dg_net *net, const void *feat, int n, int x, int y, int z, float *ou
     return DG_OK;
 }
 
+// The network's stream does not wait for the default stream by itself, and a
+// training loop that fills its batch there (dg_learned_features with stream
+// NULL) would have the forward pass read it half written: the one launch of
+// the optimizer leaves it no time.  The calls that return a loss synchronise
+// anyway, so they also wait for that work.
+int after_default_stream(dg_net *net) {
+    NET_CUDA(net, cudaEventRecord(net->ready, cudaStreamLegacy));
+    NET_CUDA(net, cudaStreamWaitEvent(net->stream, net->ready, 0));
+    return DG_OK;
+}
+
 // Backward pass from the output gradient in ws.dz[3] down to the weights of
 // layer 0 (weight gradients of every layer, input gradients of layers 1-3).
 int backward(dg_net *net, const void *feat, int n, int x, int y, int z) {
@@ -648,6 +660,7 @@ int32_t dg_net_create(const dg_net_info *info, dg_net **out) {
         return true;
     };
     if (!cu(cudaStreamCreateWithFlags(&net->stream, cudaStreamNonBlocking), "stream")) return bail(DG_ERR_CUDA);
+    if (!cu(cudaEventCreateWithFlags(&net->ready, cudaEventDisableTiming), "event")) return bail(DG_ERR_CUDA);
     size_t maxrow = 0;
     for (int l = 0; l < 4; ++l) {
         const size_t nw = (size_t)27 * kCin[l] * kCout[l], nb = kCout[l];
@@ -705,6 +718,7 @@ int32_t dg_net_destroy(dg_net *net) {
     cudaFree(net->loss_part);
     cudaFree(net->pow_part);
     cudaFree(net->status);
+    if (net->ready) cudaEventDestroy(net->ready);
     if (net->stream) cudaStreamDestroy(net->stream);
     delete net;
     return DG_OK;
@@ -785,6 +799,7 @@ int32_t dg_net_forward_backward(dg_net *net, const void *feat, const float *targ
     NET_CUDA(net, cudaSetDevice(net->device));
     if (int r = ensure_ws(net, n, x, y, z, true)) return r;
     Workspace &ws = net->ws;
+    if (int r = after_default_stream(net)) return r;
     if (int r = forward(net, feat, n, x, y, z, ws.out, true, net->stream)) return r;
     const int xo = x - 8, yo = y - 8, zo = z - 8;
     const long long nvox = (long long)n * xo * yo * zo;
@@ -829,6 +844,7 @@ int32_t dg_net_forward_backward_flux(dg_net *net, const void *feat, const float 
         ws.gbuf_elems = ntgt * 5;
     }
     ws.wsample = ws.gbuf + ws.gbuf_elems;
+    if (int r = after_default_stream(net)) return r;
     if (int r = forward(net, feat, n, x, y, z, ws.out, true, net->stream)) return r;
     const float scale = (float)(2.0 / ((double)ntgt * 5));
     const int lblocks = (int)std::min<long long>(4096, (ntgt + 255) / 256);

@@ -61,7 +61,8 @@ int32_t dg_net_get_grad(dg_net *net, int32_t layer, float *gw, float *gb);
  * network's stream. */
 int32_t dg_net_forward(dg_net *net, const void *feat, int32_t n, int32_t x, int32_t y, int32_t z, float *out);
 
-/* One forward + backward pass.  feat: device BF16 [n][x][y][z][16]; target:
+/* One forward + backward pass, after all work enqueued so far on the default
+ * stream (NULL) and on the network's own.  feat: device BF16 [n][x][y][z][16]; target:
  * device FP32 [n][x-8][y-8][z-8][16] (first `outputs` channels used).  Loss
  * = mean over positions and real outputs of (out - target)^2, returned in
  * *loss (synchronises).  Gradients are kept in the network (replacing the
