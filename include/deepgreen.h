@@ -207,8 +207,8 @@ int32_t dg_compute_step_dt(dg_ctx *ctx, double dt);
  *             cannot see the device's status: read it with
  *             dg_noalloc_status after synchronizing the stream.
  *   stream    cudaStream_t or NULL.
- * The step's scratch (control block and per-block partials) is a 1 MiB
- * array in the library's device image, held by every GPU that loads the
+ * The step's scratch (the control block, and room for 64 bytes per block of
+ * the step) is a 1 MiB array in the library's device image, held by every GPU that loads the
  * library until exit; grids needing more than it holds are rejected with
  * DG_ERR_INVALID.  All calls share that array: calls that overlap on the
  * GPU race.  The first call on a device looks up the array's address with
