@@ -56,10 +56,11 @@ template <class T> struct GridArgs {
     int limiter;               // 0 central slopes, 1 minmod
     int nparts;                // work items of this grid in a batched launch
     long long wait_budget;     // SM clocks a wait for a staged plane may take (kWaitBudget)
-    int chain;                 // kChain*: this step among the steps of one call
     Consts<T> k;
     DevCtl *ctl;
     Partial *part;             // conservation sums only (kReduceBlocks entries)
+    int chain;                 // kChain*: this step among the steps of one call (here, not ahead of k: the
+                               // constants keep their alignment, 3.09 instead of 3.18 ms per 512^3 step)
 };
 
 // GridArgs::chain.  Wait: the launch before is the step before, which lets this
