@@ -217,12 +217,13 @@ inline int waves_chunk(long long tiles, int nxi, long long small) {
 // interior tiles that fill the SMs: the frame launch's chunk (the interior
 // launch marches whole columns); with fewer interior tiles: the split of x that
 // minimises waves x (planes + 3 re-staged), at least 24 planes per block
-// unless that leaves SMs idle (40x300x130: 181 -> 102 us); with none, the split that ends first (sweep_makespan), down
-// to single planes: a small grid is latency-bound, a block's time being its
-// planes one after another, so short chunks on all SMs win although each
-// block recomputes two planes (FP32, periodic, us per step, at least 24
-// planes per block -> this rule: 48^3 116 -> 25, 64^3 146 -> 29, 128^3
-// 124 -> 93, 300x40x70 116 -> 75).
+// unless that leaves SMs idle (40x300x130: 181 -> 102 us); with none, the
+// split that ends first (sweep_makespan), down to single planes: a small grid
+// is latency-bound, a block's time being its planes one after another, so
+// short chunks on all SMs win although each block recomputes two planes (FP32,
+// periodic, us per step when the rule was chosen, at least 24 planes per block
+// -> this rule: 48^3 116 -> 25, 64^3 146 -> 29, 128^3 124 -> 93, 300x40x70 116
+// -> 75).
 inline int choose_chunk(int nx, int ny, int nz, int kind) {
     const int ty = step_tile_rows(kind), tzc = step_tile_cols(kind);
     // sweep steps whose interior tiles fill the SMs (interior_chunk): the

@@ -1119,9 +1119,9 @@ template <int TY> constexpr int sweep_max_regs() {
 // (every block has read the step's dt by then).  Without interior tiles the
 // frame launch is the whole step, and within one call (a.chain) a step's blocks
 // take the SMs as those of the step before leave them, then wait for all of it
-// (64^3: 23.5 instead of 24.7 us per step, 128x112x128 64.6 instead of 66.3;
+// (64^3: 22.0 instead of 23.9 us per step, 128x112x128 64.0 instead of 66.0;
 // with the dependents let go at the start of a block instead of before its last
-// reduction 22.8 and 67.1).
+// reduction the larger grid took 67).
 template <class T, int TY, int R, int LIM, bool GRAV, bool IN>
 __global__ void __maxnreg__(sweep_max_regs<TY>()) sweep_step_kernel(const GridArgs<T> a,
                                                                       const __grid_constant__ CUtensorMap tmap,
