@@ -69,6 +69,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "dg_conv_index.h"
 #include "dg_tc.cuh"
 
 namespace dg {
@@ -452,10 +453,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                     s[c + 1] = r.y;
                 }
             };
-            // position of the column's plane 0 in the outputs
-            const long long o0 = ((((long long)b * a.ox + x0 + a.off) * a.oy + y + a.off) * a.oz + z + a.off) * COUT + c0;
-            const long long d0 = ((((long long)b * a.xo + x0) * a.yo + y) * a.zo + z) * COUT + c0;
-            const int ostep = a.oy * a.oz * COUT, dstep = a.yo * a.zo * COUT;
+            // the column's planes in the output buffer and in a dense tensor of
+            // the output's extents
+            const PlaneIndex oi(b, x0 + a.off, y + a.off, z + a.off, a.ox, a.oy, a.oz, COUT, c0);
+            const PlaneIndex di(b, x0, y, z, a.xo, a.yo, a.zo, COUT, c0);
             for (int k = 0; k < len + 2; ++k, ++g) {
                 if ((int)(g % kEpiGroups) != grp) continue;
                 const int sl = (int)(g % R);
@@ -490,7 +491,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                 if (k < 2 || !valid) continue;
                 if constexpr (kIssuers == 2) add2(v, v2);
 
-                const long long o = o0 + (long long)(k - 2) * ostep, dn = d0 + (long long)(k - 2) * dstep;
+                const long long o = oi.plane(k - 2), dn = di.plane(k - 2);
                 // one 32-byte store per lane and tensor where the columns allow
                 // (COUT 32: 16 BF16 columns; COUT 16: 8 FP32 columns)
                 if constexpr (EPI == kEpiGelu) {
