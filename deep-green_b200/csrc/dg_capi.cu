@@ -10,12 +10,12 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 #include <new>
 #include <string>
 
 #include "../../include/deepgreen.h"
 #include "dg_ctx.h"
+#include "dg_pointer.h"
 
 using namespace dg;
 
@@ -25,17 +25,43 @@ namespace {
 // message of the calling thread's last failure outside a context
 thread_local std::string g_create_err = "no error";
 
+// A driver function by name, or NULL.
+template <class Fn> Fn driver_fn(const char *name) {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+        return reinterpret_cast<Fn>(p);
+    return nullptr;
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 get_encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    });
+    static const auto fn = driver_fn<PFN_cuTensorMapEncodeTiled_v12000>("cuTensorMapEncodeTiled");
     return fn;
+}
+
+// What the driver says of p (nothing known: not device memory).
+PointerInfo pointer_info(const void *p) {
+    static const auto get = driver_fn<PFN_cuPointerGetAttributes_v7000>("cuPointerGetAttributes");
+    static const auto current = driver_fn<PFN_cuCtxGetCurrent_v4000>("cuCtxGetCurrent");
+    PointerInfo m = {false, -1, false, 0, 0};
+    unsigned type = 0, managed = 0;
+    int device = -1;
+    CUcontext owner = nullptr, own = nullptr;
+    unsigned long long start = 0;
+    size_t size = 0;
+    CUpointer_attribute attr[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,      CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,   CU_POINTER_ATTRIBUTE_CONTEXT,
+                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *out[] = {&type, &managed, &device, &owner, &start, &size};
+    if (!get || !current || current(&own) != CUDA_SUCCESS ||
+        get(6, attr, out, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS)
+        return m;
+    m.device_memory = type == CU_MEMORYTYPE_DEVICE && !managed;
+    m.device = device;
+    m.foreign_context = owner && owner != own;      // memory of pools has no context
+    m.start = (uintptr_t)start;
+    m.size = size;
+    return m;
 }
 
 int auto_chunk(const dg_ctx *c) {
@@ -142,6 +168,27 @@ int download_dense(dg_ctx *c, void *const dst[5], const void *dense) {
     for (int f = 0; f < 5; ++f)
         DG_CUDA(c, cudaMemcpyAsync(dst[f], static_cast<const char *>(dense) + f * fb, fb, cudaMemcpyDeviceToHost,
                                    c->stream));
+    return DG_OK;
+}
+
+// Whether the kernels may access the caller's five dense device fields.
+bool kernel_fields(const dg_ctx *c, const void *const f[5]) {
+    for (int i = 0; i < 5; ++i)
+        if (!kernel_may_access(pointer_info(f[i]), reinterpret_cast<uintptr_t>(f[i]), dense_field_bytes(c),
+                               (size_t)c->elem, c->info.device))
+            return false;
+    return true;
+}
+
+// The current state into or from dense device fields that they may not, by
+// copies between the layouts.
+int copy_fields(dg_ctx *c, void *const dense[5], bool in) {
+    const size_t row = (size_t)c->nz * c->elem, pitched = (size_t)c->pitch * c->elem;
+    for (int f = 0; f < 5; ++f) {
+        char *own = static_cast<char *>(c->buf[c->cur]) + (size_t)f * c->fstride * c->elem;
+        DG_CUDA(c, cudaMemcpy2DAsync(in ? own : dense[f], in ? pitched : row, in ? dense[f] : own, in ? row : pitched,
+                                     row, (size_t)c->nx * c->ny, cudaMemcpyDeviceToDevice, c->stream));
+    }
     return DG_OK;
 }
 
@@ -349,7 +396,12 @@ int32_t dg_set_conserved_device(dg_ctx *c, const void *const cons[5]) {
     if ((r = reset_ctl(c)) != DG_OK) return r;
     void *src[5];
     for (int f = 0; f < 5; ++f) src[f] = const_cast<void *>(cons[f]);
-    if ((r = finish_state(c, src)) != DG_OK) return r;
+    if (kernel_fields(c, cons)) {
+        if ((r = finish_state(c, src)) != DG_OK) return r;
+    } else {
+        if ((r = copy_fields(c, src, true)) != DG_OK) return r;
+        if ((r = finish_state(c)) != DG_OK) return r;
+    }
     return check_flags(c);
 }
 
@@ -442,7 +494,7 @@ int32_t dg_get_conserved_device(dg_ctx *c, void *const cons[5]) {
     if (!c->has_state) return fail(c, DG_ERR_NO_STATE, "no state set");
     int r;
     if ((r = use_device(c)) != DG_OK) return r;
-    if ((r = get_state(c, cons)) != DG_OK) return r;
+    if ((r = kernel_fields(c, cons) ? get_state(c, cons) : copy_fields(c, cons, false)) != DG_OK) return r;
     // the destination belongs to the caller's streams: return after the copies
     DG_CUDA(c, cudaStreamSynchronize(c->stream));
     return DG_OK;

@@ -146,11 +146,13 @@ int32_t dg_conservation_sums(dg_ctx *ctx, double out[5]);
 
 /* Device-pointer variants of dg_set_conserved / dg_get_conserved for
  * callers that keep the fields in their own CUDA allocations (same layout
- * as the host arrays).  The copies run on the context's stream, a
- * non-blocking stream that does not order against the caller's streams:
- * work that writes the source fields must be complete when
- * dg_set_conserved_device is called.  Both calls return after their copies
- * finished. */
+ * as the host arrays).  Fields in this GPU's own memory, aligned to their
+ * elements, are read and written by the kernels themselves; all others that
+ * a device-to-device copy reaches (on another GPU, unaligned) are copied.
+ * Both run on the context's stream, a non-blocking stream that does not
+ * order against the caller's streams: work that writes the source fields
+ * must be complete when dg_set_conserved_device is called.  Both calls
+ * return when they are done with the fields. */
 int32_t dg_set_conserved_device(dg_ctx *ctx, const void *const cons[5]);
 int32_t dg_get_conserved_device(dg_ctx *ctx, void *const cons[5]);
 
