@@ -384,7 +384,7 @@ def train(net: Net, ps: PairSet, norm: Norm, steps: int, batch: int = 8, crop: i
     hist = []
     t0 = time.time()
     for it in range(steps):
-        b.fill(norm, net.stream())
+        b.fill(norm)       # behind the buffers' zeroing; the pass waits for the default stream
         loss = net.forward_backward_flux(b.feat, b.tgt, balance)
         rate = lr_min + 0.5 * (lr - lr_min) * (1.0 + math.cos(math.pi * it / max(steps, 1)))
         net.adam_step(rate)
