@@ -44,7 +44,7 @@ struct dg_net {
     int device = 0;
     int inputs = 0, outputs = 0;
     cudaStream_t stream = nullptr;
-    cudaEvent_t ready = nullptr;       // the caller's work on the default stream (after_default_stream)
+    cudaEvent_t ready = nullptr;       // work of another stream (order_streams)
     float *w[4] = {}, *b[4] = {};
     float *gw[4] = {}, *gb[4] = {};
     float *mw[4] = {}, *vw[4] = {}, *mb[4] = {}, *vb[4] = {};
@@ -575,16 +575,19 @@ int forward(dg_net *net, const void *feat, int n, int x, int y, int z, float *ou
     return DG_OK;
 }
 
+// `to` waits for all work enqueued so far on `from`.
+int order_streams(dg_net *net, cudaStream_t from, cudaStream_t to) {
+    NET_CUDA(net, cudaEventRecord(net->ready, from));
+    NET_CUDA(net, cudaStreamWaitEvent(to, net->ready, 0));
+    return DG_OK;
+}
+
 // The network's stream does not wait for the default stream by itself, and a
 // training loop that fills its batch there (dg_learned_features with stream
 // NULL) would have the forward pass read it half written: the one launch of
 // the optimizer leaves it no time.  The calls that return a loss synchronise
 // anyway, so they also wait for that work.
-int after_default_stream(dg_net *net) {
-    NET_CUDA(net, cudaEventRecord(net->ready, cudaStreamLegacy));
-    NET_CUDA(net, cudaStreamWaitEvent(net->stream, net->ready, 0));
-    return DG_OK;
-}
+int after_default_stream(dg_net *net) { return order_streams(net, cudaStreamLegacy, net->stream); }
 
 // Backward pass from the output gradient in ws.dz[3] down to the weights of
 // layer 0 (weight gradients of every layer, input gradients of layers 1-3).
@@ -620,7 +623,11 @@ int backward(dg_net *net, const void *feat, int n, int x, int y, int z) {
 int dg::net_forward_stream(dg_net *net, const void *feat, int n, int x, int y, int z, float *out, cudaStream_t st) {
     if (int r = check_extents(net, n, x, y, z)) return r;
     if (int r = ensure_ws(net, n, x, y, z, false)) return r;
-    return forward(net, feat, n, x, y, z, out, false, st);
+    // Weights and workspace belong to the network's stream: an update enqueued
+    // there comes before this pass, and this pass before the next one.
+    if (int r = order_streams(net, net->stream, st)) return r;
+    if (int r = forward(net, feat, n, x, y, z, out, false, st)) return r;
+    return order_streams(net, st, net->stream);
 }
 
 int dg::net_inputs(const dg_net *net) { return net->inputs; }
