@@ -477,8 +477,8 @@ int32_t dg_compute_step_dt(dg_ctx *c, double dt) {
 
 int32_t dg_get_conserved(dg_ctx *c, void *const cons[5]) {
     if (!c || !cons) return fail(c, DG_ERR_INVALID, "null argument");
-    if (null_field(cons)) return fail(c, DG_ERR_INVALID, "null field pointer");
     if (!c->has_state) return fail(c, DG_ERR_NO_STATE, "no state set");
+    if (null_field(cons)) return fail(c, DG_ERR_INVALID, "null field pointer");
     int r;
     if ((r = use_device(c)) != DG_OK) return r;
     if (!c->prim_scratch) DG_CUDA(c, cudaMalloc(&c->prim_scratch, c->state_bytes));
@@ -490,8 +490,8 @@ int32_t dg_get_conserved(dg_ctx *c, void *const cons[5]) {
 
 int32_t dg_get_conserved_device(dg_ctx *c, void *const cons[5]) {
     if (!c || !cons) return fail(c, DG_ERR_INVALID, "null argument");
-    if (null_field(cons)) return fail(c, DG_ERR_INVALID, "null field pointer");
     if (!c->has_state) return fail(c, DG_ERR_NO_STATE, "no state set");
+    if (null_field(cons)) return fail(c, DG_ERR_INVALID, "null field pointer");
     int r;
     if ((r = use_device(c)) != DG_OK) return r;
     if ((r = kernel_fields(c, cons) ? get_state(c, cons) : copy_fields(c, cons, false)) != DG_OK) return r;
@@ -502,8 +502,8 @@ int32_t dg_get_conserved_device(dg_ctx *c, void *const cons[5]) {
 
 int32_t dg_get_primitives(dg_ctx *c, void *const prim[5]) {
     if (!c || !prim) return fail(c, DG_ERR_INVALID, "null argument");
-    if (null_field(prim)) return fail(c, DG_ERR_INVALID, "null field pointer");
     if (!c->has_state) return fail(c, DG_ERR_NO_STATE, "no state set");
+    if (null_field(prim)) return fail(c, DG_ERR_INVALID, "null field pointer");
     int r;
     if ((r = use_device(c)) != DG_OK) return r;
     if (!c->prim_scratch) DG_CUDA(c, cudaMalloc(&c->prim_scratch, c->state_bytes));
