@@ -19,8 +19,9 @@
 //     address dz rows further.  Positions with z >= Zin-2 wrap into the next
 //     row and are dropped by the epilogue (2 of every Zin positions).
 //   * a block walks along x through columns of tiles (fixed n and p range), an
-//     equal share of all planes per block (Share).  Input plane P serves output planes P, P-1 and P-2 (taps
-//     dx = 0, 1, 2), so each (dy, dz, 16 channels) is ONE MMA with N = 3 COUT
+//     equal share of all planes per block (Share, dg_conv_index.h).  Input
+//     plane P serves output planes P, P-1 and P-2 (taps dx = 0, 1, 2), so each
+//     (dy, dz, 16 channels) is ONE MMA with N = 3 COUT
 //     against the weights [W(dx=2) | W(dx=1) | W(dx=0)]: its three column
 //     blocks land in the TMEM accumulators of output planes P-2, P-1, P,
 //     which sit in a ring of 8 consecutive slots (an MMA that would wrap the
@@ -118,48 +119,6 @@ struct WgradArgs {
     int nunits;                     // work units (n, x, z segment, y chunk): nb * xo * nseg * nyc
     float *part;                    // per block: [COUT][CIN][27] weight partials then [COUT] bias partials
     unsigned *status;
-};
-
-// A block's share of the work: columns of `len` steps, `work` steps in all.
-// As many rounds of whole columns as every block gets one of, neighbouring
-// columns at neighbouring steps (each block starts a column a little further
-// in and wraps around), so that the rows they share come from L2 without all
-// blocks asking for one plane at once; then an equal range of the remaining
-// columns' steps.  next() gives a column, its first step and the count of
-// steps in it.  (Fixed chunks of 64 planes left a third of the SMs idle at the
-// end of a layer of 200^3, and half of them on columns a little longer than a
-// chunk, whose short remainders all fell to the odd blocks, as on training
-// crops.)  A column's outputs do not depend on the split.
-struct Share {
-    long long column, pos, end;
-    int len, rounds, shift;
-    bool wrapped = false;
-    __device__ __forceinline__ Share(long long work, int len_)
-        : column(blockIdx.x), len(len_), shift((int)((long long)len_ * blockIdx.x / gridDim.x)) {
-        const long long columns = work / len, whole = columns / gridDim.x * gridDim.x, rest = (columns - whole) * len;
-        rounds = (int)(columns / gridDim.x);
-        pos = whole * len + rest * blockIdx.x / gridDim.x;
-        end = whole * len + rest * (blockIdx.x + 1) / gridDim.x;
-    }
-    __device__ __forceinline__ bool next(long long &col, int &first, int &count) {
-        if (rounds > 0) {
-            col = column;
-            first = wrapped ? 0 : shift;
-            count = wrapped ? shift : len - shift;
-            if (wrapped || shift == 0) {
-                --rounds;
-                column += gridDim.x;
-                wrapped = false;
-            } else wrapped = true;
-            return true;
-        }
-        if (pos >= end) return false;
-        col = pos / len;
-        first = (int)(pos - col * len);
-        count = (int)min((long long)(len - first), end - pos);
-        pos += count;
-        return true;
-    }
 };
 
 __device__ __forceinline__ unsigned char *align1024(unsigned char *p) {
@@ -340,7 +299,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             mbar_expect_tx(wbar, L::WB);
             tc::bulk_load(wsm, wpack, L::WB, wbar);
             long long g = 0;                      // planes issued by this block
-            Share share(a.work, a.xo);
+            Share share(a.work, a.xo, blockIdx.x, gridDim.x);
             long long column;
             int x0, len;
             while (ok && share.next(column, x0, len)) {
@@ -371,7 +330,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         long long g = 0;                      // input planes consumed = output slots completed
         const uint64_t b0 = tc::sdesc_sw(smem_u32(wsm), ROW);
         const uint32_t rbase = tbase + (uint32_t)(me * RING);
-        Share share(a.work, a.xo);
+        Share share(a.work, a.xo, blockIdx.x, gridDim.x);
         long long column;
         int x0, len;
         while (ok && share.next(column, x0, len)) {
@@ -437,7 +396,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         ok &= warp_wait(drain + me, 0);
     } else {
         long long g = 0;
-        Share share(a.work, a.xo);
+        Share share(a.work, a.xo, blockIdx.x, gridDim.x);
         long long column;
         int x0, len;
         while (ok && share.next(column, x0, len)) {
