@@ -30,14 +30,31 @@ template <class T> __global__ void __launch_bounds__(256) sums_kernel(const Grid
     long long c = blockIdx.x * 256LL + tid;
     int x = (int)(c / (nyi * nzi)), y = (int)((c / nzi) % nyi), z = (int)(c % nzi);
     const int sx = (int)(stride / (nyi * nzi)), sy = (int)((stride / nzi) % nyi), sz = (int)(stride % nzi);
-    for (; c < total; c += stride) {
-        const long long o = ((long long)(x + 2) * a.ny + (y + 2)) * a.pitch + (z + 2);
-        z += sz;
-        if (z >= nzi) { z -= (int)nzi; ++y; }
-        y += sy;
-        if (y >= nyi) { y -= (int)nyi; ++x; }
-        x += sx;
-        for (int f = 0; f < 5; ++f) sum[f] += (double)a.src[f * a.fstride + o];
+    // kAhead cells' loads in flight before their additions, which keep their
+    // order (508^3 FP32 985 us with one load after the other, 687 / 620 / 500 /
+    // 672 with 1 / 2 / 4 / 8 cells; 300^3 FP64 243, 203 / 254 / 192 / 292)
+    constexpr int kAhead = 4;
+    while (c < total) {
+        T u[kAhead][5];
+        const long long left = (total - 1 - c) / stride;   // cells behind this one
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            const long long o = ((long long)(x + 2) * a.ny + (y + 2)) * a.pitch + (z + 2);
+#pragma unroll
+            for (int f = 0; f < 5; ++f) u[k][f] = k <= left ? a.src[f * a.fstride + o] : T(0);
+            z += sz;
+            if (z >= nzi) { z -= (int)nzi; ++y; }
+            y += sy;
+            if (y >= nyi) { y -= (int)nyi; ++x; }
+            x += sx;
+        }
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+            if (k <= left) {
+#pragma unroll
+                for (int f = 0; f < 5; ++f) sum[f] += (double)u[k][f];
+            }
+        c += kAhead * stride;
     }
     auto block_sum = [&](int f) {
         double t = 0;
