@@ -8,12 +8,12 @@
 // over allocation at all.  The context API (dg_create) allocates its state
 // buffers and its scratch; this entry point allocates nothing: the caller
 // passes the input and output states, and the step's scratch memory (the
-// step control block and the per-block partial results of the dt / sum
-// reductions) lives in a fixed-size array in the library's own device image.
+// step control block) lives in a fixed-size array in the library's own device
+// image.
 //
 // Limits and rules:
-//   * the scratch array is 1 MiB; grids that need more than kMaxBlocks
-//     blocks are rejected with DG_ERR_INVALID;
+//   * the scratch array is 1 MiB; grids above the limit that it once set are
+//     rejected with DG_ERR_INVALID (dg_noalloc_limit.h);
 //   * every GPU that loads the library holds this 1 MiB until the process
 //     exits;
 //   * all calls share the one array (per device): calls that overlap on the
@@ -24,7 +24,6 @@
 //     before any stream capture.
 #include <cudaTypedefs.h>
 
-#include <algorithm>
 #include <cstddef>
 #include <cstring>
 #include <mutex>
@@ -32,15 +31,13 @@
 
 #include "../../include/deepgreen.h"
 #include "dg_kernels.cuh"
+#include "dg_noalloc_limit.h"
 
 namespace dg {
 namespace {
 
 constexpr size_t kNoAllocScratchBytes = 1u << 20;
 constexpr size_t kPartialOffset = (sizeof(DevCtl) + 255) / 256 * 256;
-// Blocks a step may have: the scratch once held 64 bytes of partial results
-// per block, and the limit on a grid's size stays what that made it.
-constexpr int kMaxBlocks = (int)((kNoAllocScratchBytes - kPartialOffset) / 64);
 static_assert((kNoAllocScratchBytes - kPartialOffset) / sizeof(Partial) >= kReduceBlocks, "partials of the sums");
 
 // The scratch.  In host code this name is only a stand-in for the device
@@ -117,40 +114,18 @@ GridArgs<T> args_for(const dg_sim_info *info, const void *src, void *dst, void *
     return a;
 }
 
-// The block count that decides whether a grid fits the scratch: that of the
-// kernels and splits this entry point's limit was first set by (32 x 4 or 32
-// x 8 tiles with the reference's rounding, 64-column tiles of 14 or 4 rows
-// with fused arithmetic, at least 20 or 24 planes per block).  A step needs
-// no memory per block now; a caller that sizes its grids by the limit keeps
-// the same answer.
-long long limit_blocks(const dg_sim_info *info, int kind) {
-    const int nx = info->nx;
-    if (kind == kFastF32 || kind == kFastF64) {
-        const int rows = kind == kFastF32 ? 14 : 4;
-        const InteriorTiles it(info->ny + 4, info->nz + 4, rows, 64);
-        const long long tiles = (long long)it.tiles_y * it.tiles_z;
-        const bool columns = it.interior() >= kSms;
-        const int chunk = columns ? std::min(nx, 64) : waves_chunk(tiles, nx, 0);
-        const long long chunks = (nx + chunk - 1) / chunk;
-        return (long long)it.interior() * (columns ? 1 : chunks) + it.frame() * chunks;
-    }
-    const long long rows = kind == kRefF32 ? 8 : 4;
-    const long long tiles = (info->ny + rows - 1) / rows * ((info->nz + 31) / 32);
-    const long long want = (2LL * kSms * 14 + tiles - 1) / tiles, most = std::max(1, nx / 20);
-    const long long chunks = std::min(want, most), per = (nx + chunks - 1) / chunks;
-    return tiles * ((nx + per - 1) / per);
-}
-
 template <class T>
 int run(const dg_sim_info *info, int kind, void *cons_in, void *cons_out, double *dt_used, cudaStream_t st,
         void *scratch) {
     const int elem = (int)sizeof(T);
     GridArgs<T> a = args_for<T>(info, cons_in, cons_out, scratch);
     const int chunk = choose_chunk(a.nx, a.ny, a.nz, kind);
-    const long long blocks = limit_blocks(info, kind);
-    if (blocks > kMaxBlocks)
-        return fail(DG_ERR_INVALID, "grid too large for the no-allocation scratch (" + std::to_string(blocks) +
-                                        " blocks > " + std::to_string(kMaxBlocks) + ")");
+    const bool fused = kind == kFastF32 || kind == kFastF64;
+    if (!noalloc::accepted(info->nx, info->ny, info->nz, elem == 8, fused))
+        return fail(DG_ERR_INVALID,
+                    "grid above the size limit that the no-allocation scratch once set (" +
+                        std::to_string(noalloc::limit_blocks(info->nx, info->ny, info->nz, elem == 8, fused)) +
+                        " by its rule > " + std::to_string(noalloc::kMostBlocks) + ")");
     auto fn = encode_fn();
     if (!fn) return fail(DG_ERR_CUDA, "cuTensorMapEncodeTiled not available from the driver");
     CUtensorMap map;

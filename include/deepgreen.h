@@ -209,9 +209,9 @@ int32_t dg_compute_step_dt(dg_ctx *ctx, double dt);
  *             cannot see the device's status: read it with
  *             dg_noalloc_status after synchronizing the stream.
  *   stream    cudaStream_t or NULL.
- * The step's scratch (the control block, and room for 64 bytes per block of
- * the step) is a 1 MiB array in the library's device image, held by every GPU that loads the
- * library until exit; grids needing more than it holds are rejected with
+ * The step's scratch (its control block) lies in a 1 MiB array in the
+ * library's device image, held by every GPU that loads the library until
+ * exit.  Grids above a size limit, which that array once set, are rejected with
  * DG_ERR_INVALID.  All calls share that array: calls that overlap on the
  * GPU race.  The first call on a device looks up the array's address with
  * that device current; make it before any stream capture.  The calling
