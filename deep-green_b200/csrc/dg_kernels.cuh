@@ -240,7 +240,7 @@ inline int choose_chunk(int nx, int ny, int nz, int kind) {
     long long best = sweep_makespan(tiles, nxi, nxi);
     for (int p = nxi - 1; p >= 1; --p) {
         // short chunks only where they fill idle SMs: a large grid's count
-        // of blocks (and of partials) stays that of 24 planes or more
+        // of blocks stays that of 24 planes or more
         const long long c = (nxi + p - 1) / p;
         if ((p < 24 || c > 64) && tiles * c > 4 * kSms) continue;
         const long long t = sweep_makespan(tiles, nxi, p);
@@ -267,7 +267,8 @@ cudaError_t launch_march(const GridArgs<double> &a, const CUtensorMap *tmap_src,
 // A state from src into a.dst with its ghosts, the dt of the coming step
 // (number `step`) and a fresh control block.  prims: src holds primitives;
 // exact: the wave speeds round like the reference (FP64 always does).  src
-// may be a.dst itself: then only the ghosts are written.
+// may be a.dst itself: then the ghosts are written, and interior cells that
+// share a 16-byte access with one, with their own values.
 template <class T>
 cudaError_t launch_set_state(const GridArgs<T> &a, const FieldView<const T> &src, bool prims, bool exact,
                              unsigned long long step, cudaStream_t st);

@@ -107,8 +107,9 @@ __device__ __forceinline__ float rcp_rn(float x) { return __frcp_rn(x); }
 __device__ __forceinline__ double rcp_rn(double x) { return __drcp_rn(x); }
 
 // ---------------------------------------------------------------------------
-// Reference rounding: Phys<T, true>'s expressions, operation for operation.
-// Face states are xt + hs / xt - hs with hs = slope * ds / 2.
+// Reference rounding: the reference's expressions (physics.rs; each function
+// cites the lines it follows), operation for operation.  Face states are
+// xt + hs / xt - hs with hs = slope * ds / 2.
 // ---------------------------------------------------------------------------
 template <class T> struct RefArith {
     using Ph = Phys<T, true>;
@@ -123,6 +124,7 @@ template <class T> struct RefArith {
         k.safe = safe_divisor(a.k.ds) && safe_divisor(a.k.two_ds) && safe_divisor(a.k.vol) && safe_divisor(a.k.gm1);
         return k;
     }
+    // calc_primitives, physics.rs:112-140
     static __device__ __forceinline__ void prim(const T u[5], T w[5], const GridArgs<T> &a, const K &k) {
         const Consts<T> &c = a.k;
         KeyBounds kb;
@@ -148,7 +150,9 @@ template <class T> struct RefArith {
             w[4] = (plain_div(u[4], c.vol) - T(0.5) * r1 * (vx * vx + vy * vy + vz * vz)) * c.gm1;
         }
     }
-    // slopes of the five fields from the lower, own and upper value
+    // slopes of the five fields from the lower, own and upper value:
+    // calc_gradients, physics.rs:206-208 (LIM 0); minmod of the one-sided
+    // differences (LIM 1)
     template <int LIM>
     static __device__ __forceinline__ void slopes(const T qm[5], const T q[5], const T qp[5], T g[5],
                                                   const GridArgs<T> &a, const K &k) {
@@ -198,9 +202,12 @@ template <class T> struct RefArith {
     static __device__ __forceinline__ T grav(const GridArgs<T> &a, int klow) {
         return (T(a.nz) - T(2.0) * T(2)) * a.k.ds - (T(klow) - T(2.0)) * a.k.ds;
     }
-    // Phys<T, true>::face from the two face states: lo = the lower cell's
-    // (reference "r"), up = the upper cell's ("l"); heat: xt is the lower
-    // cell's predicted state up to its mirrored velocity.
+    // calc_flux_reconstruction, physics.rs:313-405 (the final *ds included),
+    // from the two face states: lo = the lower cell's (reference "r"), up =
+    // the upper cell's ("l"), N = 1, 2, 3: index of the normal velocity.  heat:
+    // the first face of a lower conducting wall, whose energy flux takes Q / V
+    // after the advective part (kernels.h:561-575); xt is the lower cell's
+    // predicted state up to its mirrored velocity.
     template <int N, bool GRAV>
     static __device__ __forceinline__ void face(const T lo[5], const T up[5], T h, bool heat, const T xt[5],
                                                 const GridArgs<T> &a, const K &k, T F[5]) {
@@ -263,9 +270,11 @@ template <class T> struct RefArith {
         F[T2] = f3 * c.ds;
         F[4] = f4 * c.ds;
     }
+    // add_fluxes, physics.rs:548-554 (the caller sums in the same order)
     static __device__ __forceinline__ T update(T u, T sum, int, const K &k) { return u - k.dtds * sum; }
-    // c_s + |v| of an updated cell: ds over its maximum is the minimum of the
-    // reference's ds / (c_s + |v|), division being monotone
+    // c_s + |v| of an updated cell (calc_timestep, physics.rs:187-189): ds
+    // over its maximum is the minimum of the reference's ds / (c_s + |v|),
+    // division being monotone
     static __device__ __forceinline__ T speed(const T u[5], const GridArgs<T> &a, const K &k) {
         T w[5];
         prim(u, w, a, k);

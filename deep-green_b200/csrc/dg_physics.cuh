@@ -5,11 +5,13 @@
 // src/rs/src/physics.rs; each function cites the lines it follows):
 //
 //   Phys<T, true>   "reference rounding": the reference's operation order and
-//                   association, IEEE division and square root.  Compiled
-//                   without fused multiply-add contraction (--fmad=false) it
-//                   rounds exactly like the reference's scalar code, so the
-//                   GPU result equals the CPU restatement bit for bit.  Used
-//                   for FP64 and, on request, for FP32.
+//                   association, IEEE division.  Compiled without fused
+//                   multiply-add contraction (--fmad=false) it rounds exactly
+//                   like the reference's scalar code, so the GPU result
+//                   equals the CPU restatement bit for bit.  Used for FP64
+//                   and, on request, for FP32.  Here the conversion to
+//                   primitives and the prediction; slopes, fluxes and update
+//                   are the step kernel's (RefArith, dg_march_impl.cuh).
 //   Phys<T, false>  "fast": the conversion of a state to primitives with one
 //                   reciprocal and fused multiply-adds, as the fused-arithmetic
 //                   sweep kernel (dg_sweep_impl.cuh) computes it; used by the
@@ -132,18 +134,6 @@ template <class T> struct Phys<T, true> {
         w[4] = (u[4] / k.vol - T(0.5) * r * (vx * vx + vy * vy + vz * vz)) * k.gm1;
     }
 
-    // calc_timestep body, physics.rs:187-189
-    static __device__ __forceinline__ T wave_dt(const T w[5], const Consts<T> &k) {
-        return k.ds / (sqrt(k.gamma * w[4] / w[0]) + sqrt(w[1] * w[1] + w[2] * w[2] + w[3] * w[3]));
-    }
-
-    // calc_gradients, physics.rs:206-208 (LIM 0); minmod of the one-sided
-    // differences (LIM 1)
-    template <int LIM> static __device__ __forceinline__ T slope(T qm, T q0, T qp, const Consts<T> &k) {
-        if (LIM == 0) return (qp - qm) / k.two_ds;
-        return minmod((q0 - qm) / k.ds, (qp - q0) / k.ds);
-    }
-
     // extrapolate_primitives_t, physics.rs:251-278; gx/gy/gz are d/dx, d/dy,
     // d/dz of (rho, vx, vy, vz, p)
     static __device__ __forceinline__ void predict(const T w[5], const T gx[5], const T gy[5], const T gz[5], T dt,
@@ -155,68 +145,6 @@ template <class T> struct Phys<T, true> {
         out[2] = vy - h * (vx * gx[2] + vy * gy[2] + vz * gz[2] + (T(1.0) / rho) * gy[4]);
         out[3] = vz - h * (vx * gx[3] + vy * gy[3] + vz * gz[3] + (T(1.0) / rho) * gz[4]);
         out[4] = p - h * (k.gamma * p * (gx[1] + gy[2] + gz[3]) + vx * gx[4] + vy * gy[4] + vz * gz[4]);
-    }
-
-    // calc_flux_reconstruction, physics.rs:313-405, for the face between the
-    // lower cell (xl, gl = predicted state, slope along the face normal) and
-    // the upper cell (xu, gu).  n = 1, 2, 3: index of the normal velocity.
-    // The result includes the final *ds (physics.rs:401-405).  klow: z index
-    // of the lower cell, for the gravity term (z faces only, grav != 0).
-    // heat: the face is the first face of a lower conducting wall; its
-    // energy flux takes Q / V after the advective part (kernels.h:561-575).
-    static __device__ __forceinline__ void face(const T xl[5], const T gl[5], const T xu[5], const T gu[5], int n,
-                                                int grav, int klow, int nz, const Consts<T> &k, T F[5],
-                                                bool heat = false) {
-        const int t1 = n == 1 ? 2 : 1, t2 = n == 3 ? 2 : 3;
-        const T half = k.half_ds;
-        const T rl = xu[0] - gu[0] * half;
-        const T rr = xl[0] + gl[0] * half;
-        const T vxl = xu[n] - gu[n] * half;
-        const T vxr = xl[n] + gl[n] * half;
-        const T vyl = xu[t1] - gu[t1] * half;
-        const T vyr = xl[t1] + gl[t1] * half;
-        const T vzl = xu[t2] - gu[t2] * half;
-        const T vzr = xl[t2] + gl[t2] * half;
-        const T pl = xu[4] - gu[4] * half;
-        const T pr = xl[4] + gl[4] * half;
-        const T en_left = T(0.5) * (rl * (vxl * vxl + vyl * vyl + vzl * vzl)) + (pl / k.gm1);
-        const T en_right = T(0.5) * (rr * (vxr * vxr + vyr * vyr + vzr * vzr)) + (pr / k.gm1);
-        const T rho_star = (rl + rr) / T(2.0);
-        const T mx = (rl * vxl + rr * vxr) / T(2.0);
-        const T my = (rl * vyl + rr * vyr) / T(2.0);
-        const T mz = (rl * vzl + rr * vzr) / T(2.0);
-        const T en_star = T(0.5) * (en_left + en_right);
-        const T p_star = k.gm1 * (en_star - T(0.5) * (mx * mx + my * my + mz * mz) / rho_star);
-        T f0 = mx;
-        T f1 = (mx * mx / rho_star) + p_star;
-        T f2 = mx * my / rho_star;
-        T f3 = mx * mz / rho_star;
-        T f4 = (en_star + p_star) * (mx / rho_star);
-        if (heat) f4 += wall_heat(xl[0], xl[4], k.ds);
-        if (grav) {
-            const T h = (T(nz) - T(2.0) * T(2)) * k.ds - (T(klow) - T(2.0)) * k.ds;
-            f1 += T(1.0) * rho_star * k.g * h;
-            f4 += T(0.5) * rho_star * (vxl + vxr) * k.g * h;
-        }
-        const T c_l = sqrt(k.gamma * pl / rl) + fabs(vxl);
-        const T c_r = sqrt(k.gamma * pr / rr) + fabs(vxr);
-        const T c_star = fmax(c_l, c_r);
-        f0 = mx - T(0.5) * c_star * (rl - rr);
-        f1 -= c_star * (rl * vxl - rr * vxr) / T(2.0);
-        f2 -= c_star * (rl * vyl - rr * vyr) / T(2.0);
-        f3 -= c_star * (rl * vzl - rr * vzr) / T(2.0);
-        f4 -= c_star * (en_left - en_right) / T(2.0);
-        F[0] = f0 * k.ds;
-        F[n] = f1 * k.ds;
-        F[t1] = f2 * k.ds;
-        F[t2] = f3 * k.ds;
-        F[4] = f4 * k.ds;
-    }
-
-    // add_fluxes, physics.rs:548-554, same summation order
-    static __device__ __forceinline__ T update(T u, T fxh, T fxl, T fyh, T fyl, T fzh, T fzl, T dt,
-                                               const Consts<T> &k) {
-        return u - dt * k.ds * (fxh - fxl + fyh - fyl + fzh - fzl);
     }
 };
 
