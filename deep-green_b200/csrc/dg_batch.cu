@@ -168,6 +168,8 @@ long long batch_makespan(const dg_batch *b, const std::vector<int> &order, int c
 // rule: 1 grid of 24-40 cells an axis 203 / 98 / 26, 4 of 16-40 176 / 101 / 38,
 // 12 of 20-60 276 / 107 / 89, 12 of 32-90 351 / 181 / 177, 24 of 24-100 376 /
 // 297 / 297, 48 of 32-160 1463 / 1445 / 1432; within 1.5 % of the best in all.
+// Of large grids (2 of 508x252x252, 5 of 400x300x200, 4 of 1500x70x128) within
+// 0.5 %, longer items up to whole columns tried.
 int auto_chunk(const dg_batch *b, const std::vector<int> &order) {
     constexpr int cand[] = {64, 48, 40, 32, 28, 24, 20, 16, 12, 10, 8, 6, 5, 4, 3, 2, 1};
     int best = cand[0];
